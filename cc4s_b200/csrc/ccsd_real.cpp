@@ -496,6 +496,7 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
     c.C = vw(R2 + x0 * o * n1 + y0 * o, o * n1, o, n1, 1);
     c.alpha = x0 == y0 ? 0.5 : 1.0;  // the symmetrisation that follows adds the mirror
     c.beta = 1.0;
+    c.digits = digits_for(c, true);
     return c;
   };
   auto build_of = [&](int64_t x0, int64_t sx, int64_t y0, int64_t sy, int64_t c0, int64_t nc) {
@@ -504,13 +505,14 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
     build.A = vw(cp(dGpp) + x0 * v + c0, v, 1, 0, v * v);
     build.B = vw(cp(dGpp) + y0 * v, 0, v * v, v, 1);
     build.C = vw(slab_, sy * nc * v, v, nc * v, 1);
+    build.digits = digits_for(build, true);
     return build;
   };
-  // Split form: the X panel (operand B of every contraction of one c range, shared
+  // Digit forms: the X panel (operand B of every contraction of one c range, shared
   // by all block pairs: B depends on N = o^2, K = c_n v and the X view only) is
   // sliced once per c range into a region kept beside the per-contraction scratch.
   const Contraction c_first = contraction(0, std::min(s, v), 0, std::min(s, v), 0, std::min(cn, v));
-  const bool prepack = !taping_ && split_ok(c_first) && split_single_panel(c_first) && nb > 1;
+  const bool prepack = !taping_ && c_first.digits && split_single_panel(c_first) && nb > 1;
   if (prepack) {
     size_t regular = 0;
     for (int64_t c0 = 0; c0 < v; c0 += cn) {
@@ -521,8 +523,8 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
           const int64_t sy = std::min(s, v - Yb * s);
           const Contraction b = build_of(X * s, sx, Yb * s, sy, c0, nc);
           const Contraction c = contraction(X * s, sx, Yb * s, sy, c0, nc);
-          if (split_ok(b)) regular = std::max(regular, gemm_split_scratch_bytes(b));
-          if (split_ok(c)) regular = std::max(regular, split_scratch_bytes_packed_b(c));
+          if (b.digits) regular = std::max(regular, gemm_split_scratch_bytes(b));
+          if (c.digits) regular = std::max(regular, split_scratch_bytes_packed_b(c));
         }
       }
     }
@@ -541,7 +543,9 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
         ev_shape_.push_back({0, o * o, nc * v, 1});
         ops::event_record(ev_[2 * k], s_);
       }
-      pb = split_pack_b(contraction(0, s, 0, s, c0, nc), split_extra_, s_);
+      Contraction whole = contraction(0, s, 0, s, c0, nc);
+      whole.digits = c_first.digits;
+      pb = split_pack_b(whole, split_extra_, s_);
       if (prof) ops::event_record(ev_[2 * k + 1], s_);
     }
     for (int64_t X = 0; X < nb; ++X) {
@@ -552,7 +556,7 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
         tc_(build);
         {
           const Contraction c = contraction(x0, sx, y0, sy, c0, nc);
-          if (prepack && split_ok(c)) tc_packed_b_(c, pb);
+          if (prepack && c.digits == pb.digits) tc_packed_b_(c, pb);
           else tc_(c);
           if (taping_) {  // the slab is rebuilt before this contraction's adjoint
             tape_.back().recompute = true;

@@ -44,6 +44,8 @@ struct Contraction {
   View C;   // rows m, cols n
   View C2;  // optional second output (C2.p == nullptr: none): C2 = alpha*AB + beta*C2
   double alpha = 1.0, beta = 0.0;
+  // Digit form of the tensor-core contractions (split_gemm.cuh): 7 is the FP64 one.
+  int digits = 4;
 };
 
 // Scratch memory used by split-K partial sums.

@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -52,19 +53,34 @@ void Schedule::gemm_(const Contraction& c) {
     ev_split_.push_back(0);
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
-    gemm(c, s_, scratch_);
+    fp64_exec(c);
     ops::event_record(ev_[2 * k + 1], s_);
     return;
   }
-  gemm(c, s_, scratch_);
+  fp64_exec(c);
 }
 
 namespace {
 constexpr size_t kSplitDataOffset = 128;  // doubles: 1 KiB
 }  // namespace
 
-bool Schedule::split_ok(const Contraction& c) const {
-  return precision_ != 0 && c.batch == 1 && c.K >= 64 && c.M >= 64 && c.N >= 64;
+// FP64 contractions: the seven-digit form where its time (slicing, then the integer
+// tensor cores) is below the FP64 tensor pipe's.
+static bool digits7_pays(const Contraction& c) {
+  if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K < 64) return false;
+  const double M = double(c.M), N = double(c.N), K = double(c.K);
+  auto up = [](double x, double t) { return std::ceil(x / t) * t; };
+  // microseconds: launches, slicing, waves of one tile per SM
+  const double tiles7 = up(M, 128) * up(N, 64) / (128 * 64);
+  const double d7 = 20.0 + 24.0 * (M + N) * K / 3.5e6 +
+                    std::ceil(tiles7 / 148.0) * (3.3 + 0.021 * up(K, 32));
+  const double dmma = 12.0 + 2.0 * up(M, 128) * up(N, 128) * K / 22e6;
+  return d7 < dmma;
+}
+
+int Schedule::digits_for(const Contraction& c, bool big) const {
+  if (big && precision_ != 0 && c.batch == 1 && c.K >= 64 && c.M >= 64 && c.N >= 64) return 4;
+  return digits7_pays(c) ? 7 : 0;
 }
 
 void Schedule::split_reserve(size_t regular, size_t extra) {
@@ -76,6 +92,7 @@ void Schedule::split_reserve(size_t regular, size_t extra) {
   ops::sync(s_);
   if (split_mem_) ops::release(split_mem_);
   split_mem_ = nullptr;
+  split_ = SplitScratch();  // nothing is left if the allocation fails
   split_extra_ = nullptr;
   split_extra_bytes_ = 0;
   // The error word sits in the first double; the packed slices start 1 KiB in,
@@ -99,6 +116,26 @@ void Schedule::split_exec(const Contraction& c) {
   // operand is live across a contraction that needs more than the reserved part)
   if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
   gemm_split(c, s_, split_);
+}
+
+void Schedule::fp64_exec(const Contraction& c) {
+  if (digits_for(c, false) == 7) {
+    Contraction d = c;
+    d.digits = 7;
+    bool fits = true;
+    try {
+      const size_t need = gemm_split_scratch_bytes(d);
+      if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
+    } catch (const Error& e) {
+      if (e.status != ERR_OUT_OF_MEMORY) throw;
+      fits = false;  // no room for the digits: the FP64 tensor pipe needs none
+    }
+    if (fits) {
+      gemm_split(d, s_, split_);
+      return;
+    }
+  }
+  gemm(c, s_, scratch_);
 }
 
 void Schedule::tc_packed_b_(const Contraction& c, const SplitPackedB& b) {
@@ -142,12 +179,12 @@ void Schedule::tc_prepacked_(const Contraction& c, const SplitOperand& A, const 
 // A contraction of the reverse sweep (or a recomputed forward one): split
 // precision under the same rule as tc_, else FP64; neither recorded nor counted.
 void Schedule::exec_(const Contraction& c) {
-  if (split_ok(c)) split_exec(c);
-  else gemm(c, s_, scratch_);
+  if (digits_for(c, true) == 4) split_exec(c);
+  else fp64_exec(c);
 }
 
 void Schedule::tc_(const Contraction& c) {
-  if (!split_ok(c)) {
+  if (digits_for(c, true) != 4) {
     gemm_(c);
     return;
   }

@@ -41,8 +41,8 @@ class Schedule {
   size_t device_bytes() const { return bytes_; }
 
   void set_profile(bool on) { profile_ = on; }
-  // 0: FP64 throughout; 3: the large ladder / ring / vertex contractions run as
-  // three-slice split-precision products on the tcgen05 tensor cores (in adjoint
+  // 0: FP64 throughout; 3: the large ladder / ring / vertex contractions run in
+  // split precision (four digits) on the tcgen05 tensor cores (in adjoint
   // mode also the recorded forward pass and the large contractions of the
   // reverse sweep).
   void set_precision(int slices) { precision_ = slices; }
@@ -148,8 +148,12 @@ class Schedule {
   // A large contraction: split precision when enabled (batch 1), else FP64.
   // Recorded on the tape when taping, like gemm_.
   void tc_(const Contraction& c);
-  bool split_ok(const Contraction& c) const;
+  // The digit form a contraction runs in: 4 (a large one in split precision), 7 (FP64 on
+  // the integer tensor cores) or 0 (the FP64 tensor pipe).
+  int digits_for(const Contraction& c, bool big) const;
   void split_exec(const Contraction& c);
+  // One contraction in FP64, in the faster of its two forms.
+  void fp64_exec(const Contraction& c);
   // Makes the split scratch hold `regular` bytes for per-contraction packing plus a
   // second region of `extra` bytes (split_extra_) that survives those calls; may
   // reallocate (synchronises).  A later split_exec that needs more than `regular`

@@ -1,28 +1,29 @@
-// Split-precision FP64 contraction: FP16 integer slices on tcgen05 tensor cores.
+// FP64 contraction in signed 8-bit digits on the tcgen05 tensor cores (kind::i8).
 //
-// Kernel layout (one 128 x 128 output tile per CTA, 320 threads):
-//   warp 0      TMA producer: per k-block of 32, three A-slice and three
-//               B-slice tiles (128 x 32 FP16, 64-byte swizzle) into a 4-stage
-//               shared-memory ring, completion tracked by mbarriers;
-//   warp 1      allocates 512 TMEM columns; one thread issues tcgen05.mma
-//               (M=128, N=128, K=16) for the six slice products into three
-//               FP32 accumulators (TMEM columns 0, 128, 256) and commits to
-//               mbarriers that release smem stages and publish K chunks;
-//   warps 2..9  epilogue: after each K chunk, tcgen05.ld the three groups and
-//               add them into FP64 register accumulators (two warps per TMEM
-//               lane quadrant, 64 columns each); after the last chunk, scale,
-//               stage the tile in the idle stage buffers and store C once,
-//               coalesced along the output's contiguous index.
+// Kernel layout (persistent, one CTA of 320 threads per SM, 128 x TN output tiles,
+// TN = 128 with 4 digits, 64 with 7):
+//   warp 0      TMA producer: per k-block all digit planes of the A rows and of the
+//               B rows (two 3-D boxes, swizzled) into a shared-memory ring, completion
+//               tracked by mbarriers;
+//   warp 1      allocates 512 TMEM columns; one thread issues tcgen05.mma (M = 128,
+//               N up to 256, K = 32) for the digit products of equal weight p + q into
+//               one S32 accumulator each (TN columns at TN (p + q)): A digit p times
+//               the adjacent B digits q is one MMA into adjacent groups;
+//   warps 2..9  epilogue: tcgen05.ld of the groups, exact 64-bit integer combination of
+//               four groups at a time, conversion to FP64, then scale and store of the
+//               tile (through warp-private transposes where the columns are contiguous)
+//               while the MMA issuer is on the next tile.
+// Integer accumulation is exact, so a tile is drained once per 16384 of K.
 // Every mbarrier wait is bounded; on expiry the kernel records an error flag
 // and every role leaves its loop, so the kernel always terminates.
 #include "split_gemm.cuh"
 
 #include <cuda.h>
-#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <climits>
 #include <cstdlib>
 #include <mutex>
 #include <vector>
@@ -31,26 +32,30 @@ namespace cc4s_b200 {
 
 namespace {
 
-// Stage geometry.  Wide stages: k-blocks of 64 (128-byte rows, 128-byte swizzle),
-// two 96 KB stages, half as many TMA row requests per byte as the narrow form
-// (k-blocks of 32, 64-byte rows and swizzle, four 48 KB stages).
-#ifndef CC4S_SPLIT_WIDE_STAGES
-#define CC4S_SPLIT_WIDE_STAGES 0
-#endif
-#if CC4S_SPLIT_WIDE_STAGES
-constexpr int TK = 64, NST = 2;
-constexpr uint32_t ROW_BYTES = 128;               // smem row of one k-block (bytes)
-#else
-constexpr int TK = 32, NST = 4;
-constexpr uint32_t ROW_BYTES = 64;
-#endif
-constexpr int TM = 128, TN = 128, NSLICE = 3;
-constexpr int KCHUNK = 4096;                      // exact FP32 span of the leading group
-constexpr int TILE_BYTES = TM * TK * 2;           // one slice tile: 8 KB (narrow), 16 KB (wide)
-constexpr int STAGE_BYTES = 2 * NSLICE * TILE_BYTES;
-constexpr int SMEM_BYTES = NST * STAGE_BYTES + 1024 + 256;
+constexpr int TM = 128;
+constexpr int KPAD = 32;                         // K step of one MMA: packed K granularity
+// |digit product| <= 2^14, at most 7 products per group and k: exact in S32 up to here
+constexpr int KCHUNK = 16384;
 constexpr uint32_t WAIT_LIMIT = 1u << 28;         // bounded mbarrier waits
 constexpr int64_t RASTER_M = 8;                  // tile rows per raster group
+constexpr int WBUF_DOUBLES = 32 * 16;            // transpose buffer of one epilogue warp
+constexpr int EXP_NONFINITE = INT_MAX;           // exponent of a row holding Inf or NaN
+
+// Geometry of the two forms: NS digits, groups p + q < NG, TN columns per tile (TN NG =
+// the 512 TMEM columns), k-blocks of TK bytes (= the swizzle width), NST ring stages.
+template <int NS_> struct Form;
+template <> struct Form<4> {
+  static constexpr int NS = 4, NG = 4, TN = 128, TK = 64, NST = 3;
+};
+template <> struct Form<7> {
+  static constexpr int NS = 7, NG = 8, TN = 64, TK = 64, NST = 2;
+};
+template <class F> __host__ __device__ constexpr int a_bytes() { return F::NS * TM * F::TK; }
+template <class F> __host__ __device__ constexpr int stage_bytes() { return F::NS * (TM + F::TN) * F::TK; }
+template <class F> constexpr int smem_bytes() {
+  return F::NST * stage_bytes<F>() + 8 * WBUF_DOUBLES * 8 + 1024 + 256;
+}
+int tile_n(int digits) { return digits == 7 ? Form<7>::TN : Form<4>::TN; }
 
 std::atomic<uint64_t> g_split_launches{0};
 std::atomic<uint64_t> g_pack_launches{0};
@@ -68,7 +73,7 @@ Ax mkax(int64_t inner, int64_t s_o, int64_t s_i) {
 }
 
 // ---------------------------------------------------------------------------
-// Packing: operand element (r, k) -> three FP16 integer slices P[q][r][k]
+// Packing: operand element (r, k) -> NS signed 8-bit digits P[q][r][k]
 // (row-padded to Rp, k-padded to Kp) and a per-row exponent.
 struct PackArgs {
   const double* src;
@@ -76,15 +81,21 @@ struct PackArgs {
   int64_t R, K, Rp, Kp;
   unsigned long long* rmax;  // per-row max |x| as IEEE bits (non-negative doubles)
   int* rexp;              // per-row exponent
-  __half* dst;            // [3][Rp][Kp]
+  int8_t* dst;            // [NS][Rp][Kp]
   int r_contig;           // 1: the row index is the contiguous one in memory
+};
+// One launch slices up to two operands (A and B of a contraction).
+struct PackPair {
+  PackArgs op[2];
+  int64_t first;          // work items of op[0]; the rest belong to op[1]
+  int64_t total;
 };
 
 // Packing works on tiles of 64 rows x 64 k staged in shared memory.  The row and
 // k offsets of a tile are computed once per tile (two-level index maps need an
-// integer division each), every thread keeps 16 loads in flight, and the FP16
-// slices leave as 16-byte vector stores along k.
-constexpr int PR = 64, PKT = 64, PTHREADS = 256, PSTRIP = 16;  // strip: k tiles per row max
+// integer division each), every thread keeps 16 loads in flight, and the digits
+// leave as 16-byte vector stores along k.
+constexpr int PR = 64, PKT = 64, PTHREADS = 256;
 
 struct PackTile {
   double v[PR][PKT + 1];
@@ -123,75 +134,146 @@ __device__ __forceinline__ void pack_load_tile(const PackArgs& a, int64_t r0, in
   __syncthreads();
 }
 
-// Row maxima |x| over all k, as IEEE bits of non-negative doubles: each block
-// walks PSTRIP k tiles of one row strip, one atomicMax per row and strip.
-__global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackArgs a) {
-  __shared__ PackTile t;
-  const int64_t nr = a.Rp / PR, nks = (a.Kp + PKT * PSTRIP - 1) / (PKT * PSTRIP);
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3;  // 4 threads per row, 16 k each
-  for (int64_t w = blockIdx.x; w < nr * nks; w += gridDim.x) {
-    const int64_t r0 = (w / nks) * PR, kbeg = (w % nks) * PKT * PSTRIP;
-    double m = 0.0;
-    for (int64_t k0 = kbeg; k0 < kbeg + PKT * PSTRIP && k0 < a.Kp; k0 += PKT) {
-      pack_load_tile(a, r0, k0, t);
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return static_cast<unsigned long long>(__double_as_longlong(fabs(x)));
+}
+
+// Row maxima |x| as IEEE bits of non-negative doubles (Inf and NaN order above every
+// number).  A work item is 64 rows x `kstrip` k, read straight from memory with the lanes
+// along the contiguous index and 16 loads in flight per thread; one atomicMax per row.
+// Bound by latency until a few hundred items are in flight, which sets kstrip: strips of
+// 1024 k left two 1024 x 1024 operands to 32 blocks (whole seven-digit contraction 79 us,
+// 63 us with strips of 128).
+__global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackPair pp, int kstrip) {
+  __shared__ unsigned long long part[8][PR];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int64_t it = blockIdx.x; it < pp.total; it += gridDim.x) {
+    const PackArgs& a = pp.op[it < pp.first ? 0 : 1];
+    const int64_t w = it < pp.first ? it : it - pp.first;
+    const int64_t nks = (a.K + kstrip - 1) / kstrip;
+    const int64_t r0 = (w / nks) * PR, kbeg = (w % nks) * kstrip;
+    const int64_t kend = min(a.K, kbeg + kstrip);
+    if (a.r_contig) {  // lanes on rows; the eight warps take every eighth k
+      unsigned long long m[2] = {0, 0};
+      const int64_t ra = r0 + lane, rb = ra + 32;
+      const double* sa = a.src + (ra < a.R ? a.ar.off(static_cast<uint32_t>(ra)) : 0);
+      const double* sb = a.src + (rb < a.R ? a.ar.off(static_cast<uint32_t>(rb)) : 0);
+      for (int64_t k0 = kbeg + warp; k0 < kend; k0 += 64) {
+        double x[2][8];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) m = fmax(m, fabs(t.v[row][16 * part + j]));
+        for (int j = 0; j < 8; ++j) {
+          const int64_t k = k0 + 8 * j;
+          const int64_t ko = k < kend ? a.ak.off(static_cast<uint32_t>(k)) : 0;
+          x[0][j] = k < kend && ra < a.R ? sa[ko] : 0.0;
+          x[1][j] = k < kend && rb < a.R ? sb[ko] : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) m[h] = max(m[h], abs_bits(x[h][j]));
+      }
+      part[warp][lane] = m[0];
+      part[warp][lane + 32] = m[1];
       __syncthreads();
+      if (threadIdx.x < PR) {
+        unsigned long long v = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v = max(v, part[q][threadIdx.x]);
+        if (r0 + threadIdx.x < a.R && v != 0) atomicMax(&a.rmax[r0 + threadIdx.x], v);
+      }
+      __syncthreads();
+    } else {           // lanes on k; every warp takes eight rows
+      const int64_t rw = r0 + 8 * warp;
+      unsigned long long m[8];
+      const double* src[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        m[q] = 0;
+        src[q] = rw + q < a.R ? a.src + a.ar.off(static_cast<uint32_t>(rw + q)) : nullptr;
+      }
+      for (int64_t k0 = kbeg + lane; k0 < kend; k0 += 64) {
+        const int64_t k1 = k0 + 32;
+        const int64_t o0 = a.ak.off(static_cast<uint32_t>(k0));
+        const int64_t o1 = k1 < kend ? a.ak.off(static_cast<uint32_t>(k1)) : o0;
+        double x[2][8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          x[0][q] = src[q] ? src[q][o0] : 0.0;
+          x[1][q] = src[q] ? src[q][o1] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) m[q] = max(m[q], max(abs_bits(x[0][q]), abs_bits(x[1][q])));
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) m[q] = max(m[q], __shfl_xor_sync(0xffffffffu, m[q], s));
+        if (lane == q && src[q] && m[q] != 0) atomicMax(&a.rmax[rw + q], m[q]);
+      }
     }
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    const int64_t r = r0 + row;
-    if (part == 0 && r < a.R && m > 0.0)
-      atomicMax(&a.rmax[r], static_cast<unsigned long long>(__double_as_longlong(m)));
   }
 }
 
-// Three FP16 integer slices of every element (row-padded to Rp, k-padded to Kp)
-// and the per-row exponent.
-__global__ void __launch_bounds__(PTHREADS) pack_slices_kernel(PackArgs a) {
+// 2^e as an exact double: built from its exponent bits in the normal range.
+__device__ __forceinline__ double pow2i(int e) {
+  if (e >= -1022 && e <= 1023) return __longlong_as_double(static_cast<long long>(e + 1023) << 52);
+  return ldexp(1.0, e);
+}
+
+// The digits of every element (row-padded to Rp, k-padded to Kp) and the per-row
+// exponent: x = 2^e X 2^-(8 NS - 2) with |X| <= 2^(8 NS - 2) rounded to an integer and
+// written in balanced base 256, lowest digit first (each in [-128, 127], the top one in
+// [-64, 65]).  Memory bound: 8 B read and NS B written per element.
+template <int NS>
+__global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackPair pp) {
   __shared__ PackTile t;
-  __shared__ int rexp_s[PR];
-  const int64_t nr = a.Rp / PR, nk = (a.Kp + PKT - 1) / PKT;
+  __shared__ double scale_s[2][PR];
   const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  const int64_t pl = a.Rp * a.Kp;
-  for (int64_t w = blockIdx.x; w < nr * nk; w += gridDim.x) {
+  for (int64_t it = blockIdx.x; it < pp.total; it += gridDim.x) {
+    const PackArgs& a = pp.op[it < pp.first ? 0 : 1];
+    const int64_t w = it < pp.first ? it : it - pp.first;
+    const int64_t nk = (a.Kp + PKT - 1) / PKT, pl = a.Rp * a.Kp;
     const int64_t r0 = (w / nk) * PR, k0 = (w % nk) * PKT;
     if (threadIdx.x < PR) {
       const int64_t r = r0 + threadIdx.x;
-      int e = 0;
+      double s1 = 0.0, s2 = 0.0;  // their product 2^(8 NS - 2 - e), each in the normal range
       if (r < a.R) {
-        const double m = __longlong_as_double(static_cast<long long>(a.rmax[r]));
-        if (m > 0.0) frexp(m, &e);
+        const unsigned long long mb = a.rmax[r];
+        int e = 0;
+        if (mb >= 0x7ff0000000000000ull) {
+          e = EXP_NONFINITE;
+        } else if (mb != 0) {
+          frexp(__longlong_as_double(static_cast<long long>(mb)), &e);
+          const int sh = 8 * NS - 2 - e;
+          s1 = pow2i(sh / 2);
+          s2 = pow2i(sh - sh / 2);
+        }
         if (k0 == 0) a.rexp[r] = e;
       }
-      rexp_s[threadIdx.x] = e;
+      scale_s[0][threadIdx.x] = s1;
+      scale_s[1][threadIdx.x] = s2;
     }
-    pack_load_tile(a, r0, k0, t);   // its first barrier also publishes rexp_s
+    pack_load_tile(a, r0, k0, t);   // its first barrier also publishes scale_s
     const int64_t r = r0 + row, kb = k0 + 16 * part;
     if (kb < a.Kp) {
-      const int e = rexp_s[row];
-      __align__(16) __half h[3][16];
+      const double s1 = scale_s[0][row], s2 = scale_s[1][row];
+      __align__(16) int8_t h[NS][16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        double x = ldexp(t.v[row][16 * part + j], -e) * 64.0;   // |x| <= 64
-        const double s1 = rint(x);
-        double u = (x - s1) * 2048.0;                            // |u| <= 1024
-        const double s2 = rint(u);
-        u = (u - s2) * 2048.0;
-        const double s3 = rint(u);
-        // integers of at most 11 bits: exact in FP32 and FP16
-        h[0][j] = __float2half_rn(static_cast<float>(s1));
-        h[1][j] = __float2half_rn(static_cast<float>(s2));
-        h[2][j] = __float2half_rn(static_cast<float>(s3));
+        const double v = t.v[row][16 * part + j];
+        long long X = s1 != 0.0 ? __double2ll_rn(v * s1 * s2) : 0;
+#pragma unroll
+        for (int q = NS - 1; q > 0; --q) {
+          const int8_t d = static_cast<int8_t>(X & 255);
+          h[q][j] = d;
+          X = (X - d) >> 8;
+        }
+        h[0][j] = static_cast<int8_t>(X);
       }
       const int64_t o = r * a.Kp + kb;
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        uint4* d = reinterpret_cast<uint4*>(a.dst + q * pl + o);
-        const uint4* src = reinterpret_cast<const uint4*>(h[q]);
-        d[0] = src[0];
-        d[1] = src[1];
-      }
+      for (int q = 0; q < NS; ++q)
+        *reinterpret_cast<uint4*>(a.dst + q * pl + o) = *reinterpret_cast<const uint4*>(h[q]);
     }
     __syncthreads();
   }
@@ -231,56 +313,92 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   }
   return false;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int c0, int c1) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
+                                            int c0, int c1, int c2) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];\n"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];\n"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-// Shared-memory matrix descriptor: K-major, swizzled rows of ROW_BYTES (64 or 128),
-// 8-row groups 8 * ROW_BYTES apart.
+// Shared-memory matrix descriptor: K-major, swizzled rows of ROW bytes (32, 64 or 128),
+// 8-row groups 8 * ROW apart.
+template <int ROW>
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFF);        // start address
   d |= static_cast<uint64_t>(1) << 16;                       // leading byte offset (16 B)
-  d |= static_cast<uint64_t>((8 * ROW_BYTES) >> 4) << 32;    // stride byte offset
+  d |= static_cast<uint64_t>((8 * ROW) >> 4) << 32;          // stride byte offset
   d |= static_cast<uint64_t>(1) << 46;                       // descriptor version (sm100)
-  d |= static_cast<uint64_t>(ROW_BYTES == 128 ? 2 : 4) << 61;  // SWIZZLE_128B / SWIZZLE_64B
+  d |= static_cast<uint64_t>(ROW == 128 ? 2 : ROW == 64 ? 4 : 6) << 61;  // swizzle width
   return d;
 }
-// Instruction descriptors: D = F32, A = B = F16, both K-major, M = 128, N = 128 or 256.
-constexpr uint32_t IDESC128 = (1u << 4) | ((TN >> 3) << 17) | ((TM >> 4) << 24);
-constexpr uint32_t IDESC256 = (1u << 4) | (((2 * TN) >> 3) << 17) | ((TM >> 4) << 24);
+// Instruction descriptor: D = S32, A = B = signed 8 bit, both K-major, M = 128.
+__host__ __device__ constexpr uint32_t idesc_i8(int n) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
+         (static_cast<uint32_t>(TM >> 4) << 24);
+}
 
 __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
                                      uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n"
       ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc));
+}
+// COLS columns of D at column d: A (one digit) times COLS consecutive rows of the B planes.
+template <int COLS, int ROW>
+__device__ __forceinline__ void umma_row(uint32_t d, uint64_t da, uint32_t b, uint32_t acc) {
+#pragma unroll
+  for (int c = 0; c < COLS; c += 256) {
+    constexpr int W = 256;
+    if (COLS - c >= W) umma(d + c, da, sdesc<ROW>(b + c * ROW), idesc_i8(W), acc);
+    else umma(d + c, da, sdesc<ROW>(b + c * ROW), idesc_i8(COLS % W), acc);
+  }
+}
+// All digit products with p + q < NG of one K step of 32: A digit p against B digits
+// 0 .. min(NS, NG - p) - 1, into groups p and up.  `init` starts the accumulators: group
+// g is first written by p = 0, or by p = 1 where g = NS.
+template <class F, int P>
+__device__ __forceinline__ void umma_digits(uint32_t tmem, uint32_t a, uint32_t b, bool init) {
+  if constexpr (P < F::NS) {
+    constexpr int CNT = F::NS < F::NG - P ? F::NS : F::NG - P;
+    const uint64_t da = sdesc<F::TK>(a + P * TM * F::TK);
+    if constexpr (P == 1 && F::NG > F::NS) {
+      if (init) {
+        umma_row<(CNT - 1) * F::TN, F::TK>(tmem + F::TN, da, b, 1u);
+        umma_row<F::TN, F::TK>(tmem + CNT * F::TN, da, b + (CNT - 1) * F::TN * F::TK, 0u);
+      } else {
+        umma_row<CNT * F::TN, F::TK>(tmem + F::TN, da, b, 1u);
+      }
+    } else {
+      umma_row<CNT * F::TN, F::TK>(tmem + P * F::TN, da, b, P == 0 && init ? 0u : 1u);
+    }
+    umma_digits<F, P + 1>(tmem, a, b, init);
+  }
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
                ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&r)[8]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-      "%14,%15}, [%16];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
+        "=r"(r[7])
       : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-// 2^e as an exact double: built from its exponent bits in the normal range.
-__device__ __forceinline__ double pow2i(int e) {
-  if (e >= -1022 && e <= 1023) return __longlong_as_double(static_cast<long long>(e + 1023) << 52);
-  return ldexp(1.0, e);
+// The power of two of a packed row or column, NaN where it held a non-finite element.
+__device__ __forceinline__ double row_scale(double alpha, int e, int shift) {
+  if (e == EXP_NONFINITE) return __longlong_as_double(0x7ff8000000000000ll);
+  return alpha * pow2i(e - shift);
+}
+// Four groups of neighbouring weight 2^-8 as one exact integer, in units of the last.
+__device__ __forceinline__ long long combine4(int g0, int g1, int g2, int g3) {
+  return ((static_cast<long long>(g0) * 256 + g1) * 256 + g2) * 256 + g3;
 }
 // Accumulating store of NB output elements: every old value is loaded before the
 // first store, so the NB reads are in flight together (a store followed by a load
@@ -304,7 +422,7 @@ __device__ __forceinline__ void rmw_store(double* const (&ptr)[NB], const double
 
 struct SplitParams {
   int64_t M, N, K;                 // logical extents
-  int64_t Mp, Np;                  // padded row counts of the packed operands (slice strides)
+  int64_t Kp;                      // packed K (a multiple of KPAD)
   int nkb;                         // k-blocks of TK
   Ax Cm, Cn, C2m, C2n;
   double* C; double* C2;
@@ -319,212 +437,13 @@ struct SplitParams {
   int64_t b_run, b_stride, b_base, b_tiles, nNt;
 };
 
-__global__ void __launch_bounds__(320)
-split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-             SplitParams p) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  // 1024-byte aligned stage buffers, then barriers
-  unsigned char* base = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + NST * STAGE_BYTES);
-  // bars[0..NST): full, [NST..2NST): empty, [2NST]: acc_full, [2NST+1]: acc_empty
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NST + 2);
-  __shared__ int abort_flag;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Tile order: groups of RASTER_M tile rows sweep the tile columns together, so
-  // the CTAs resident at one time share a few A row tiles and reuse each B tile
-  // RASTER_M times from L2 instead of streaming B from DRAM once per tile row.
-  int64_t m0, n0;
-  {
-    const int64_t nM = p.Mp / TM, nN = p.Np / TN, b = blockIdx.x;
-    const int64_t per_group = RASTER_M * nN, group = b / per_group;
-    const int64_t first = group * RASTER_M;
-    const int64_t rows = nM - first < RASTER_M ? nM - first : RASTER_M;
-    const int64_t in = b - group * per_group;
-    m0 = (first + in % rows) * TM;
-    n0 = (in / rows) * TN;
-  }
-  const int nchunks = (p.nkb * TK + KCHUNK - 1) / KCHUNK;
-  constexpr int KB_PER_CHUNK = KCHUNK / TK;
-
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    for (int s = 0; s < NST; ++s) {
-      mbar_init(smem_u32(&bars[s]), 1);
-      mbar_init(smem_u32(&bars[NST + s]), 1);
-    }
-    mbar_init(smem_u32(&bars[2 * NST]), 1);
-    mbar_init(smem_u32(&bars[2 * NST + 1]), 256);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                 ::"r"(smem_u32(tmem_slot)), "r"(512));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-
-  if (warp == 0 && lane == 0) {
-    // ---- TMA producer ----
-    for (int kb = 0; kb < p.nkb; ++kb) {
-      const int s = kb % NST;
-      if (kb >= NST && !mbar_wait(smem_u32(&bars[NST + s]), ((kb / NST) - 1) & 1)) {
-        atomicExch(&abort_flag, 1);
-        break;
-      }
-      if (abort_flag) break;
-      const uint32_t full = smem_u32(&bars[s]);
-      mbar_expect_tx(full, STAGE_BYTES);
-      unsigned char* st = base + s * STAGE_BYTES;
-      for (int q = 0; q < NSLICE; ++q) {
-        tma_load_2d(smem_u32(st + q * TILE_BYTES), &tmA, full, kb * TK, static_cast<int>(q * p.Mp + m0));
-        tma_load_2d(smem_u32(st + (NSLICE + q) * TILE_BYTES), &tmB, full, kb * TK,
-                    static_cast<int>(q * p.Np + n0));
-      }
-    }
-  } else if (warp == 1 && lane == 0) {
-    // ---- MMA issuer ----
-    int kb = 0;
-    for (int c = 0; c < nchunks && !abort_flag; ++c) {
-      if (c > 0 && !mbar_wait(smem_u32(&bars[2 * NST + 1]), (c - 1) & 1)) {
-        atomicExch(&abort_flag, 1);
-        break;
-      }
-      tc_fence_after();
-      const int kb_end = min(p.nkb, (c + 1) * KB_PER_CHUNK);
-      bool first = true;
-      for (; kb < kb_end; ++kb) {
-        const int s = kb % NST;
-        if (!mbar_wait(smem_u32(&bars[s]), (kb / NST) & 1)) { atomicExch(&abort_flag, 1); break; }
-        tc_fence_after();
-        const uint32_t st = smem_u32(base + s * STAGE_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < TK / 16; ++kk) {
-          // 32 bytes per 16-element K step inside the swizzled rows
-          const uint32_t koff = kk * 32;
-          // Groups of equal weight live at TMEM columns 0 (S1S1), 128 (S1S2 + S2S1)
-          // and 256 (S1S3 + S2S2 + S3S1).  B slices 1 and 2 are adjacent in shared
-          // memory, so A_p x [B1 | B2] is one N = 256 MMA into groups p and p+1.
-          const uint32_t init = (first && kk == 0) ? 0u : 1u;
-          const uint64_t a1 = sdesc(st + 0 * TILE_BYTES + koff);
-          const uint64_t a2 = sdesc(st + 1 * TILE_BYTES + koff);
-          const uint64_t a3 = sdesc(st + 2 * TILE_BYTES + koff);
-          const uint64_t b12 = sdesc(st + (NSLICE + 0) * TILE_BYTES + koff);
-          const uint64_t b1 = b12;
-          const uint64_t b3 = sdesc(st + (NSLICE + 2) * TILE_BYTES + koff);
-          umma(tmem + 0 * TN, a1, b12, IDESC256, init);  // S1 x [S1|S2] -> groups 0, 1
-          umma(tmem + 2 * TN, a1, b3, IDESC128, init);   // S1 x S3      -> group 2
-          umma(tmem + 1 * TN, a2, b12, IDESC256, 1u);    // S2 x [S1|S2] -> groups 1, 2
-          umma(tmem + 2 * TN, a3, b1, IDESC128, 1u);     // S3 x S1      -> group 2
-        }
-        umma_commit(smem_u32(&bars[NST + s]));  // stage free once these MMAs retire
-        first = false;
-      }
-      umma_commit(smem_u32(&bars[2 * NST]));    // chunk accumulators ready
-    }
-  } else if (warp >= 2) {
-    // ---- epilogue: TMEM -> FP64 accumulators (all K chunks) -> one store of C ----
-    // Two warps per TMEM lane quadrant (warp % 4): each thread owns one row and
-    // 64 of the 128 columns, summing the three groups of every chunk in FP64.
-    const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int row = quad * 32 + lane;
-    double acc[64];
-#pragma unroll
-    for (int j = 0; j < 64; ++j) acc[j] = 0.0;
-    for (int c = 0; c < nchunks; ++c) {
-      if (!mbar_wait(smem_u32(&bars[2 * NST]), c & 1)) { atomicExch(&abort_flag, 1); break; }
-      tc_fence_after();
-#pragma unroll
-      for (int cb = 0; cb < 64; cb += 16) {
-        const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) +
-                               static_cast<uint32_t>(64 * half + cb);
-        uint32_t g[16];
-        tmem_ld16(taddr, g);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[cb + j] += static_cast<double>(__uint_as_float(g[j])) * 0x1p-12;
-        tmem_ld16(taddr + TN, g);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[cb + j] += static_cast<double>(__uint_as_float(g[j])) * 0x1p-23;
-        tmem_ld16(taddr + 2 * TN, g);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[cb + j] += static_cast<double>(__uint_as_float(g[j])) * 0x1p-34;
-      }
-      tc_fence_before();
-      mbar_arrive(smem_u32(&bars[2 * NST + 1]));
-    }
-    // After the last chunk every MMA has retired and every TMA load has been
-    // consumed, so the stage buffers hold the scaled tile T[128][129] for a
-    // store along whichever index of the output is contiguous.
-    double* T = reinterpret_cast<double*>(base);
-    constexpr int LDT = TN + 1;
-    const int64_t m = m0 + row;
-    const double sa = m < p.M ? ldexp(p.alpha, p.ea[m]) : 0.0;
-#pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      const int64_t n = n0 + 64 * half + j;
-      T[row * LDT + 64 * half + j] = n < p.N ? acc[j] * sa * ldexp(1.0, p.eb[n]) : 0.0;
-    }
-    asm volatile("bar.sync 1, 256;\n" ::: "memory");
-    if (!abort_flag) {
-      const int ew = warp - 2;  // 0..7
-      for (int out = 0; out < 2; ++out) {
-        double* O = out == 0 ? p.C : p.C2;
-        if (!O) continue;
-        const Ax& Om = out == 0 ? p.Cm : p.C2m;
-        const Ax& On = out == 0 ? p.Cn : p.C2n;
-        const bool n_contig = On.s_i == 1 && On.inner > 1;
-        for (int q = 0; q < 16; ++q) {
-          double* ptr[4];
-          double val[4];
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            // n-contiguous: warp row r, lanes along columns; otherwise warp column, lanes along rows
-            const int r = n_contig ? ew + 8 * q : 32 * b + lane;
-            const int cc = n_contig ? 32 * b + lane : ew + 8 * q;
-            const int64_t mm = m0 + r, nn = n0 + cc;
-            const bool in = mm < p.M && nn < p.N;
-            ptr[b] = in ? O + Om.off(static_cast<uint32_t>(mm)) + On.off(static_cast<uint32_t>(nn))
-                        : nullptr;
-            val[b] = T[r * LDT + cc];
-          }
-          rmw_store<4>(ptr, val, p.beta);
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (abort_flag && threadIdx.x == 0) atomicExch(p.error, 1);
-  if (warp == 1) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Persistent variant: one CTA per SM walks the tiles (same raster order), so
-// barrier set-up and TMEM allocation happen once, and the producer and the MMA
-// issuer run ahead into the next tile while the epilogue warps store the last
-// one.  TMEM is handed back after each chunk's drain as before; the stores use
-// warp-private transposes (32 rows x 16 columns, XOR-swizzled), so no barrier
-// spans warps and every warp leaves on an abort by a warp-uniform decision.
-constexpr int WBUF_DOUBLES = 32 * 16;
-constexpr int SMEM_BYTES_P = NST * STAGE_BYTES + 8 * WBUF_DOUBLES * 8 + 1024 + 256;
-
 // Tile t in the grouped raster order: logical origins (m0, n0), packed-row origins
 // (pa, pb) and the valid extents (mlim, nlim) of the tile.
 struct TileAt {
   int64_t m0, n0, pa, pb;
   int mlim, nlim;
 };
+template <int TN>
 __device__ __forceinline__ TileAt tile_at(const SplitParams& p, int64_t t) {
   const int64_t nM = p.nMt, nN = p.nNt;
   const int64_t per_group = RASTER_M * nN, group = t / per_group;
@@ -545,22 +464,25 @@ __device__ __forceinline__ TileAt tile_at(const SplitParams& p, int64_t t) {
   return a;
 }
 
+template <class F>
 __global__ void __launch_bounds__(320)
 split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB, SplitParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  double* wbufs = reinterpret_cast<double*>(base + NST * STAGE_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + NST * STAGE_BYTES + 8 * WBUF_DOUBLES * 8);
+  constexpr int TN = F::TN, TK = F::TK, NST = F::NST, STAGE = stage_bytes<F>();
+  constexpr int COLS = TN / 2;  // columns of one epilogue warp
+  double* wbufs = reinterpret_cast<double*>(base + NST * STAGE);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + NST * STAGE + 8 * WBUF_DOUBLES * 8);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NST + 2);
   __shared__ int abort_flag;
   volatile int* abort_v = &abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ntiles = p.nMt * p.nNt;
-  const int nchunks = (p.nkb * TK + KCHUNK - 1) / KCHUNK;
   constexpr int KB_PER_CHUNK = KCHUNK / TK;
+  const int nchunks = (p.nkb + KB_PER_CHUNK - 1) / KB_PER_CHUNK;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -586,7 +508,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
     // ---- TMA producer: every k-block of every tile of this CTA ----
     uint32_t it = 0;
     for (int64_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
-      const TileAt ta = tile_at(p, t);
+      const TileAt ta = tile_at<TN>(p, t);
       for (int kb = 0; kb < p.nkb; ++kb, ++it) {
         const int s = it % NST;
         if (it >= NST && !mbar_wait(smem_u32(&bars[NST + s]), ((it / NST) - 1) & 1)) {
@@ -595,14 +517,10 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
         }
         if (*abort_v) break;
         const uint32_t full = smem_u32(&bars[s]);
-        mbar_expect_tx(full, STAGE_BYTES);
-        unsigned char* st = base + s * STAGE_BYTES;
-        for (int q = 0; q < NSLICE; ++q) {
-          tma_load_2d(smem_u32(st + q * TILE_BYTES), &tmA, full, kb * TK,
-                      static_cast<int>(q * p.Mp + ta.pa));
-          tma_load_2d(smem_u32(st + (NSLICE + q) * TILE_BYTES), &tmB, full, kb * TK,
-                      static_cast<int>(q * p.Np + ta.pb));
-        }
+        mbar_expect_tx(full, STAGE);
+        unsigned char* st = base + s * STAGE;
+        tma_load_3d(smem_u32(st), &tmA, full, kb * TK, static_cast<int>(ta.pa), 0);
+        tma_load_3d(smem_u32(st + a_bytes<F>()), &tmB, full, kb * TK, static_cast<int>(ta.pb), 0);
       }
     }
   } else if (warp == 1 && lane == 0) {
@@ -622,21 +540,11 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
           const int s = it % NST;
           if (!mbar_wait(smem_u32(&bars[s]), (it / NST) & 1)) { atomicExch(&abort_flag, 1); break; }
           tc_fence_after();
-          const uint32_t st = smem_u32(base + s * STAGE_BYTES);
+          const uint32_t st = smem_u32(base + s * STAGE);
 #pragma unroll
-          for (int kk = 0; kk < TK / 16; ++kk) {
-            const uint32_t koff = kk * 32;
-            const uint32_t init = (first && kk == 0) ? 0u : 1u;
-            const uint64_t a1 = sdesc(st + 0 * TILE_BYTES + koff);
-            const uint64_t a2 = sdesc(st + 1 * TILE_BYTES + koff);
-            const uint64_t a3 = sdesc(st + 2 * TILE_BYTES + koff);
-            const uint64_t b12 = sdesc(st + (NSLICE + 0) * TILE_BYTES + koff);
-            const uint64_t b3 = sdesc(st + (NSLICE + 2) * TILE_BYTES + koff);
-            umma(tmem + 0 * TN, a1, b12, IDESC256, init);  // S1 x [S1|S2] -> groups 0, 1
-            umma(tmem + 2 * TN, a1, b3, IDESC128, init);   // S1 x S3      -> group 2
-            umma(tmem + 1 * TN, a2, b12, IDESC256, 1u);    // S2 x [S1|S2] -> groups 1, 2
-            umma(tmem + 2 * TN, a3, b12, IDESC128, 1u);    // S3 x S1      -> group 2
-          }
+          for (int kk = 0; kk < TK; kk += KPAD)
+            if (kb * TK + kk < p.Kp)  // the last k-block may be a half one
+              umma_digits<F, 0>(tmem, st + kk, st + a_bytes<F>() + kk, first && kk == 0);
           umma_commit(smem_u32(&bars[NST + s]));
           first = false;
         }
@@ -653,46 +561,45 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
     uint32_t q = 0;
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
       if (__any_sync(0xffffffffu, *abort_v != 0)) break;
-      const TileAt ta = tile_at(p, t);
+      const TileAt ta = tile_at<TN>(p, t);
       const int64_t m0 = ta.m0, n0 = ta.n0;
-      double acc[64];
+      double acc[COLS];  // in units of the fourth group
 #pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] = 0.0;
+      for (int j = 0; j < COLS; ++j) acc[j] = 0.0;
       bool ok = true;
       for (int c = 0; c < nchunks; ++c, ++q) {
         const bool got = mbar_wait(smem_u32(&bars[2 * NST]), q & 1);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
-        for (int cb = 0; cb < 64; cb += 16) {
+        for (int cb = 0; cb < COLS; cb += 8) {
           const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) +
-                                 static_cast<uint32_t>(64 * half + cb);
-          uint32_t g[16];
-          tmem_ld16(taddr, g);
+                                 static_cast<uint32_t>(COLS * half + cb);
+          int g[F::NG][8];
+#pragma unroll
+          for (int w = 0; w < F::NG; ++w) tmem_ld8(taddr + w * TN, g[w]);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[cb + j] += static_cast<double>(__uint_as_float(g[j])) * 0x1p-12;
-          tmem_ld16(taddr + TN, g);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) acc[cb + j] += static_cast<double>(__uint_as_float(g[j])) * 0x1p-23;
-          tmem_ld16(taddr + 2 * TN, g);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) acc[cb + j] += static_cast<double>(__uint_as_float(g[j])) * 0x1p-34;
+          for (int j = 0; j < 8; ++j) {
+            double x = static_cast<double>(combine4(g[0][j], g[1][j], g[2][j], g[3][j]));
+            if constexpr (F::NG == 8)
+              x = fma(static_cast<double>(combine4(g[4][j], g[5][j], g[6][j], g[7][j])), 0x1p-32, x);
+            acc[cb + j] += x;
+          }
         }
         tc_fence_before();
         mbar_arrive(smem_u32(&bars[2 * NST + 1]));  // TMEM free: the next chunk may start
       }
       if (!ok) { atomicExch(&abort_flag, 1); break; }
-      // store this warp's 32 rows x 64 columns (the MMA issuer is already on the next tile).
+      // store this warp's 32 rows x COLS columns (the MMA issuer is already on the next tile).
       // The offset of a row belongs to the lane of that row; the offset and the
       // power-of-two scale of a column are computed by one lane per group of 32 (or 16)
       // columns; both reach the lanes that store an element through warp shuffles
       // (offset -1: outside the output).
       const int64_t m = m0 + row;
       const bool mv = row < ta.mlim;
-      const double sa = mv ? ldexp(p.alpha, p.ea[ta.pa + row]) : 0.0;
+      // acc counts 2^-36: digit 0 weighs 2^-6 in each operand, the fourth group 2^-24 of the first
+      const double sa = mv ? row_scale(p.alpha, p.ea[ta.pa + row], 18) : 0.0;
       const int64_t rowoff = mv ? p.Cm.off(static_cast<uint32_t>(m)) : -1;
       const int64_t rowoff2 = (mv && p.C2) ? p.C2m.off(static_cast<uint32_t>(m)) : -1;
       if (m_major && !p.C2 && p.beta != 0.0) {
@@ -700,13 +607,13 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
         // values of the next group of four columns are loaded before the current group
         // is written (the elements of one output tile are distinct, so the loads may
         // pass the stores), keeping two groups of loads in flight per lane.
-        int64_t colL[2];
-        double scL[2];
+        int64_t colL[COLS / 32];
+        double scL[COLS / 32];
 #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-          const int jl = 64 * half + 32 * h2 + lane;
+        for (int h2 = 0; h2 < COLS / 32; ++h2) {
+          const int jl = COLS * half + 32 * h2 + lane;
           colL[h2] = jl < ta.nlim ? p.Cn.off(static_cast<uint32_t>(n0 + jl)) : -1;
-          scL[h2] = jl < ta.nlim ? pow2i(p.eb[ta.pb + jl]) : 0.0;
+          scL[h2] = jl < ta.nlim ? row_scale(1.0, p.eb[ta.pb + jl], 18) : 0.0;
         }
         auto fetch = [&](int g, double* (&ptr)[4], double (&val)[4], double (&old)[4]) {
           const int h2 = g >> 3, j0 = (g & 7) * 4;
@@ -724,14 +631,14 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
         double vc[4], oc[4];
         fetch(0, pc, vc, oc);
 #pragma unroll
-        for (int g = 0; g < 16; ++g) {
+        for (int g = 0; g < COLS / 4; ++g) {
           double* pn[4];
           double vn[4], on[4];
-          if (g + 1 < 16) fetch(g + 1, pn, vn, on);
+          if (g + 1 < COLS / 4) fetch(g + 1, pn, vn, on);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if (pc[j]) *pc[j] = vc[j] + p.beta * oc[j];
-          if (g + 1 < 16) {
+          if (g + 1 < COLS / 4) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) { pc[j] = pn[j]; vc[j] = vn[j]; oc[j] = on[j]; }
           }
@@ -739,10 +646,10 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
       } else if (m_major) {
         // lanes are consecutive rows: store column by column straight from registers
 #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
-          const int jl = 64 * half + 32 * h2 + lane;  // this lane's column of the group
+        for (int h2 = 0; h2 < COLS / 32; ++h2) {
+          const int jl = COLS * half + 32 * h2 + lane;  // this lane's column of the group
           const int64_t colL = jl < ta.nlim ? p.Cn.off(static_cast<uint32_t>(n0 + jl)) : -1;
-          const double scL = jl < ta.nlim ? pow2i(p.eb[ta.pb + jl]) : 0.0;
+          const double scL = jl < ta.nlim ? row_scale(1.0, p.eb[ta.pb + jl], 18) : 0.0;
 #pragma unroll
           for (int j0 = 0; j0 < 32; j0 += 4) {
             double* ptr[4];
@@ -758,7 +665,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
             if (p.C2) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const int jc = 64 * half + 32 * h2 + j0 + j;
+                const int jc = COLS * half + 32 * h2 + j0 + j;
                 ptr[j] = (rowoff2 >= 0 && jc < ta.nlim)
                              ? p.C2 + rowoff2 + p.C2n.off(static_cast<uint32_t>(n0 + jc)) : nullptr;
               }
@@ -771,12 +678,12 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
         // buffer), pipelined like the row-major case: the old values of the next four
         // rows are loaded before the current four are written.
 #pragma unroll
-        for (int piece = 0; piece < 4; ++piece) {
+        for (int piece = 0; piece < COLS / 16; ++piece) {
           const int cc = lane & 15;
-          const int jn = 64 * half + 16 * piece + cc;
+          const int jn = COLS * half + 16 * piece + cc;
           const int64_t nn = n0 + jn;
           const int64_t cn = jn < ta.nlim ? p.Cn.off(static_cast<uint32_t>(nn)) : -1;
-          const double scL = jn < ta.nlim ? pow2i(p.eb[ta.pb + jn]) : 0.0;
+          const double scL = jn < ta.nlim ? row_scale(1.0, p.eb[ta.pb + jn], 18) : 0.0;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const double sc = __shfl_sync(0xffffffffu, scL, j);
@@ -815,12 +722,12 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
       } else {
         // 16-column pieces through the warp's buffer; lanes then run along columns
 #pragma unroll
-        for (int piece = 0; piece < 4; ++piece) {
+        for (int piece = 0; piece < COLS / 16; ++piece) {
           const int cc = lane & 15;  // this lane's column within the piece
-          const int jn = 64 * half + 16 * piece + cc;
+          const int jn = COLS * half + 16 * piece + cc;
           const int64_t nn = n0 + jn;
           const int64_t cn = jn < ta.nlim ? p.Cn.off(static_cast<uint32_t>(nn)) : -1;
-          const double scL = jn < ta.nlim ? pow2i(p.eb[ta.pb + jn]) : 0.0;
+          const double scL = jn < ta.nlim ? row_scale(1.0, p.eb[ta.pb + jn], 18) : 0.0;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const double sc = __shfl_sync(0xffffffffu, scL, j);
@@ -884,17 +791,21 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// 2-D map over packed slices [3*Rp][Kp] FP16, box TK (k) x 128 (rows), rows of
-// ROW_BYTES swizzled like the MMA descriptors expect.
-CUtensorMap make_map(void* base, int64_t rows, int64_t Kp) {
+// 3-D map over the digit planes [digits][Rp][Kp], box tk (k) x rows x digits, rows of
+// tk bytes swizzled like the MMA descriptors expect.  Rows and k beyond the operand
+// read zero.
+CUtensorMap make_map(void* base, int digits, int64_t Rp, int64_t Kp, int tk, int rows) {
   CUtensorMap m;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(Kp * 2)};
-  const cuuint32_t box[2] = {TK, 128};
-  const cuuint32_t es[2] = {1, 1};
-  CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, es,
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(Rp),
+                              static_cast<cuuint64_t>(digits)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(Kp * Rp)};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(tk), static_cast<cuuint32_t>(rows),
+                             static_cast<cuuint32_t>(digits)};
+  const cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           ROW_BYTES == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           tk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                           : tk == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw Error(ERR_CUDA, "cuTensorMapEncodeTiled failed");
   return m;
@@ -902,23 +813,26 @@ CUtensorMap make_map(void* base, int64_t rows, int64_t Kp) {
 
 inline int64_t rup(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
+int digits_of(const Contraction& g) { return g.digits == 7 ? 7 : 4; }
+
 struct Layout2 {
   int64_t Mp, Np, Kp;
   size_t a_bytes, b_bytes, meta_bytes;
 };
 Layout2 layout_of(const Contraction& g) {
+  const int D = digits_of(g);
   Layout2 L;
   L.Mp = rup(g.M, TM);
-  L.Np = rup(g.N, TN);
-  L.Kp = rup(std::max<int64_t>(g.K, 1), TK);
-  L.a_bytes = rup(static_cast<int64_t>(NSLICE * L.Mp * L.Kp * 2), 1024);
-  L.b_bytes = rup(static_cast<int64_t>(NSLICE * L.Np * L.Kp * 2), 1024);
+  L.Np = rup(g.N, tile_n(D));
+  L.Kp = rup(std::max<int64_t>(g.K, 1), KPAD);
+  L.a_bytes = rup(static_cast<int64_t>(D * L.Mp * L.Kp), 1024);
+  L.b_bytes = rup(static_cast<int64_t>(D * L.Np * L.Kp), 1024);
   L.meta_bytes = rup((L.Mp + L.Np) * (8 + 4), 1024);
   return L;
 }
 
-void pack(const View& v, bool rows_are_m, const Contraction& g, int64_t R, int64_t Rp,
-          int64_t Kp, __half* dst, unsigned long long* rmax, int* rexp, cudaStream_t s) {
+PackArgs pack_args(const View& v, bool rows_are_m, const Contraction& g, int64_t R, int64_t Rp,
+                   int64_t Kp, void* dst, unsigned long long* rmax, int* rexp) {
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
   const int64_t Ki = g.Ki > 0 ? g.Ki : std::max<int64_t>(g.K, 1);
   PackArgs a;
@@ -933,14 +847,33 @@ void pack(const View& v, bool rows_are_m, const Contraction& g, int64_t R, int64
     a.r_contig = (v.s_ci == 1 && v.s_ri != 1) ? 1 : 0;
   }
   a.R = R; a.K = g.K; a.Rp = Rp; a.Kp = Kp;
-  a.rmax = rmax; a.rexp = rexp; a.dst = dst;
+  a.rmax = rmax; a.rexp = rexp; a.dst = static_cast<int8_t*>(dst);
   if (Rp % PR || Kp % 16) throw Error(ERR_BAD_SHAPE, "gemm_split: packed extents not tiled");
-  CC_CHECK(cudaMemsetAsync(rmax, 0, R * sizeof(unsigned long long), s));
-  const int64_t strips = (Rp / PR) * ((Kp + PKT * PSTRIP - 1) / (PKT * PSTRIP));
-  const int64_t tiles = (Rp / PR) * ((Kp + PKT - 1) / PKT);
-  pack_max_kernel<<<static_cast<unsigned>(std::min<int64_t>(strips, 148 * 8)), PTHREADS, 0, s>>>(a);
+  return a;
+}
+
+// Row maxima and digits of one or two operands.  Their rmax arrays are one block of
+// `rows` entries starting at a.rmax (cleared here).
+void pack(const PackArgs& a, const PackArgs* b, int64_t rows, int digits, cudaStream_t s) {
+  CC_CHECK(cudaMemsetAsync(a.rmax, 0, rows * sizeof(unsigned long long), s));
+  PackPair pp;
+  pp.op[0] = a;
+  pp.op[1] = b ? *b : a;
+  // strips of k for the maxima: the longest of 128 .. 1024 that gives 148 x 6 work items
+  int64_t kstrip = 1024;
+  auto strips = [&](const PackArgs& x) { return (x.Rp / PR) * ((x.K + kstrip - 1) / kstrip); };
+  while (kstrip > 128 && strips(a) + (b ? strips(*b) : 0) < 148 * 6) kstrip /= 2;
+  auto tiles = [](const PackArgs& x) { return (x.Rp / PR) * ((x.Kp + PKT - 1) / PKT); };
+  pp.first = strips(a);
+  pp.total = pp.first + (b ? strips(*b) : 0);
+  pack_max_kernel<<<static_cast<unsigned>(std::min<int64_t>(pp.total, 148 * 8)), PTHREADS, 0, s>>>(
+      pp, static_cast<int>(kstrip));
   CC_LAUNCH_CHECK();
-  pack_slices_kernel<<<static_cast<unsigned>(std::min<int64_t>(tiles, 148 * 8)), PTHREADS, 0, s>>>(a);
+  pp.first = tiles(a);
+  pp.total = pp.first + (b ? tiles(*b) : 0);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(pp.total, 148 * 8));
+  if (digits == 7) pack_digits_kernel<7><<<grid, PTHREADS, 0, s>>>(pp);
+  else pack_digits_kernel<4><<<grid, PTHREADS, 0, s>>>(pp);
   CC_LAUNCH_CHECK();
   g_pack_launches.fetch_add(2);
 }
@@ -961,10 +894,11 @@ size_t panel_bytes() {
 }
 
 int64_t panel_len(const Contraction& g) {
-  const int64_t per_k = 2 * NSLICE * (rup(g.M, TM) + rup(g.N, TN));  // bytes per k
+  const int D = digits_of(g);
+  const int64_t per_k = D * (rup(g.M, TM) + rup(g.N, tile_n(D)));  // bytes per k
   int64_t P = static_cast<int64_t>(panel_bytes()) / per_k;
   if (P >= KCHUNK) P = P / KCHUNK * KCHUNK;
-  else P = std::max<int64_t>(TK, P / TK * TK);
+  else P = std::max<int64_t>(2 * KPAD, P / KPAD * KPAD);
   return P;
 }
 
@@ -1029,8 +963,8 @@ SplitPackedB split_pack_b(const Contraction& g, void* dst, cudaStream_t s) {
   b.slices = p;
   auto* bmax = reinterpret_cast<unsigned long long*>(p + L.b_bytes);
   b.exps = reinterpret_cast<int*>(p + L.b_bytes + rup(L.Np * 8, 1024));
-  b.N = g.N; b.K = g.K; b.Np = L.Np; b.Kp = L.Kp;
-  pack(g.B, false, g, g.N, L.Np, L.Kp, static_cast<__half*>(b.slices), bmax, b.exps, s);
+  b.N = g.N; b.K = g.K; b.Np = L.Np; b.Kp = L.Kp; b.digits = digits_of(g);
+  pack(pack_args(g.B, false, g, g.N, L.Np, L.Kp, b.slices, bmax, b.exps), nullptr, g.N, b.digits, s);
   return b;
 }
 
@@ -1059,104 +993,104 @@ void gemm_split(const Contraction& g, cudaStream_t s, SplitScratch& ws) {
 
 namespace {
 
-// Persistent tile loop by default; CC4S_SPLIT_PERSISTENT=0 selects one tile per CTA.
-bool persistent_mode() {
-  static const bool persistent = [] {
-    const char* e = std::getenv("CC4S_SPLIT_PERSISTENT");
-    return !(e && e[0] == '0');
-  }();
-  return persistent;
-}
-
-void launch_persistent(const CUtensorMap& ta, const CUtensorMap& tb, const SplitParams& sp,
-                       int64_t tiles, cudaStream_t s) {
-  static int sms = 0;
-  if (!sms) {
+template <class F>
+void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, SplitParams sp, cudaStream_t s) {
+  static std::atomic<int> sms{0};
+  int n = sms.load();
+  if (!n) {
     int dev = 0;
     CC_CHECK(cudaGetDevice(&dev));
-    CC_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CC_CHECK(cudaFuncSetAttribute(split_kernel_persistent,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES_P));
+    CC_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    CC_CHECK(cudaFuncSetAttribute(split_kernel_persistent<F>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<F>()));
+    sms.store(n);
   }
-  dim3 grid(static_cast<unsigned>(std::min<int64_t>(tiles, sms)));
-  split_kernel_persistent<<<grid, 320, SMEM_BYTES_P, s>>>(ta, tb, sp);
+  sp.nkb = static_cast<int>((sp.Kp + F::TK - 1) / F::TK);
+  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(sp.nMt * sp.nNt, n)));
+  split_kernel_persistent<F><<<grid, 320, smem_bytes<F>(), s>>>(ta, tb, sp);
+  CC_LAUNCH_CHECK();
+  g_split_launches.fetch_add(1);
 }
 
-void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const SplitPackedB* pb) {
-  const Layout2 L = layout_of(g);
-  // with a pre-packed B the scratch holds A and the metadata only
-  const size_t need = L.a_bytes + (pb ? 0 : L.b_bytes) + L.meta_bytes;
-  if (need > ws.bytes) throw Error(ERR_OUT_OF_MEMORY, "gemm_split: scratch too small");
-  if (L.Mp * NSLICE >= (int64_t(1) << 31) || L.Np * NSLICE >= (int64_t(1) << 31) || L.Kp >= (int64_t(1) << 31))
-    throw Error(ERR_BAD_SHAPE, "gemm_split: extent too large");
-  unsigned char* p = static_cast<unsigned char*>(ws.p);
-  __half* Apk = reinterpret_cast<__half*>(p);
-  __half* Bpk = reinterpret_cast<__half*>(p + L.a_bytes);
-  unsigned char* meta = p + L.a_bytes + (pb ? 0 : L.b_bytes);
-  auto* amax = reinterpret_cast<unsigned long long*>(meta);
-  auto* bmax = amax + L.Mp;
-  int* aexp = reinterpret_cast<int*>(bmax + L.Np);
-  int* bexp = aexp + L.Mp;
-  pack(g.A, true, g, g.M, L.Mp, L.Kp, Apk, amax, aexp, s);
-  if (pb) {   // B sliced before, by split_pack_b, for this N, K and padding
-    if (pb->N != g.N || pb->K != g.K || pb->Np != L.Np || pb->Kp != L.Kp)
-      throw Error(ERR_INVALID_ARGUMENT, "gemm_split: pre-packed B of another shape");
-    Bpk = static_cast<__half*>(pb->slices);
-    bexp = pb->exps;
-  } else {
-    pack(g.B, false, g, g.N, L.Np, L.Kp, Bpk, bmax, bexp, s);
-  }
-  const CUtensorMap ta = make_map(Apk, NSLICE * L.Mp, L.Kp);
-  const CUtensorMap tb = make_map(Bpk, NSLICE * L.Np, L.Kp);
+// The output side of a contraction and the runs of its packed rows -> one launch.
+void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t Ap,
+            const SplitRuns& ar, int64_t nra, void* Bpk, const int* eb, int64_t Bp,
+            const SplitRuns& br, int64_t nrb, int64_t Kp, cudaStream_t s, SplitScratch& ws) {
+  const int tn = tile_n(digits), tk = digits == 7 ? Form<7>::TK : Form<4>::TK;
+  const CUtensorMap ta = make_map(Apk, digits, Ap, Kp, tk, TM);
+  const CUtensorMap tb = make_map(Bpk, digits, Bp, Kp, tk, tn);
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
   SplitParams sp;
-  sp.M = g.M; sp.N = g.N; sp.K = g.K; sp.Mp = L.Mp; sp.Np = L.Np;
-  sp.nkb = static_cast<int>(L.Kp / TK);
+  sp.M = g.M; sp.N = g.N; sp.K = g.K; sp.Kp = Kp; sp.nkb = 0;
   sp.Cm = mkax(Mi, g.C.s_ro, g.C.s_ri);
   sp.Cn = mkax(Ni, g.C.s_co, g.C.s_ci);
   sp.C2m = mkax(Mi, g.C2.s_ro, g.C2.s_ri);
   sp.C2n = mkax(Ni, g.C2.s_co, g.C2.s_ci);
   sp.C = g.C.p; sp.C2 = g.C2.p;
   sp.alpha = g.alpha; sp.beta = g.beta;
-  sp.ea = aexp; sp.eb = bexp;
+  sp.ea = ea; sp.eb = eb;
   sp.error = ws.error;
-  sp.a_run = g.M; sp.a_stride = 0; sp.a_base = 0; sp.a_tiles = L.Mp / TM; sp.nMt = L.Mp / TM;
-  sp.b_run = g.N; sp.b_stride = 0; sp.b_base = 0; sp.b_tiles = L.Np / TN; sp.nNt = L.Np / TN;
-  const int64_t tiles = (L.Np / TN) * (L.Mp / TM);
-  if (tiles >= (int64_t(1) << 31)) throw Error(ERR_BAD_SHAPE, "gemm_split: too many tiles");
-  if (persistent_mode()) {
-    launch_persistent(ta, tb, sp, tiles, s);
+  sp.a_run = ar.run; sp.a_stride = ar.stride; sp.a_base = ar.base;
+  sp.a_tiles = (ar.run + TM - 1) / TM; sp.nMt = nra * sp.a_tiles;
+  sp.b_run = br.run; sp.b_stride = br.stride; sp.b_base = br.base;
+  sp.b_tiles = (br.run + tn - 1) / tn; sp.nNt = nrb * sp.b_tiles;
+  if (sp.nMt * sp.nNt >= (int64_t(1) << 31) || Ap >= (int64_t(1) << 31) ||
+      Bp >= (int64_t(1) << 31) || Kp >= (int64_t(1) << 31))
+    throw Error(ERR_BAD_SHAPE, "gemm_split: extent too large");
+  if (digits == 7) launch_form<Form<7>>(ta, tb, sp, s);
+  else launch_form<Form<4>>(ta, tb, sp, s);
+}
+
+void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const SplitPackedB* pb) {
+  const Layout2 L = layout_of(g);
+  const int D = digits_of(g);
+  // with a pre-packed B the scratch holds A and the metadata only
+  const size_t need = L.a_bytes + (pb ? 0 : L.b_bytes) + L.meta_bytes;
+  if (need > ws.bytes) throw Error(ERR_OUT_OF_MEMORY, "gemm_split: scratch too small");
+  unsigned char* p = static_cast<unsigned char*>(ws.p);
+  void* Apk = p;
+  void* Bpk = p + L.a_bytes;
+  unsigned char* meta = p + L.a_bytes + (pb ? 0 : L.b_bytes);
+  auto* amax = reinterpret_cast<unsigned long long*>(meta);
+  auto* bmax = amax + L.Mp;
+  int* aexp = reinterpret_cast<int*>(bmax + L.Np);
+  int* bexp = aexp + L.Mp;
+  const PackArgs pa = pack_args(g.A, true, g, g.M, L.Mp, L.Kp, Apk, amax, aexp);
+  if (pb) {   // B sliced before, by split_pack_b, for this N, K and padding
+    if (pb->N != g.N || pb->K != g.K || pb->Np != L.Np || pb->Kp != L.Kp || pb->digits != D)
+      throw Error(ERR_INVALID_ARGUMENT, "gemm_split: pre-packed B of another shape");
+    Bpk = pb->slices;
+    bexp = pb->exps;
+    pack(pa, nullptr, L.Mp, D, s);
   } else {
-    static bool configured = false;
-    if (!configured) {
-      CC_CHECK(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-      configured = true;
-    }
-    dim3 grid(static_cast<unsigned>(tiles));
-    split_kernel<<<grid, 320, SMEM_BYTES, s>>>(ta, tb, sp);
+    const PackArgs pbk = pack_args(g.B, false, g, g.N, L.Np, L.Kp, Bpk, bmax, bexp);
+    pack(pa, &pbk, L.Mp + L.Np, D, s);
   }
-  CC_LAUNCH_CHECK();
-  g_split_launches.fetch_add(1);
+  SplitRuns ar, br;
+  ar.run = g.M;
+  br.run = g.N;
+  launch(g, D, Apk, aexp, L.Mp, ar, 1, Bpk, bexp, L.Np, br, 1, L.Kp, s, ws);
 }
 
 }  // namespace
-size_t split_operand_bytes(int64_t R, int64_t K) {
-  const int64_t Rp = rup(std::max<int64_t>(R, 1), TM), Kp = rup(std::max<int64_t>(K, 1), TK);
-  return static_cast<size_t>(rup(NSLICE * Rp * Kp * 2, 1024) + rup(Rp * 8, 1024) +
+size_t split_operand_bytes(int64_t R, int64_t K, int digits) {
+  const int64_t Rp = rup(std::max<int64_t>(R, 1), TM), Kp = rup(std::max<int64_t>(K, 1), KPAD);
+  return static_cast<size_t>(rup(digits * Rp * Kp, 1024) + rup(Rp * 8, 1024) +
                              rup(Rp * 4, 1024));
 }
 
 SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_t s_ro,
-                                int64_t s_ri, int64_t K, int64_t s_k, void* dst, cudaStream_t s) {
+                                int64_t s_ri, int64_t K, int64_t s_k, void* dst, cudaStream_t s,
+                                int digits) {
   if (R <= 0 || K <= 0) throw Error(ERR_BAD_SHAPE, "split_pack_operand: empty operand");
   SplitOperand o;
-  o.R = R; o.K = K;
+  o.R = R; o.K = K; o.digits = digits;
   o.Rp = rup(R, TM);
-  o.Kp = rup(K, TK);
-  if (o.Rp * NSLICE >= (int64_t(1) << 31) || o.Kp >= (int64_t(1) << 31))
+  o.Kp = rup(K, KPAD);
+  if (o.Rp >= (int64_t(1) << 31) || o.Kp >= (int64_t(1) << 31))
     throw Error(ERR_BAD_SHAPE, "split_pack_operand: extent too large");
   unsigned char* p = static_cast<unsigned char*>(dst);
-  const int64_t sb = rup(NSLICE * o.Rp * o.Kp * 2, 1024);
+  const int64_t sb = rup(digits * o.Rp * o.Kp, 1024);
   o.slices = p;
   auto* rmax = reinterpret_cast<unsigned long long*>(p + sb);
   o.exps = reinterpret_cast<int*>(p + sb + rup(o.Rp * 8, 1024));
@@ -1164,7 +1098,7 @@ SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_
   g.M = R; g.Mi = Ri; g.K = K;
   g.A.p = const_cast<double*>(src);
   g.A.s_ro = s_ro; g.A.s_ri = s_ri; g.A.s_co = 0; g.A.s_ci = s_k;
-  pack(g.A, true, g, R, o.Rp, o.Kp, static_cast<__half*>(o.slices), rmax, o.exps, s);
+  pack(pack_args(g.A, true, g, R, o.Rp, o.Kp, o.slices, rmax, o.exps), nullptr, R, digits, s);
   return o;
 }
 
@@ -1172,9 +1106,7 @@ void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const Spl
                           const SplitOperand& B, const SplitRuns& br, cudaStream_t s,
                           SplitScratch& ws) {
   if (g.M <= 0 || g.N <= 0) return;
-  if (!persistent_mode())
-    throw Error(ERR_UNSUPPORTED, "gemm_split_prepacked: needs the persistent kernel");
-  if (A.K != g.K || B.K != g.K || A.Kp != B.Kp)
+  if (A.K != g.K || B.K != g.K || A.Kp != B.Kp || A.digits != B.digits)
     throw Error(ERR_INVALID_ARGUMENT, "gemm_split_prepacked: operands of another K");
   // every packed row that a valid logical row reads lies inside the operand
   auto check = [](const SplitRuns& r, int64_t X, int64_t R, const char* what) {
@@ -1189,29 +1121,8 @@ void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const Spl
     return nr;
   };
   const int64_t nra = check(ar, g.M, A.R, "A"), nrb = check(br, g.N, B.R, "B");
-  const CUtensorMap ta = make_map(A.slices, NSLICE * A.Rp, A.Kp);
-  const CUtensorMap tb = make_map(B.slices, NSLICE * B.Rp, B.Kp);
-  const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
-  SplitParams sp;
-  sp.M = g.M; sp.N = g.N; sp.K = g.K; sp.Mp = A.Rp; sp.Np = B.Rp;
-  sp.nkb = static_cast<int>(A.Kp / TK);
-  sp.Cm = mkax(Mi, g.C.s_ro, g.C.s_ri);
-  sp.Cn = mkax(Ni, g.C.s_co, g.C.s_ci);
-  sp.C2m = mkax(Mi, g.C2.s_ro, g.C2.s_ri);
-  sp.C2n = mkax(Ni, g.C2.s_co, g.C2.s_ci);
-  sp.C = g.C.p; sp.C2 = g.C2.p;
-  sp.alpha = g.alpha; sp.beta = g.beta;
-  sp.ea = A.exps; sp.eb = B.exps;
-  sp.error = ws.error;
-  sp.a_run = ar.run; sp.a_stride = ar.stride; sp.a_base = ar.base;
-  sp.a_tiles = (ar.run + TM - 1) / TM; sp.nMt = nra * sp.a_tiles;
-  sp.b_run = br.run; sp.b_stride = br.stride; sp.b_base = br.base;
-  sp.b_tiles = (br.run + TN - 1) / TN; sp.nNt = nrb * sp.b_tiles;
-  const int64_t tiles = sp.nMt * sp.nNt;
-  if (tiles >= (int64_t(1) << 31)) throw Error(ERR_BAD_SHAPE, "gemm_split_prepacked: too many tiles");
-  launch_persistent(ta, tb, sp, tiles, s);
-  CC_LAUNCH_CHECK();
-  g_split_launches.fetch_add(1);
+  launch(g, A.digits, A.slices, A.exps, A.Rp, ar, nra, B.slices, B.exps, B.Rp, br, nrb, A.Kp, s,
+         ws);
 }
 
 }  // namespace cc4s_b200

@@ -1,16 +1,19 @@
-// Split-precision FP64 contraction on the 5th-generation tensor cores (tcgen05).
+// FP64 contraction on the 5th-generation tensor cores (tcgen05) in integer digits.
 //
-// C = alpha * A B + beta * C with FP64 operands, computed from FP16 slices
-// (Ozaki-style): every row of A (and every column of B) is scaled by a power
-// of two so that its largest element is below 1 and cut into three integer
-// slices of 6, 11 and 11 bits,
-//     a = 2^e (S1 2^-6 + S2 2^-17 + S3 2^-28),
-// each slice an integer stored exactly in FP16.  The six slice products with
-// p + q <= 4 are summed by tcgen05.mma (kind::f16, FP32 accumulation in
-// TMEM) into three groups of equal weight 2^-12, 2^-23 and 2^-34.  The
-// leading group (|S1 S1| <= 2^12) is exact in FP32 over K chunks of 4096;
-// after each chunk the groups are combined in FP64 and added to C.
-// Precision: 28 bits of each operand relative to its row / column maximum.
+// C = alpha * A B + beta * C with FP64 operands (the Ozaki scheme on signed 8-bit
+// integers): every row of A (and every column of B) is scaled by a power of two so that
+// its largest element is below 1 and written in balanced base-256 digits,
+//     a = 2^e 2^-6 (d0 + d1 2^-8 + d2 2^-16 + ...),  -128 <= d <= 127.
+// The digit products d_p d_q are summed exactly by tcgen05.mma (kind::i8, S32
+// accumulation in TMEM) into one group per weight 2^-8(p+q), and the groups are
+// combined in exact 64-bit integers before the one conversion to FP64.
+//   digits = 4 (30 bits of each operand relative to its row / column maximum): the ten
+//     products p + q < 4; the split-precision form.
+//   digits = 7 (54 bits, i.e. FP64's 53 for the largest element of a row): the 34
+//     products p + q < 8.  What is left out is below 2^-63 of the row times the column
+//     maximum, and the sum over k adds no rounding, so the result is at least as close
+//     to the exact one as an FP64 accumulation of more than a few terms.
+// A row or column holding an Inf or NaN gives NaN in all its outputs.
 #pragma once
 
 #include "gemm_f64.cuh"
@@ -35,9 +38,10 @@ size_t gemm_split_scratch_bytes(const Contraction& g);
 // contractions that share B (same N, K and B view), e.g. the ladder's X panel
 // for every block pair of one c range.
 struct SplitPackedB {
-  void* slices = nullptr;  // [3][Np][Kp] FP16
+  void* slices = nullptr;  // [digits][Np][Kp] signed bytes
   int* exps = nullptr;     // [Np] power-of-two column scales
   int64_t N = 0, K = 0, Np = 0, Kp = 0;
+  int digits = 4;
 };
 // Bytes split_pack_b writes (slices, row maxima, exponents).
 size_t split_packed_b_bytes(const Contraction& g);
@@ -52,20 +56,22 @@ SplitPackedB split_pack_b(const Contraction& g, void* dst, cudaStream_t s);
 void gemm_split_packed_b(const Contraction& g, const SplitPackedB& b, cudaStream_t s,
                          SplitScratch& ws);
 
-// An operand sliced once for many contractions: R rows of K elements as three FP16
-// planes [3][Rp][Kp] with one power-of-two exponent per row (the scaling of every
+// An operand sliced once for many contractions: R rows of K elements as digit
+// planes [digits][Rp][Kp] with one power-of-two exponent per row (the scaling of every
 // row over its whole K, as gemm_split slices its operands).
 struct SplitOperand {
   void* slices = nullptr;
   int* exps = nullptr;   // [Rp]
   int64_t R = 0, K = 0, Rp = 0, Kp = 0;
+  int digits = 4;
 };
 // Device bytes of a sliced operand of R rows and K columns.
-size_t split_operand_bytes(int64_t R, int64_t K);
+size_t split_operand_bytes(int64_t R, int64_t K, int digits = 4);
 // Slices the rows of src into dst (device memory of split_operand_bytes bytes):
 // element (r, k) at src[(r / Ri) * s_ro + (r % Ri) * s_ri + k * s_k] (Ri = 0: one level).
 SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_t s_ro,
-                                int64_t s_ri, int64_t K, int64_t s_k, void* dst, cudaStream_t s);
+                                int64_t s_ri, int64_t K, int64_t s_k, void* dst, cudaStream_t s,
+                                int digits = 4);
 // The rows of a contraction inside a sliced operand: logical index x is packed row
 //   base + (x / run) * stride + x % run.
 struct SplitRuns {
@@ -74,13 +80,14 @@ struct SplitRuns {
 // C = alpha A B + beta C (g gives M, N, K, the output views, alpha, beta) with the rows
 // m of A and the columns n of B taken from sliced operands (B sliced by its columns,
 // i.e. its rows are n).  Tiles never straddle a run, so a run shorter than a tile
-// costs a partial tile.  Persistent kernel only.
+// costs a partial tile.
 void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const SplitRuns& ar,
                           const SplitOperand& B, const SplitRuns& br, cudaStream_t s,
                           SplitScratch& ws);
 
 uint64_t split_launch_count();
-// Number of operand-slicing kernel launches issued so far (two per sliced operand).
+// Number of operand-slicing kernel launches issued so far (two per
+// contraction whose operands are sliced in it).
 uint64_t split_pack_launch_count();
 
 }  // namespace cc4s_b200

@@ -176,7 +176,8 @@ void Triples::connected(const ops::TriplesBlock& b, const int64_t X[3], const in
 void Triples::pack_operands(int w, const double* Ac, const double* Bc) {
   const int64_t o = o_, v = v_, n1 = n1_, kc = kc_;
   const int planes = cplx_ ? 2 : 1;
-  const size_t ba = split_operand_bytes(n1 * o, kc), bb = split_operand_bytes(v * n1, kc);
+  const size_t ba = split_operand_bytes(n1 * o, kc, digits_),
+               bb = split_operand_bytes(v * n1, kc, digits_);
   const size_t per = 2 * ba + bb;
   if (!sl_mem_[w]) sl_mem_[w] = take((planes * per + 7) / 8);
   unsigned char* p = reinterpret_cast<unsigned char*>(sl_mem_[w]);
@@ -184,9 +185,9 @@ void Triples::pack_operands(int w, const double* Ac, const double* Bc) {
     const double* A = Ac + pl * ai_;
     const double* B = Bc + pl * bi_;
     Sliced& s = sl_[w][pl];
-    s.A = split_pack_operand(A, n1 * o, 0, 0, kc, kc, 1, p, s_);
-    s.A2 = split_pack_operand(A, o * n1, n1, kc, o * kc, kc, 1, p + ba, s_);
-    s.B = split_pack_operand(B, v * n1, 0, 0, kc, kc, 1, p + 2 * ba, s_);
+    s.A = split_pack_operand(A, n1 * o, 0, 0, kc, kc, 1, p, s_, digits_);
+    s.A2 = split_pack_operand(A, o * n1, n1, kc, o * kc, kc, 1, p + ba, s_, digits_);
+    s.B = split_pack_operand(B, v * n1, 0, 0, kc, kc, 1, p + 2 * ba, s_, digits_);
   }
 }
 
@@ -459,12 +460,19 @@ TriplesOutcome Triples::run(const double* T) {
   if (complete_) complete_intermediates(T);
   concat_operands(T, Vppph_, Vhhhp_, Ac_, Bc_);
   if (complete_) concat_operands(T, Ip_, Ih_, AcM_, BcM_);
-  // split form (the contractions' K = v + o long enough for it): both operands sliced once here
-  const bool packed = precision_ == 3 && kc_ >= 64;
-  if (packed) {
-    pack_operands(0, Ac_, Bc_);
-    if (complete_) pack_operands(1, AcM_, BcM_);
+  // Both operands sliced once here where the contractions' K = v + o is long enough: in
+  // four digits (split precision), or in seven (FP64) once a block of pairs fills tiles.
+  digits_ = kc_ < 64 ? 0 : precision_ == 3 ? 4 : nb * o >= 128 ? 7 : 0;
+  if (digits_) {
+    try {
+      pack_operands(0, Ac_, Bc_);
+      if (complete_) pack_operands(1, AcM_, BcM_);
+    } catch (const Error& e) {
+      if (e.status != ERR_OUT_OF_MEMORY || digits_ != 7) throw;
+      digits_ = 0;  // no room for the digits: the FP64 tensor pipe needs none
+    }
   }
+  const bool packed = digits_ != 0;
   ops::event_record(e1, s_);
   out.setup_seconds += ops::event_ms(e0, e1) * 1e-3;
   const int64_t Lm = nb * o;

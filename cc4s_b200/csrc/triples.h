@@ -126,6 +126,7 @@ class Triples : public Schedule {
     SplitOperand A, A2, B;  // Ac rows (pair, hole), Ac rows (hole, pair), Bc rows (virtual, pair)
   };
   Sliced sl_[2][2];         // [S or M][plane]
+  int digits_ = 0;          // digit form of the sliced operands (0: not sliced)
   double* sl_mem_[2] = {nullptr, nullptr};
   double* ws_ = nullptr;     // reduction partials
   double* slots_ = nullptr;  // two energy sums of every block triple, then their totals

@@ -61,10 +61,9 @@ void gemm(const Contraction& g, cudaStream_t, const GemmScratch&) {
   }
 }
 
-// Emulation of the split-precision contraction: the same row/column scaling,
-// integer slices (6, 11, 11 bits) and the six slice products p + q <= 2
-// (0-based), summed exactly in FP64 (the device sums the leading group exactly
-// in FP32 per 4096-wide chunk; the lower groups differ only below 2^-50 relative).
+// Emulation of the digit-form contraction: the same row/column scaling, balanced
+// base-256 digits and digit products (p + q < 4 of four digits, p + q < 8 of seven), each
+// weight summed exactly as on the device.
 static uint64_t g_split = 0, g_pack = 0;
 uint64_t split_launch_count() { return g_split; }
 uint64_t split_pack_launch_count() { return g_pack; }
@@ -72,58 +71,55 @@ size_t gemm_split_scratch_bytes(const Contraction&) { return 64; }
 
 void gemm_split(const Contraction& g, cudaStream_t, SplitScratch&) {
   ++g_split;
-  g_pack += 4;  // the device slices both operands (two launches each)
+  g_pack += 2;  // the device slices both operands together (two launches)
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
   const int64_t Ki = g.Ki > 0 ? g.Ki : std::max<int64_t>(g.K, 1);
   Ax Am = ax(Mi, g.A.s_ro, g.A.s_ri), Ak = ax(Ki, g.A.s_co, g.A.s_ci);
   Ax Bk = ax(Ki, g.B.s_ro, g.B.s_ri), Bn = ax(Ni, g.B.s_co, g.B.s_ci);
   Ax Cm = ax(Mi, g.C.s_ro, g.C.s_ri), Cn = ax(Ni, g.C.s_co, g.C.s_ci);
   Ax C2m = ax(Mi, g.C2.s_ro, g.C2.s_ri), C2n = ax(Ni, g.C2.s_co, g.C2.s_ci);
-  auto split = [](const std::vector<double>& x, std::vector<double> (&s)[3], int& e) {
+  const int D = g.digits == 7 ? 7 : 4, NG = D == 7 ? 8 : 4;
+  using Digits = std::vector<std::vector<double>>;  // [digit][k]
+  auto split = [&](const std::vector<double>& x, Digits& s, int& e) {
     double m = 0.0;
     for (double v : x) m = std::max(m, std::fabs(v));
     e = 0;
     if (m > 0.0) std::frexp(m, &e);
-    for (auto& v : s) v.assign(x.size(), 0.0);
+    s.assign(D, std::vector<double>(x.size(), 0.0));
     for (size_t k = 0; k < x.size(); ++k) {
-      double y = std::ldexp(x[k], -e) * 64.0;
-      const double s1 = std::nearbyint(y);
-      double t = (y - s1) * 2048.0;
-      const double s2 = std::nearbyint(t);
-      t = (t - s2) * 2048.0;
-      s[0][k] = s1; s[1][k] = s2; s[2][k] = std::nearbyint(t);
+      long long X = std::llrint(std::ldexp(x[k], 8 * D - 2 - e));
+      for (int q = D - 1; q > 0; --q) {
+        const auto d = static_cast<int8_t>(X & 255);
+        s[q][k] = d;
+        X = (X - d) >> 8;
+      }
+      s[0][k] = static_cast<double>(X);
     }
   };
-  std::vector<std::vector<double>> as[3], bs[3];
+  std::vector<Digits> as(g.M), bs(g.N);
   std::vector<int> ea(g.M), eb(g.N);
-  for (auto& v : as) v.resize(g.M);
-  for (auto& v : bs) v.resize(g.N);
   std::vector<double> row(g.K);
   for (int64_t m = 0; m < g.M; ++m) {
     for (int64_t k = 0; k < g.K; ++k) row[k] = g.A.p[Am.off(m) + Ak.off(k)];
-    std::vector<double> s[3];
-    split(row, s, ea[m]);
-    for (int q = 0; q < 3; ++q) as[q][m] = s[q];
+    split(row, as[m], ea[m]);
   }
   for (int64_t n = 0; n < g.N; ++n) {
     for (int64_t k = 0; k < g.K; ++k) row[k] = g.B.p[Bk.off(k) + Bn.off(n)];
-    std::vector<double> s[3];
-    split(row, s, eb[n]);
-    for (int q = 0; q < 3; ++q) bs[q][n] = s[q];
+    split(row, bs[n], eb[n]);
   }
-  const double w[3] = {0x1p-12, 0x1p-23, 0x1p-34};
   for (int64_t m = 0; m < g.M; ++m)
     for (int64_t n = 0; n < g.N; ++n) {
-      double acc[3] = {0, 0, 0};
-      for (int pa = 0; pa < 3; ++pa)
-        for (int pb = 0; pb + pa < 3; ++pb) {
-          double s = 0.0;
-          const auto& x = as[pa][m];
-          const auto& y = bs[pb][n];
-          for (int64_t k = 0; k < g.K; ++k) s += x[k] * y[k];
-          acc[pa + pb] += s;
+      double sum = 0.0;
+      for (int w = NG - 1; w >= 0; --w) {  // smallest weight first
+        double grp = 0.0;
+        for (int pa = std::max(0, w - D + 1); pa <= std::min(w, D - 1); ++pa) {
+          const auto& x = as[m][pa];
+          const auto& y = bs[n][w - pa];
+          for (int64_t k = 0; k < g.K; ++k) grp += x[k] * y[k];
         }
-      const double v = g.alpha * std::ldexp(acc[0] * w[0] + acc[1] * w[1] + acc[2] * w[2], ea[m] + eb[n]);
+        sum += std::ldexp(grp, -12 - 8 * w);
+      }
+      const double v = g.alpha * std::ldexp(sum, ea[m] + eb[n]);
       double* c = g.C.p + Cm.off(m) + Cn.off(n);
       *c = g.beta != 0.0 ? v + g.beta * *c : v;
       if (g.C2.p) {
@@ -146,35 +142,35 @@ SplitPackedB split_pack_b(const Contraction& g, void* dst, cudaStream_t) {
   for (int64_t n = 0; n < g.N; ++n)
     for (int64_t k = 0; k < g.K; ++k) d[n * g.K + k] = g.B.p[Bk.off(k) + Bn.off(n)];
   SplitPackedB b;
-  b.slices = dst; b.N = g.N; b.K = g.K; b.Np = g.N; b.Kp = g.K;
+  b.slices = dst; b.N = g.N; b.K = g.K; b.Np = g.N; b.Kp = g.K; b.digits = g.digits;
   g_pack += 2;
   return b;
 }
 
 void gemm_split_packed_b(const Contraction& g, const SplitPackedB& b, cudaStream_t s,
                          SplitScratch& ws) {
-  if (b.N != g.N || b.K != g.K) throw Error(ERR_INVALID_ARGUMENT, "pre-packed B of another shape");
+  if (b.N != g.N || b.K != g.K || b.digits != g.digits) throw Error(ERR_INVALID_ARGUMENT, "pre-packed B of another shape");
   const int64_t Ni = g.Ni > 0 ? g.Ni : g.N, Ki = g.Ki > 0 ? g.Ki : std::max<int64_t>(g.K, 1);
   Contraction h = g;   // B(k, n) = copy[n * K + k] in the contraction's two-level k and n
   h.B.p = static_cast<double*>(b.slices);
   h.B.s_ro = Ki; h.B.s_ri = 1; h.B.s_co = Ni * g.K; h.B.s_ci = g.K;
   gemm_split(h, s, ws);
-  g_pack -= 2;  // B was sliced before
 }
 
 // Sliced operands: the emulation keeps the rows as a dense copy [R][K] and slices the
 // rows a contraction reads again in gemm_split (same rows, same slices).
-size_t split_operand_bytes(int64_t R, int64_t K) { return size_t(R) * K * 8 + 64; }
+size_t split_operand_bytes(int64_t R, int64_t K, int) { return size_t(R) * K * 8 + 64; }
 
 SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_t s_ro,
-                                int64_t s_ri, int64_t K, int64_t s_k, void* dst, cudaStream_t) {
+                                int64_t s_ri, int64_t K, int64_t s_k, void* dst, cudaStream_t,
+                                int digits) {
   if (R <= 0 || K <= 0) throw Error(ERR_BAD_SHAPE, "split_pack_operand: empty operand");
   Ax r = ax(Ri > 0 ? Ri : R, s_ro, s_ri);
   double* d = static_cast<double*>(dst);
   for (int64_t i = 0; i < R; ++i)
     for (int64_t k = 0; k < K; ++k) d[i * K + k] = src[r.off(i) + k * s_k];
   SplitOperand o;
-  o.slices = dst; o.R = R; o.K = K; o.Rp = R; o.Kp = K;
+  o.slices = dst; o.R = R; o.K = K; o.Rp = R; o.Kp = K; o.digits = digits;
   g_pack += 2;
   return o;
 }
@@ -183,7 +179,7 @@ void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const Spl
                           const SplitOperand& B, const SplitRuns& br, cudaStream_t s,
                           SplitScratch& ws) {
   if (g.M <= 0 || g.N <= 0) return;
-  if (A.K != g.K || B.K != g.K)
+  if (A.K != g.K || B.K != g.K || A.digits != B.digits)
     throw Error(ERR_INVALID_ARGUMENT, "gemm_split_prepacked: operands of another K");
   const int64_t K = g.K;
   auto rows = [&](const SplitOperand& o, const SplitRuns& r, int64_t X) {
@@ -199,10 +195,11 @@ void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const Spl
     return d;
   };
   std::vector<double> Ad = rows(A, ar, g.M), Bd = rows(B, br, g.N);
-  g_pack -= 4;  // nothing is sliced here on the device (gemm_split below counts four)
+  g_pack -= 2;  // nothing is sliced here on the device (gemm_split below counts two)
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
   Contraction h = g;
   h.Ki = 0;
+  h.digits = A.digits;
   h.A.p = Ad.data(); h.A.s_ro = Mi * K; h.A.s_ri = K; h.A.s_co = 0; h.A.s_ci = 1;
   h.B.p = Bd.data(); h.B.s_ro = 0; h.B.s_ri = 1; h.B.s_co = Ni * K; h.B.s_ci = K;
   gemm_split(h, s, ws);

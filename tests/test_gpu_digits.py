@@ -1,0 +1,24 @@
+"""The digit-form contraction kernels (four digits: split precision, seven: FP64) at the
+edges of their tiles (128 x 128 and 128 x 64), of the K step of 32 and of the K blocks of
+64, beyond one S32 accumulation span (K > 16384), and with a non-finite input, against
+128-bit dot products with a derived bound (tests/kernels/digits_check.cu)."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+sys.path.insert(0, os.path.join(os.path.dirname(__file__), "kernels"))
+
+
+@pytest.mark.parametrize("shape", [
+    (1, 1, 1, 0, 0), (128, 64, 32, 0, 1), (129, 65, 33, 1, 0), (127, 191, 97, 0, 0),
+    (300, 520, 160, 1, 1), (2500, 1300, 64, 0, 0), (130, 70, 16417, 1, 0)])
+def test_digit_forms(shape):
+    import build as kbuild
+    exe = kbuild.build("digits_check")
+    r = subprocess.run([exe] + [str(x) for x in shape], capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.count("errflag=0") == 8
