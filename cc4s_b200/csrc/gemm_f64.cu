@@ -1,23 +1,37 @@
 // FP64 DMMA contraction kernel (mma.sync.m16n8k16.f64) with cp.async staging.
 //
-// Tile 128 (m) x 128 (n) x 32 (k), 256 threads = 8 warps in a 2 x 4 grid,
-// each warp owns a 64 x 32 sub-tile = 4 x 4 MMA tiles of 16 x 8.  Operand
-// tiles are staged through a 3-stage cp.async ring in shared memory (212 KB).
-// Shared-memory rows are padded by 4 doubles so that the fragment reads of
-// both storage orders ([m][k] and [k][m]) are free of bank conflicts.
-// Address arithmetic is kept off the critical path: offsets of the m / n
-// tile rows are computed once per tile, k offsets with 32-bit division once
-// per thread and k-tile, then stepped incrementally.
+// A tile of BM (m) x BN (n) x BK (k), one warp per WM x WN sub-tile of 16 x 8 MMA tiles;
+// operand tiles are staged through a ring of STAGES cp.async buffers in shared memory.
+// Shared-memory rows are padded by 4 doubles so that the fragment reads of both storage
+// orders ([m][k] and [k][m]) are free of bank conflicts.  Address arithmetic is kept off
+// the critical path: offsets of the m / n tile rows are computed once per tile, k offsets
+// with 32-bit division once per thread and k-tile, then stepped incrementally.
 #include "gemm_f64.cuh"
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
+#include <utility>
 
 namespace cc4s_b200 {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3, THREADS = 256;
+// Tile shapes.  The wide one (212 KB of shared memory, one CTA per SM) is bound by the
+// FP64 tensor pipe; the others leave room for three or four CTAs per SM and pad narrow
+// outputs less.  The many contractions with a hole index as N (or, transposed, as M) are
+// bound by reading their operands once N is padded to 16 or 32 instead of 128:
+// 16 x 16 x 262144 680 -> 44 us, 128 x 16 x 128 in 512 batches 112 -> 24 us,
+// 32 x 32 x 256 in 8192 batches 2714 -> 411 us (2.8 TB/s), 2048 x 1 x 2048 63 -> 17 us.
+template <int BM_, int BN_, int BK_, int STAGES_, int WM_, int WN_>
+struct Tile {
+  static constexpr int BM = BM_, BN = BN_, BK = BK_, STAGES = STAGES_, WM = WM_, WN = WN_;
+  static constexpr int THREADS = (BM / WM) * (BN / WN) * 32;
+};
+using TileWide = Tile<128, 128, 32, 3, 64, 32>;   // 256 threads
+using TileMid = Tile<64, 64, 16, 3, 32, 32>;      // 128 threads, 61 KB
+using TileN32 = Tile<64, 32, 16, 4, 16, 32>;      // 128 threads, 61 KB
+using TileN16 = Tile<64, 16, 16, 4, 16, 16>;      // 128 threads, 51 KB
 constexpr int64_t RASTER_M = 8;  // tile rows per raster group
 
 static std::atomic<uint64_t> g_launches{0};
@@ -58,7 +72,7 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 // Loader of one operand tile stored S[u][w] (w contiguous in shared memory,
 // row length W + 4).  One of (u, w) is the k index, the other is m or n.
 // KU: the strided tile axis u is k; otherwise w is k.
-template <int U, int W, int V, bool KU>
+template <int U, int W, int V, bool KU, int THREADS>
 struct Loader {
   static constexpr int LD = W + 4;
   static constexpr int WCH = W / V;               // chunks per smem row
@@ -130,11 +144,13 @@ __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[8], con
 }
 
 // A_KC: A tile stored [m][k]; otherwise [k][m].  B_NC: B tile stored [k][n]; otherwise [n][k].
-template <bool A_KC, bool B_NC, int VA, int VB>
-__global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
+template <class T, bool A_KC, bool B_NC, int VA, int VB>
+__global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
   extern __shared__ __align__(16) double smem[];
-  using LA = Loader<A_KC ? BM : BK, A_KC ? BK : BM, VA, !A_KC>;
-  using LB = Loader<B_NC ? BK : BN, B_NC ? BN : BK, VB, B_NC>;
+  constexpr int BM = T::BM, BN = T::BN, BK = T::BK, STAGES = T::STAGES;
+  constexpr int MT = T::WM / 16, NT = T::WN / 8;  // MMA tiles of a warp
+  using LA = Loader<A_KC ? BM : BK, A_KC ? BK : BM, VA, !A_KC, T::THREADS>;
+  using LB = Loader<B_NC ? BK : BN, B_NC ? BN : BK, VB, B_NC, T::THREADS>;
   constexpr int A_SIZE = (A_KC ? BM : BK) * LA::LD;
   constexpr int B_SIZE = (B_NC ? BK : BN) * LB::LD;
   constexpr int STAGE = A_SIZE + B_SIZE;
@@ -143,7 +159,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = (warp >> 2) * 64, wn = (warp & 3) * 32;
+  constexpr int WN_COUNT = BN / T::WN;
+  const int wm = (warp / WN_COUNT) * T::WM, wn = (warp % WN_COUNT) * T::WN;
 
   // Grouped tile order: the blocks launched together cover RASTER_M tile rows
   // and sweep the tile columns, so each B column tile is read from DRAM once per
@@ -174,11 +191,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
   la.init(tid, m0, p.M, p.Am);
   lb.init(tid, n0, p.N, p.Bn);
 
-  double acc[4][4][4];
+  double acc[MT][NT][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
 
@@ -210,9 +227,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
     const double* Bs = As + A_SIZE;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 16) {
-      double a[4][8], bf[4][4];
+      double a[MT][8], bf[NT][4];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int mr = wm + mt * 16 + g + ((q & 1) << 3);
@@ -220,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
           a[mt][q] = A_KC ? As[mr * ALD + kc] : As[kc * ALD + mr];
         }
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int nc = wn + nt * 8 + g;
@@ -228,9 +245,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
           bf[nt][q] = B_NC ? Bs[kc * BLD + nc] : Bs[nc * BLD + kc];
         }
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) dmma16(acc[mt][nt], a[mt], bf[nt]);
+        for (int nt = 0; nt < NT; ++nt) dmma16(acc[mt][nt], a[mt], bf[nt]);
     }
   }
   cp_wait<0>();
@@ -239,9 +256,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
   if (p.partial) {
     double* P = p.partial + (static_cast<int64_t>(split) * p.batch + b) * p.M * p.N;
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int64_t m = m0 + wm + mt * 16 + g + ((q >> 1) << 3);
@@ -252,44 +269,44 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
   }
   double* Cb = p.C + p.Cb.off(static_cast<uint32_t>(b));
   double* C2b = p.C2 ? p.C2 + p.C2b.off(static_cast<uint32_t>(b)) : nullptr;
-  int64_t co[8], co2[8];
+  int64_t co[2 * NT], co2[2 * NT];
 #pragma unroll
-  for (int h = 0; h < 8; ++h) {  // column offsets: nt = h >> 1, parity h & 1
+  for (int h = 0; h < 2 * NT; ++h) {  // column offsets: nt = h >> 1, parity h & 1
     const int64_t n = n0 + wn + (h >> 1) * 8 + 2 * t + (h & 1);
     co[h] = n < p.N ? p.Cn.off(static_cast<uint32_t>(n)) : 0;
     co2[h] = (C2b && n < p.N) ? p.C2n.off(static_cast<uint32_t>(n)) : 0;
   }
-  // Accumulating stores: the eight old values of a fragment row are loaded before
+  // Accumulating stores: the old values of a fragment row are loaded before
   // any of them is stored, so the reads are in flight together (a store followed
   // by a load through another pointer would serialise them: the two may alias).
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
       const int64_t m = m0 + wm + mt * 16 + g + hh * 8;
       if (m >= p.M) continue;
       const int64_t ro = p.Cm.off(static_cast<uint32_t>(m));
       const int64_t ro2 = C2b ? p.C2m.off(static_cast<uint32_t>(m)) : 0;
-      double val[8], old[8];
+      double val[2 * NT], old[2 * NT];
 #pragma unroll
-      for (int h = 0; h < 8; ++h) {
+      for (int h = 0; h < 2 * NT; ++h) {
         const int64_t n = n0 + wn + (h >> 1) * 8 + 2 * t + (h & 1);
         val[h] = p.alpha * acc[mt][h >> 1][hh * 2 + (h & 1)];
         old[h] = (p.beta != 0.0 && n < p.N) ? Cb[ro + co[h]] : 0.0;
       }
 #pragma unroll
-      for (int h = 0; h < 8; ++h) {
+      for (int h = 0; h < 2 * NT; ++h) {
         const int64_t n = n0 + wn + (h >> 1) * 8 + 2 * t + (h & 1);
         if (n < p.N) Cb[ro + co[h]] = val[h] + p.beta * old[h];
       }
       if (C2b) {
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
+        for (int h = 0; h < 2 * NT; ++h) {
           const int64_t n = n0 + wn + (h >> 1) * 8 + 2 * t + (h & 1);
           old[h] = (p.beta != 0.0 && n < p.N) ? C2b[ro2 + co2[h]] : 0.0;
         }
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
+        for (int h = 0; h < 2 * NT; ++h) {
           const int64_t n = n0 + wn + (h >> 1) * 8 + 2 * t + (h & 1);
           if (n < p.N) C2b[ro2 + co2[h]] = val[h] + p.beta * old[h];
         }
@@ -297,26 +314,45 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f64_kernel(KParams p) {
     }
 }
 
-// Fixed-order reduction of split-K partials, then the alpha/beta epilogue.
-__global__ void splitk_reduce_kernel(KParams p) {
+// Fixed-order reduction of split-K partials, then the alpha/beta epilogue.  GROUPS = 8
+// (eight splits and more): 32 elements per block, the eight warps sum every eighth split
+// and the eight sums are added in order; GROUPS = 1: one thread per element (one thread per element left a 16 x 16 output with 512 splits to one block's
+// chain of 512 loads).
+template <int GROUPS>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(KParams p) {
+  constexpr int PER = 256 / GROUPS;  // elements per block
+  __shared__ double part[GROUPS][PER];
   const int64_t total = p.batch * p.M * p.N;
-  const int64_t slab = total;
-  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  const int lane = threadIdx.x % PER, warp = threadIdx.x / PER;
+  for (int64_t e0 = static_cast<int64_t>(blockIdx.x) * PER; e0 < total;
+       e0 += static_cast<int64_t>(gridDim.x) * PER) {
+    const int64_t e = e0 + lane;
     double s = 0.0;
-    for (int q = 0; q < p.nsplit; ++q) s += p.partial[q * slab + e];
-    const int64_t b = e / (p.M * p.N);
-    const int64_t r = e - b * p.M * p.N;
-    const int64_t m = r / p.N, n = r - (r / p.N) * p.N;
-    const double v = p.alpha * s;
-    double* c = p.C + p.Cb.off(static_cast<uint32_t>(b)) + p.Cm.off(static_cast<uint32_t>(m)) +
-                p.Cn.off(static_cast<uint32_t>(n));
-    *c = (p.beta != 0.0) ? v + p.beta * *c : v;
-    if (p.C2) {
-      double* c2 = p.C2 + p.C2b.off(static_cast<uint32_t>(b)) +
-                   p.C2m.off(static_cast<uint32_t>(m)) + p.C2n.off(static_cast<uint32_t>(n));
-      *c2 = (p.beta != 0.0) ? v + p.beta * *c2 : v;
+    if (e < total) {
+#pragma unroll 8
+      for (int q = warp; q < p.nsplit; q += GROUPS) s += p.partial[q * total + e];
     }
+    if (GROUPS > 1) {
+      part[warp][lane] = s;
+      __syncthreads();
+    }
+    if (warp == 0 && e < total) {
+#pragma unroll
+      for (int q = 1; q < GROUPS; ++q) s += part[q][lane];
+      const int64_t b = e / (p.M * p.N);
+      const int64_t r = e - b * p.M * p.N;
+      const int64_t m = r / p.N, n = r - (r / p.N) * p.N;
+      const double v = p.alpha * s;
+      double* c = p.C + p.Cb.off(static_cast<uint32_t>(b)) + p.Cm.off(static_cast<uint32_t>(m)) +
+                  p.Cn.off(static_cast<uint32_t>(n));
+      *c = (p.beta != 0.0) ? v + p.beta * *c : v;
+      if (p.C2) {
+        double* c2 = p.C2 + p.C2b.off(static_cast<uint32_t>(b)) +
+                     p.C2m.off(static_cast<uint32_t>(m)) + p.C2n.off(static_cast<uint32_t>(n));
+        *c2 = (p.beta != 0.0) ? v + p.beta * *c2 : v;
+      }
+    }
+    if (GROUPS > 1) __syncthreads();
   }
 }
 
@@ -330,18 +366,18 @@ inline Axis axis(int64_t inner, int64_t s_o, int64_t s_i) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <bool AK, bool BN_, int VA, int VB>
+template <class T, bool AK, bool BN_, int VA, int VB>
 void launch(const KParams& p, dim3 grid, cudaStream_t s) {
-  constexpr int A_SIZE = AK ? BM * (BK + 4) : BK * (BM + 4);
-  constexpr int B_SIZE = BN_ ? BK * (BN + 4) : BN * (BK + 4);
-  constexpr size_t smem = static_cast<size_t>(STAGES) * (A_SIZE + B_SIZE) * sizeof(double);
+  constexpr int A_SIZE = AK ? T::BM * (T::BK + 4) : T::BK * (T::BM + 4);
+  constexpr int B_SIZE = BN_ ? T::BK * (T::BN + 4) : T::BN * (T::BK + 4);
+  constexpr size_t smem = static_cast<size_t>(T::STAGES) * (A_SIZE + B_SIZE) * sizeof(double);
   static bool configured = false;
   if (!configured) {
-    CC_CHECK(cudaFuncSetAttribute(gemm_f64_kernel<AK, BN_, VA, VB>,
+    CC_CHECK(cudaFuncSetAttribute(gemm_f64_kernel<T, AK, BN_, VA, VB>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  gemm_f64_kernel<AK, BN_, VA, VB><<<grid, THREADS, smem, s>>>(p);
+  gemm_f64_kernel<T, AK, BN_, VA, VB><<<grid, T::THREADS, smem, s>>>(p);
   CC_LAUNCH_CHECK();
 }
 
@@ -349,8 +385,29 @@ void launch(const KParams& p, dim3 grid, cudaStream_t s) {
 
 uint64_t gemm_launch_count() { return g_launches.load(); }
 
+namespace {
+// The same contraction with C transposed: C^T = B^T A^T.
+Contraction transposed(const Contraction& g) {
+  auto t = [](View v) {
+    std::swap(v.s_ro, v.s_co);
+    std::swap(v.s_ri, v.s_ci);
+    return v;
+  };
+  Contraction h = g;
+  std::swap(h.M, h.N);
+  std::swap(h.Mi, h.Ni);
+  h.A = t(g.B);
+  h.B = t(g.A);
+  h.C = t(g.C);
+  h.C2 = t(g.C2);
+  return h;
+}
+}  // namespace
+
 void gemm(const Contraction& g0, cudaStream_t s, const GemmScratch& ws) {
   Contraction g = g0;
+  // a narrow M becomes a narrow N (not where the M tiles would exceed the grid)
+  if (g.M <= 32 && g.N > g.M && g.N < 65535 * 64) g = transposed(g0);
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return;
   if (g.K < 0) throw Error(ERR_INVALID_ARGUMENT, "gemm: negative K");
   const int64_t lim = int64_t(1) << 31;
@@ -399,16 +456,30 @@ void gemm(const Contraction& g0, cudaStream_t s, const GemmScratch& ws) {
     vb2 = g.B.s_ri == 1 && even(Ki) && even(g.K) && even(g.B.s_ro) && even(g.B.s_co) &&
           even(g.B.s_ci) && even(g.B.s_bo) && even(g.B.s_bi) && aligned16(g.B.p);
 
-  const int64_t mt = (g.M + BM - 1) / BM, nt = (g.N + BN - 1) / BN;
+  // Tile: by N where it is narrow; else 64 x 64 where 128 x 128 pads the output by a fifth
+  // more or has fewer tiles than SMs (171 x 171 x 19 in 613 batches 249 -> 172 us, 320 x 320
+  // x 320 40 -> 17 us); 128 x 128 has the higher rate where neither holds (29 TFLOP/s).
+  enum { WIDE, MID, N32, N16 } shape = WIDE;
+  auto cdiv = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  if (g.M <= 65535 * 64) {
+    const int64_t wide = cdiv(g.M, 128) * cdiv(g.N, 128), mid = cdiv(g.M, 64) * cdiv(g.N, 64);
+    if (g.N <= 16) shape = N16;
+    else if (g.N <= 32) shape = N32;
+    else if (mid * 10 < wide * 4 * 8 || wide * g.batch < 148) shape = MID;
+  }
+  const int BM = shape == WIDE ? 128 : 64, BK = shape == WIDE ? 32 : 16;
+  const int BN = shape == WIDE ? 128 : shape == MID ? 64 : shape == N32 ? 32 : 16;
+  const int64_t mt = cdiv(g.M, BM), nt = cdiv(g.N, BN);
   const int64_t tiles = mt * nt * g.batch;
   // Split K when the output has too few tiles to fill 148 SMs.
   int nsplit = 1;
-  const int64_t target = 2 * 148;
+  const int64_t target = (shape == WIDE ? 2 : shape == MID ? 3 : 4) * 148;
   if (tiles < target && g.K >= 8 * BK && ws.p) {
     int64_t want = (target + tiles - 1) / tiles;
     want = std::min<int64_t>(want, g.K / (4 * BK));
-    want = std::min<int64_t>(want, 64);
-    while (want > 1 && static_cast<size_t>(want * g.batch * g.M * g.N) > ws.elems) --want;
+    want = std::min<int64_t>(want, shape == WIDE ? 64 : 592);
+    const int64_t fit = static_cast<int64_t>(ws.elems) / std::max<int64_t>(g.batch * g.M * g.N, 1);
+    want = std::min(want, fit);
     if (want > 1) nsplit = static_cast<int>(want);
   }
   int64_t klen = g.K;
@@ -425,19 +496,29 @@ void gemm(const Contraction& g0, cudaStream_t s, const GemmScratch& ws) {
   dim3 grid(static_cast<unsigned>(nt), static_cast<unsigned>(mt),
             static_cast<unsigned>(g.batch * nsplit));
 
-#define CC_GEMM_DISPATCH(AK, BNC)                                   \
-  if (va2 && vb2) launch<AK, BNC, 2, 2>(p, grid, s);                \
-  else if (va2) launch<AK, BNC, 2, 1>(p, grid, s);                  \
-  else if (vb2) launch<AK, BNC, 1, 2>(p, grid, s);                  \
-  else launch<AK, BNC, 1, 1>(p, grid, s);
-  if (a_kc && b_nc) { CC_GEMM_DISPATCH(true, true) }
-  else if (a_kc) { CC_GEMM_DISPATCH(true, false) }
-  else if (b_nc) { CC_GEMM_DISPATCH(false, true) }
-  else { CC_GEMM_DISPATCH(false, false) }
-#undef CC_GEMM_DISPATCH
+  auto go = [&](auto tile) {
+    using T = decltype(tile);
+    auto vec = [&](auto ak, auto bnc) {
+      constexpr bool AK = decltype(ak)::value, BNC = decltype(bnc)::value;
+      if (va2 && vb2) launch<T, AK, BNC, 2, 2>(p, grid, s);
+      else if (va2) launch<T, AK, BNC, 2, 1>(p, grid, s);
+      else if (vb2) launch<T, AK, BNC, 1, 2>(p, grid, s);
+      else launch<T, AK, BNC, 1, 1>(p, grid, s);
+    };
+    if (a_kc && b_nc) vec(std::true_type(), std::true_type());
+    else if (a_kc) vec(std::true_type(), std::false_type());
+    else if (b_nc) vec(std::false_type(), std::true_type());
+    else vec(std::false_type(), std::false_type());
+  };
+  if (shape == WIDE) go(TileWide());
+  else if (shape == MID) go(TileMid());
+  else if (shape == N32) go(TileN32());
+  else go(TileN16());
   g_launches.fetch_add(1);
   if (nsplit > 1) {
-    splitk_reduce_kernel<<<grid_for(g.batch * g.M * g.N, 256), 256, 0, s>>>(p);
+    const int64_t out = g.batch * g.M * g.N;
+    if (nsplit >= 8) splitk_reduce_kernel<8><<<grid_for(out, 32), 256, 0, s>>>(p);
+    else splitk_reduce_kernel<1><<<grid_for(out, 256), 256, 0, s>>>(p);
     CC_LAUNCH_CHECK();
     g_launches.fetch_add(1);
   }
