@@ -67,7 +67,15 @@ CcsdComplex::CcsdComplex(const ComplexSystem& sys, const RealOptions& opt, Strea
         1, std::min<int64_t>(v, budget / (slab_rows_ * slab_rows_ * v)));
     const int64_t npanels = (v + cmax - 1) / cmax;
     slab_cols_ = (v + npanels - 1) / npanels;
-    if (opt.ppl) slab_ = z(slab_rows_ * slab_rows_ * slab_cols_ * v);
+    // The off-diagonal slices of one a slice are contracted together, slab_group_ of them at
+    // a time (2^26 complex values, 1 GiB): the same terms, and s^2 = o^2 rows per
+    // contraction become s^2 slab_group_ (one 256 x 256 output of K = 25600 at
+    // o = 16, v = 160 filled 4 of 148 SMs).
+    const int64_t slice = slab_rows_ * slab_rows_ * slab_cols_ * v;
+    slab_group_ = std::max<int64_t>(
+        1, std::min<int64_t>((v + slab_rows_ - 1) / slab_rows_ - 1,
+                             std::min(budget, int64_t(1) << 26) / slice));
+    if (opt.ppl) slab_ = z(slab_group_ * slice);
   } catch (...) {
     release_all();
     throw;
@@ -420,14 +428,15 @@ void CcsdComplex::residual(const double* T, double* R) {
       c.alpha = -1.0; c.beta = 1.0;
       zgemm(c, pl, gph, gpp);
     }
-    const int64_t s = slab_rows_, cn = slab_cols_, nb = (v + s - 1) / s;
-    const int64_t sz = s * s * cn * v;  // imaginary plane of the slab
+    const int64_t s = slab_rows_, cn = slab_cols_, nb = (v + s - 1) / s, ng = slab_group_;
+    const int64_t sz = ng * s * s * cn * v;  // imaginary plane of the slab
     for (int64_t c0 = 0; c0 < v; c0 += cn) {
       const int64_t nc = std::min(cn, v - c0);
       for (int64_t X = 0; X < nb; ++X)
-        for (int64_t Yb = 0; Yb <= X; ++Yb) {
-          const int64_t x0 = X * s, sx = std::min(s, v - x0);
-          const int64_t y0 = Yb * s, sy = std::min(s, v - y0);
+        for (int64_t Yb = 0; Yb <= X; Yb += Yb < X ? std::min(ng, X - Yb) : 1) {
+          // slices Yb .. of one group (mirrored into (b,a,j,i)), then the diagonal one
+          const int64_t x0 = X * s, sx = std::min(s, v - x0), y0 = Yb * s;
+          const int64_t sy = Yb < X ? std::min(ng, X - Yb) * s : sx;
           const size_t t_build = tape_.size();
           {  // slab[x][y][c'][d], m = (x, c'), n = (y, d)
             Contraction c; c.M = sx * nc; c.N = sy * v; c.K = G; c.Mi = nc; c.Ni = v;

@@ -70,6 +70,7 @@ class CcsdComplex : public Schedule {
          *Xkl1_ = nullptr, *Xkl2_ = nullptr, *kck_ = nullptr, *P1_ = nullptr, *P_ = nullptr,
          *slab_ = nullptr;
   int64_t slab_rows_ = 0, slab_cols_ = 0;  // ladder block size, c-panel size
+  int64_t slab_group_ = 1;                 // off-diagonal slices contracted together
 };
 
 }  // namespace cc4s_b200

@@ -210,6 +210,41 @@ void Schedule::tc_(const Contraction& c) {
   split_exec(c);
 }
 
+// A complex contraction in a digit form, if one pays: the four real ones in two launches.
+bool Schedule::zgemm_split(const Contraction& c, int64_t a_im, int64_t b_im, int64_t c_im,
+                           bool conjA, bool conjB, bool big) {
+  if (taping_) return false;  // reverse mode records the four real contractions
+  Contraction d = c;
+  d.digits = digits_for(c, big);
+  if (d.digits != 4) {
+    Contraction k2 = c;
+    k2.K = 2 * c.K;
+    d.digits = digits_for(k2, false);
+  }
+  if (!d.digits) return false;
+  try {
+    const size_t need = gemm_split_complex_scratch_bytes(d);
+    if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
+  } catch (const Error& e) {
+    if (e.status != ERR_OUT_OF_MEMORY || d.digits != 7) throw;
+    return false;
+  }
+  const double f = 8.0 * double(c.M) * double(c.N) * double(c.K);
+  if (count_flops_) flops_ += f;
+  const bool prof = profile_ && count_flops_;
+  const size_t k = ev_flops_.size();
+  if (prof) {
+    while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
+    ev_flops_.push_back(f);
+    ev_split_.push_back(d.digits == 4);
+    ev_shape_.push_back({c.M, c.N, 2 * c.K, 2});
+    ops::event_record(ev_[2 * k], s_);
+  }
+  gemm_split_complex(d, a_im, b_im, c_im, conjA, conjB, s_, split_);
+  if (prof) ops::event_record(ev_[2 * k + 1], s_);
+  return true;
+}
+
 void Schedule::zgemm(Contraction c, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
                      bool conjB, bool big) {
   auto run = [&](const Contraction& x) { if (big) tc_(x); else gemm_(x); };
@@ -219,6 +254,7 @@ void Schedule::zgemm(Contraction c, int64_t a_im, int64_t b_im, int64_t c_im, bo
   double* Br = c.B.p;
   double* Cr = c.C.p;
   double* C2r = c.C2.p;
+  if (a_im && b_im && c_im && zgemm_split(c, a_im, b_im, c_im, conjA, conjB, big)) return;
   // real plane: Re(A) Re(B) - sA sB Im(A) Im(B)
   run(c);
   if (a_im && b_im) {

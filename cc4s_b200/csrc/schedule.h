@@ -172,6 +172,8 @@ class Schedule {
   // contractions; `big` routes them through tc_.
   void zgemm(Contraction c, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA = false,
              bool conjB = false, bool big = false);
+  bool zgemm_split(const Contraction& c, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
+                   bool conjB, bool big);
   // A labelled operand of ein(): a dense row-major tensor whose indices are named
   // by one character each, in memory order (last fastest), with their extents;
   // `im` the element offset of the imaginary plane (0: real), `conj` conjugates it.

@@ -83,12 +83,21 @@ struct PackArgs {
   int* rexp;              // per-row exponent
   int8_t* dst;            // [NS][Rp][Kp]
   int r_contig;           // 1: the row index is the contiguous one in memory
+  // Two planes of a complex operand side by side along k: k < K1 reads at offset off[0]
+  // with sign[0], the others at off[1] with sign[1] (K1 = K: one plane).
+  int64_t K1;
+  int64_t off[2];
+  double sign[2];
+  __device__ __forceinline__ int64_t koff(int64_t k) const {
+    return k < K1 ? off[0] + ak.off(static_cast<uint32_t>(k))
+                  : off[1] + ak.off(static_cast<uint32_t>(k - K1));
+  }
 };
-// One launch slices up to two operands (A and B of a contraction).
-struct PackPair {
-  PackArgs op[2];
-  int64_t first;          // work items of op[0]; the rest belong to op[1]
-  int64_t total;
+// One launch slices up to three operands: A and B of a contraction, one of them in two
+// forms in a complex one.
+struct PackSet {
+  PackArgs op[3];
+  int64_t end[3];         // work items of the operands, cumulative; the last is the total
 };
 
 // Packing works on tiles of 64 rows x 64 k staged in shared memory.  The row and
@@ -112,7 +121,7 @@ __device__ __forceinline__ void pack_load_tile(const PackArgs& a, int64_t r0, in
       t.roff[q] = r < a.R ? a.ar.off(static_cast<uint32_t>(r)) : -1;
     } else {
       const int64_t k = k0 + (q - PR);
-      t.koff[q - PR] = k < a.K ? a.ak.off(static_cast<uint32_t>(k)) : -1;
+      t.koff[q - PR] = k < a.K ? a.koff(k) : -1;
     }
   }
   __syncthreads();
@@ -144,12 +153,13 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
 // Bound by latency until a few hundred items are in flight, which sets kstrip: strips of
 // 1024 k left two 1024 x 1024 operands to 32 blocks (whole seven-digit contraction 79 us,
 // 63 us with strips of 128).
-__global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackPair pp, int kstrip) {
+__global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackSet pp, int kstrip) {
   __shared__ unsigned long long part[8][PR];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int64_t it = blockIdx.x; it < pp.total; it += gridDim.x) {
-    const PackArgs& a = pp.op[it < pp.first ? 0 : 1];
-    const int64_t w = it < pp.first ? it : it - pp.first;
+  for (int64_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
+    const int which = it < pp.end[0] ? 0 : it < pp.end[1] ? 1 : 2;
+    const PackArgs& a = pp.op[which];
+    const int64_t w = which ? it - pp.end[which - 1] : it;
     const int64_t nks = (a.K + kstrip - 1) / kstrip;
     const int64_t r0 = (w / nks) * PR, kbeg = (w % nks) * kstrip;
     const int64_t kend = min(a.K, kbeg + kstrip);
@@ -163,7 +173,7 @@ __global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackPair pp, int kst
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int64_t k = k0 + 8 * j;
-          const int64_t ko = k < kend ? a.ak.off(static_cast<uint32_t>(k)) : 0;
+          const int64_t ko = k < kend ? a.koff(k) : 0;
           x[0][j] = k < kend && ra < a.R ? sa[ko] : 0.0;
           x[1][j] = k < kend && rb < a.R ? sb[ko] : 0.0;
         }
@@ -193,8 +203,8 @@ __global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackPair pp, int kst
       }
       for (int64_t k0 = kbeg + lane; k0 < kend; k0 += 64) {
         const int64_t k1 = k0 + 32;
-        const int64_t o0 = a.ak.off(static_cast<uint32_t>(k0));
-        const int64_t o1 = k1 < kend ? a.ak.off(static_cast<uint32_t>(k1)) : o0;
+        const int64_t o0 = a.koff(k0);
+        const int64_t o1 = k1 < kend ? a.koff(k1) : o0;
         double x[2][8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -225,13 +235,14 @@ __device__ __forceinline__ double pow2i(int e) {
 // written in balanced base 256, lowest digit first (each in [-128, 127], the top one in
 // [-64, 65]).  Memory bound: 8 B read and NS B written per element.
 template <int NS>
-__global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackPair pp) {
+__global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
   __shared__ PackTile t;
   __shared__ double scale_s[2][PR];
   const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  for (int64_t it = blockIdx.x; it < pp.total; it += gridDim.x) {
-    const PackArgs& a = pp.op[it < pp.first ? 0 : 1];
-    const int64_t w = it < pp.first ? it : it - pp.first;
+  for (int64_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
+    const int which = it < pp.end[0] ? 0 : it < pp.end[1] ? 1 : 2;
+    const PackArgs& a = pp.op[which];
+    const int64_t w = which ? it - pp.end[which - 1] : it;
     const int64_t nk = (a.Kp + PKT - 1) / PKT, pl = a.Rp * a.Kp;
     const int64_t r0 = (w / nk) * PR, k0 = (w % nk) * PKT;
     if (threadIdx.x < PR) {
@@ -260,7 +271,7 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackPair pp) {
       __align__(16) int8_t h[NS][16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const double v = t.v[row][16 * part + j];
+        const double v = t.v[row][16 * part + j] * a.sign[kb + j < a.K1 ? 0 : 1];
         long long X = s1 != 0.0 ? __double2ll_rn(v * s1 * s2) : 0;
 #pragma unroll
         for (int q = NS - 1; q > 0; --q) {
@@ -769,34 +780,44 @@ PackArgs pack_args(const View& v, bool rows_are_m, const Contraction& g, int64_t
   }
   a.R = R; a.K = g.K; a.Rp = Rp; a.Kp = Kp;
   a.rmax = rmax; a.rexp = rexp; a.dst = static_cast<int8_t*>(dst);
+  a.K1 = a.K; a.off[0] = a.off[1] = 0; a.sign[0] = a.sign[1] = 1.0;
   if (Rp % PR || Kp % 16) throw Error(ERR_BAD_SHAPE, "gemm_split: packed extents not tiled");
   return a;
 }
 
-// Row maxima and digits of one or two operands.  Their rmax arrays are one block of
-// `rows` entries starting at a.rmax (cleared here).
-void pack(const PackArgs& a, const PackArgs* b, int64_t rows, int digits, cudaStream_t s) {
-  CC_CHECK(cudaMemsetAsync(a.rmax, 0, rows * sizeof(unsigned long long), s));
-  PackPair pp;
-  pp.op[0] = a;
-  pp.op[1] = b ? *b : a;
+// Row maxima and digits of one to three operands.  Their rmax arrays are one block of
+// `rows` entries starting at that of the first (cleared here).
+void pack(const PackArgs* const* ops, int n, int64_t rows, int digits, cudaStream_t s) {
+  CC_CHECK(cudaMemsetAsync(ops[0]->rmax, 0, rows * sizeof(unsigned long long), s));
+  PackSet pp;
+  for (int k = 0; k < 3; ++k) pp.op[k] = *ops[std::min(k, n - 1)];
   // strips of k for the maxima: the longest of 128 .. 1024 that gives 148 x 6 work items
   int64_t kstrip = 1024;
   auto strips = [&](const PackArgs& x) { return (x.Rp / PR) * ((x.K + kstrip - 1) / kstrip); };
-  while (kstrip > 128 && strips(a) + (b ? strips(*b) : 0) < 148 * 6) kstrip /= 2;
   auto tiles = [](const PackArgs& x) { return (x.Rp / PR) * ((x.Kp + PKT - 1) / PKT); };
-  pp.first = strips(a);
-  pp.total = pp.first + (b ? strips(*b) : 0);
-  pack_max_kernel<<<static_cast<unsigned>(std::min<int64_t>(pp.total, 148 * 8)), PTHREADS, 0, s>>>(
+  auto items = [&](auto&& count) {
+    int64_t t = 0;
+    for (int k = 0; k < 3; ++k) pp.end[k] = t += k < n ? count(pp.op[k]) : 0;
+    return t;
+  };
+  int64_t work = items(strips);
+  while (kstrip > 128 && work < 148 * 6) {
+    kstrip /= 2;
+    work = items(strips);
+  }
+  pack_max_kernel<<<static_cast<unsigned>(std::min<int64_t>(work, 148 * 8)), PTHREADS, 0, s>>>(
       pp, static_cast<int>(kstrip));
   CC_LAUNCH_CHECK();
-  pp.first = tiles(a);
-  pp.total = pp.first + (b ? tiles(*b) : 0);
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(pp.total, 148 * 8));
+  work = items(tiles);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(work, 148 * 8));
   if (digits == 7) pack_digits_kernel<7><<<grid, PTHREADS, 0, s>>>(pp);
   else pack_digits_kernel<4><<<grid, PTHREADS, 0, s>>>(pp);
   CC_LAUNCH_CHECK();
   g_pack_launches.fetch_add(2);
+}
+void pack_one(const PackArgs& a, int64_t rows, int digits, cudaStream_t s) {
+  const PackArgs* op = &a;
+  pack(&op, 1, rows, digits, s);
 }
 
 // Packed slices of both operands are limited to this many bytes: a longer K is
@@ -885,7 +906,7 @@ SplitPackedB split_pack_b(const Contraction& g, void* dst, cudaStream_t s) {
   auto* bmax = reinterpret_cast<unsigned long long*>(p + L.b_bytes);
   b.exps = reinterpret_cast<int*>(p + L.b_bytes + rup(L.Np * 8, 1024));
   b.N = g.N; b.K = g.K; b.Np = L.Np; b.Kp = L.Kp; b.digits = digits_of(g);
-  pack(pack_args(g.B, false, g, g.N, L.Np, L.Kp, b.slices, bmax, b.exps), nullptr, g.N, b.digits, s);
+  pack_one(pack_args(g.B, false, g, g.N, L.Np, L.Kp, b.slices, bmax, b.exps), g.N, b.digits, s);
   return b;
 }
 
@@ -982,10 +1003,11 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const S
       throw Error(ERR_INVALID_ARGUMENT, "gemm_split: pre-packed B of another shape");
     Bpk = pb->slices;
     bexp = pb->exps;
-    pack(pa, nullptr, L.Mp, D, s);
+    pack_one(pa, L.Mp, D, s);
   } else {
     const PackArgs pbk = pack_args(g.B, false, g, g.N, L.Np, L.Kp, Bpk, bmax, bexp);
-    pack(pa, &pbk, L.Mp + L.Np, D, s);
+    const PackArgs* both[2] = {&pa, &pbk};
+    pack(both, 2, L.Mp + L.Np, D, s);
   }
   SplitRuns ar, br;
   ar.run = g.M;
@@ -994,6 +1016,108 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const S
 }
 
 }  // namespace
+namespace {
+// Scratch of one complex panel: the operand with more rows as one form of K' = 2 K, the
+// other as two.
+struct ComplexLayout {
+  int64_t Mp, Np, Kp;
+  int na, nb;            // forms of A and of B
+  size_t a_bytes, b_bytes, meta_bytes;  // per form; all forms
+};
+ComplexLayout complex_layout(const Contraction& g, int64_t K) {
+  const int D = digits_of(g);
+  ComplexLayout L;
+  L.Mp = rup(g.M, TM);
+  L.Np = rup(g.N, tile_n(D));
+  L.Kp = rup(2 * std::max<int64_t>(K, 1), KPAD);
+  L.na = g.M < g.N ? 2 : 1;
+  L.nb = 3 - L.na;
+  L.a_bytes = rup(D * L.Mp * L.Kp, 1024);
+  L.b_bytes = rup(D * L.Np * L.Kp, 1024);
+  L.meta_bytes = rup((L.na * L.Mp + L.nb * L.Np) * (8 + 4), 1024);
+  return L;
+}
+int64_t complex_panel_len(const Contraction& g) {
+  const ComplexLayout L = complex_layout(g, 1);
+  const int64_t per_k = 2 * digits_of(g) * (L.na * L.Mp + L.nb * L.Np);
+  const int64_t P = static_cast<int64_t>(panel_bytes()) / per_k;
+  return std::max<int64_t>(KPAD, P / KPAD * KPAD);
+}
+size_t complex_bytes(const ComplexLayout& L) {
+  return L.na * L.a_bytes + L.nb * L.b_bytes + L.meta_bytes;
+}
+}  // namespace
+
+size_t gemm_split_complex_scratch_bytes(const Contraction& g) {
+  return complex_bytes(complex_layout(g, std::min(g.K, complex_panel_len(g))));
+}
+
+void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
+                        bool conjB, cudaStream_t s, SplitScratch& ws) {
+  if (g.M <= 0 || g.N <= 0) return;
+  if (g.batch != 1) throw Error(ERR_UNSUPPORTED, "gemm_split_complex: batched contraction");
+  if (g.K <= 0) throw Error(ERR_UNSUPPORTED, "gemm_split_complex: empty K");
+  const int D = digits_of(g);
+  const double sA = conjA ? -1.0 : 1.0, sB = conjB ? -1.0 : 1.0;
+  for (const Panel& pn : panels_of(g, complex_panel_len(g))) {
+    Contraction h = g;
+    h.K = pn.kl;
+    h.Ki = pn.ki;
+    h.A.p = g.A.p + pn.a_off;
+    h.B.p = g.B.p + pn.b_off;
+    if (pn.k0 > 0) h.beta = 1.0;
+    const ComplexLayout L = complex_layout(h, h.K);
+    if (complex_bytes(L) > ws.bytes)
+      throw Error(ERR_OUT_OF_MEMORY, "gemm_split_complex: scratch too small");
+    unsigned char* p = static_cast<unsigned char*>(ws.p);
+    auto* rmax = reinterpret_cast<unsigned long long*>(p + L.na * L.a_bytes + L.nb * L.b_bytes);
+    const int64_t rows = L.na * L.Mp + L.nb * L.Np;
+    int* rexp = reinterpret_cast<int*>(rmax + rows);
+    PackArgs op[3];
+    const PackArgs* ops[3] = {&op[0], &op[1], &op[2]};
+    int64_t r = 0;
+    for (int k = 0; k < 3; ++k) {
+      const bool isA = k < L.na;
+      const int form = isA ? k : k - L.na;
+      void* dst = isA ? p + k * L.a_bytes : p + L.na * L.a_bytes + form * L.b_bytes;
+      op[k] = pack_args(isA ? h.A : h.B, isA, h, isA ? h.M : h.N, isA ? L.Mp : L.Np, L.Kp, dst,
+                        rmax + r, rexp + r);
+      r += isA ? L.Mp : L.Np;
+      const int64_t im = isA ? a_im : b_im;
+      op[k].K = 2 * h.K;
+      op[k].K1 = h.K;
+      op[k].off[1] = im;
+      if ((isA ? L.na : L.nb) == 2) {
+        // C_re = [Ar | Ai] [Br ; -sA sB Bi],  C_im = [Ar | Ai] [sB Bi ; sA Br], or the same
+        // with the two forms on the A side: [Ar | -sA sB Ai], [sA Ai | sB Ar] on [Br ; Bi]
+        if (form == 0) {
+          op[k].sign[1] = -sA * sB;
+        } else {
+          op[k].off[0] = im;
+          op[k].off[1] = 0;
+          op[k].sign[0] = isA ? sA : sB;
+          op[k].sign[1] = isA ? sB : sA;
+        }
+      }
+    }
+    pack(ops, 3, rows, D, s);
+    SplitRuns ar, br;
+    ar.run = h.M;
+    br.run = h.N;
+    for (int part = 0; part < 2; ++part) {
+      const PackArgs& A = op[L.na == 2 ? part : 0];
+      const PackArgs& B = op[L.na + (L.nb == 2 ? part : 0)];
+      Contraction c = h;
+      c.K = 2 * h.K;
+      if (part) {
+        c.C.p = g.C.p + c_im;
+        if (g.C2.p) c.C2.p = g.C2.p + c_im;
+      }
+      launch(c, D, A.dst, A.rexp, L.Mp, ar, 1, B.dst, B.rexp, L.Np, br, 1, L.Kp, s, ws);
+    }
+  }
+}
+
 size_t split_operand_bytes(int64_t R, int64_t K, int digits) {
   const int64_t Rp = rup(std::max<int64_t>(R, 1), TM), Kp = rup(std::max<int64_t>(K, 1), KPAD);
   return static_cast<size_t>(rup(digits * Rp * Kp, 1024) + rup(Rp * 8, 1024) +
@@ -1019,7 +1143,7 @@ SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_
   g.M = R; g.Mi = Ri; g.K = K;
   g.A.p = const_cast<double*>(src);
   g.A.s_ro = s_ro; g.A.s_ri = s_ri; g.A.s_co = 0; g.A.s_ci = s_k;
-  pack(pack_args(g.A, true, g, R, o.Rp, o.Kp, o.slices, rmax, o.exps), nullptr, R, digits, s);
+  pack_one(pack_args(g.A, true, g, R, o.Rp, o.Kp, o.slices, rmax, o.exps), R, digits, s);
   return o;
 }
 

@@ -34,6 +34,14 @@ void gemm_split(const Contraction& g, cudaStream_t s, SplitScratch& ws);
 // Bytes of scratch gemm_split needs for this contraction.
 size_t gemm_split_scratch_bytes(const Contraction& g);
 
+// The planar complex contraction (imaginary planes at the given element offsets, conjA /
+// conjB conjugate an operand) as two real ones over K' = 2 K with the planes side by side
+// along k: every plane is sliced once or twice instead of twice or four times, and each
+// output plane is written once.
+void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
+                        bool conjB, cudaStream_t s, SplitScratch& ws);
+size_t gemm_split_complex_scratch_bytes(const Contraction& g);
+
 // Operand B of a one-panel split contraction, sliced once and reused by several
 // contractions that share B (same N, K and B view), e.g. the ladder's X panel
 // for every block pair of one c range.

@@ -129,6 +129,27 @@ void gemm_split(const Contraction& g, cudaStream_t, SplitScratch&) {
     }
 }
 
+// The complex form: the emulation runs the four real contractions it stands for.
+size_t gemm_split_complex_scratch_bytes(const Contraction&) { return 64; }
+void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
+                        bool conjB, cudaStream_t s, SplitScratch& ws) {
+  const double sA = conjA ? -1.0 : 1.0, sB = conjB ? -1.0 : 1.0;
+  for (int part = 0; part < 2; ++part)
+    for (int term = 0; term < 2; ++term) {
+      Contraction c = g;
+      const bool ai = term == 1, bi = part == 0 ? term == 1 : term == 0;
+      if (ai) c.A.p += a_im;
+      if (bi) c.B.p += b_im;
+      if (part) {
+        c.C.p += c_im;
+        if (c.C2.p) c.C2.p += c_im;
+      }
+      c.alpha = g.alpha * (part == 0 ? (term ? -sA * sB : 1.0) : (term ? sA : sB));
+      if (term) c.beta = 1.0;
+      gemm_split(c, s, ws);
+    }
+}
+
 // Pre-packed B: the emulation keeps a dense copy B[n][k] of the operand's values
 // and slices it again in gemm_split (same values, same slices).
 size_t split_packed_b_bytes(const Contraction& g) { return size_t(g.N) * g.K * 8 + 64; }
