@@ -72,8 +72,9 @@ static bool digits7_pays(const Contraction& c) {
   auto up = [](double x, double t) { return std::ceil(x / t) * t; };
   // microseconds: launches, slicing, waves of one tile per SM
   const double tiles7 = up(M, 128) * up(N, 64) / (128 * 64);
-  const double d7 = 20.0 + 24.0 * (M + N) * K / 3.5e6 +
-                    std::ceil(tiles7 / 148.0) * (3.3 + 0.021 * up(K, 32));
+  const int parts = split_k_parts(static_cast<int64_t>(tiles7), c.M, c.N, c.K, 7);
+  const double d7 = 20.0 + 24.0 * (M + N) * K / 3.5e6 + (parts > 1 ? 6.0 : 0.0) +
+                    std::ceil(tiles7 * parts / 148.0) * (3.3 + 0.021 * up(K, 32) / parts);
   const double dmma = 12.0 + 2.0 * up(M, 128) * up(N, 128) * K / 22e6;
   return d7 < dmma;
 }

@@ -448,7 +448,10 @@ struct SplitParams {
   double alpha, beta;
   const int* ea; const int* eb;    // exponents of the packed rows of A and of B
   int* error;
-  // Packed rows (persistent kernel): logical row m of A is packed row
+  // nsplit ranges of kb_len k-blocks; range q stores at C + q part_stride.
+  int nsplit, kb_len;
+  int64_t part_stride;
+  // Packed rows: logical row m of A is packed row
   //   a_base + (m / a_run) * a_stride + m % a_run,
   // and tiles never straddle a run (a_tiles tiles per run, nMt tile rows in all);
   // likewise n for B.  One run over the whole extent is the plain case.
@@ -461,16 +464,23 @@ struct SplitParams {
 struct TileAt {
   int64_t m0, n0, pa, pb;
   int mlim, nlim;
+  int kb0, nkb;     // k-blocks of the work item
+  int64_t out;      // offset of its output
 };
 template <int TN>
 __device__ __forceinline__ TileAt tile_at(const SplitParams& p, int64_t t) {
+  TileAt a;
+  const int64_t tiles = p.nMt * p.nNt, part = t / tiles;
+  t -= part * tiles;
+  a.kb0 = static_cast<int>(part) * p.kb_len;
+  a.nkb = min(p.kb_len, p.nkb - a.kb0);
+  a.out = part * p.part_stride;
   const int64_t nM = p.nMt, nN = p.nNt;
   const int64_t per_group = RASTER_M * nN, group = t / per_group;
   const int64_t first = group * RASTER_M;
   const int64_t rows = nM - first < RASTER_M ? nM - first : RASTER_M;
   const int64_t in = t - group * per_group;
   const int64_t tm = first + in % rows, tn = in / rows;
-  TileAt a;
   const int64_t rm = tm / p.a_tiles, om = (tm - rm * p.a_tiles) * TM;
   const int64_t rn = tn / p.b_tiles, on = (tn - rn * p.b_tiles) * TN;
   a.m0 = rm * p.a_run + om;
@@ -499,9 +509,9 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
   volatile int* abort_v = &abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ntiles = p.nMt * p.nNt;
+  const int64_t ntiles = p.nMt * p.nNt * p.nsplit;
   constexpr int KB_PER_CHUNK = KCHUNK / TK;
-  const int nchunks = (p.nkb + KB_PER_CHUNK - 1) / KB_PER_CHUNK;
+  auto chunks_of = [](int nkb) { return (nkb + KB_PER_CHUNK - 1) / KB_PER_CHUNK; };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -528,7 +538,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
     uint32_t it = 0;
     for (int64_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
       const TileAt ta = tile_at<TN>(p, t);
-      for (int kb = 0; kb < p.nkb; ++kb, ++it) {
+      for (int kb = ta.kb0; kb < ta.kb0 + ta.nkb; ++kb, ++it) {
         const int s = it % NST;
         if (it >= NST && !mbar_wait(smem_u32(&bars[NST + s]), ((it / NST) - 1) & 1)) {
           atomicExch(&abort_flag, 1);
@@ -546,14 +556,16 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
     // ---- MMA issuer: chunks of all tiles, global stage and chunk counters ----
     uint32_t it = 0, q = 0;
     for (int64_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
-      int kb = 0;
+      const TileAt ta = tile_at<TN>(p, t);
+      const int nchunks = chunks_of(ta.nkb), kb_last = ta.kb0 + ta.nkb;
+      int kb = ta.kb0;
       for (int c = 0; c < nchunks && !*abort_v; ++c, ++q) {
         if (q > 0 && !mbar_wait(smem_u32(&bars[2 * NST + 1]), (q - 1) & 1)) {
           atomicExch(&abort_flag, 1);
           break;
         }
         tc_fence_after();
-        const int kb_end = min(p.nkb, (c + 1) * KB_PER_CHUNK);
+        const int kb_end = min(kb_last, kb + KB_PER_CHUNK);
         bool first = true;
         for (; kb < kb_end; ++kb, ++it) {
           const int s = it % NST;
@@ -586,6 +598,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
 #pragma unroll
       for (int j = 0; j < COLS; ++j) acc[j] = 0.0;
       bool ok = true;
+      const int nchunks = chunks_of(ta.nkb);
       for (int c = 0; c < nchunks; ++c, ++q) {
         const bool got = mbar_wait(smem_u32(&bars[2 * NST]), q & 1);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
@@ -619,7 +632,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
       const bool mv = row < ta.mlim;
       // acc counts 2^-36: digit 0 weighs 2^-6 in each operand, the fourth group 2^-24 of the first
       const double sa = mv ? row_scale(p.alpha, p.ea[ta.pa + row], 18) : 0.0;
-      const int64_t rowoff = mv ? p.Cm.off(static_cast<uint32_t>(m)) : -1;
+      const int64_t rowoff = mv ? ta.out + p.Cm.off(static_cast<uint32_t>(m)) : -1;
       const int64_t rowoff2 = (mv && p.C2) ? p.C2m.off(static_cast<uint32_t>(m)) : -1;
       if (m_major) {
         // lanes are consecutive rows: store column by column straight from registers
@@ -703,6 +716,24 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
   }
 }
 
+// C = sum over the k ranges, in order, + beta C (C2 likewise).
+__global__ void __launch_bounds__(256) split_k_sum_kernel(SplitParams p, const double* part) {
+  const int64_t total = p.M * p.N;
+  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
+       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < p.nsplit; ++q) v += part[q * total + e];
+    const uint32_t m = static_cast<uint32_t>(e / p.N), n = static_cast<uint32_t>(e - m * p.N);
+    double* c = p.C + p.Cm.off(m) + p.Cn.off(n);
+    *c = p.beta != 0.0 ? v + p.beta * *c : v;
+    if (p.C2) {
+      c = p.C2 + p.C2m.off(m) + p.C2n.off(n);
+      *c = p.beta != 0.0 ? v + p.beta * *c : v;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                               const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -747,9 +778,24 @@ inline int64_t rup(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
 int digits_of(const Contraction& g) { return g.digits == 7 ? 7 : 4; }
 
+// Partials of the k ranges of a contraction packed over Kp.
+int parts_of(const Contraction& g, int64_t Kp) {
+  const int D = digits_of(g);
+  return split_k_parts(rup(g.M, TM) / TM * (rup(g.N, tile_n(D)) / tile_n(D)), g.M, g.N, Kp, D);
+}
+size_t part_bytes(const Contraction& g, int64_t Kp) {
+  const int n = parts_of(g, Kp);
+  return n > 1 ? rup(n * g.M * g.N * 8, 1024) : 0;
+}
+// The most any panel of the contraction may need (a shorter panel may take more parts).
+size_t part_bound(const Contraction& g, int64_t Kp) {
+  const int64_t n = split_k_most(g.M, g.N, Kp);
+  return n > 1 ? rup(n * g.M * g.N * 8, 1024) : 0;
+}
+
 struct Layout2 {
   int64_t Mp, Np, Kp;
-  size_t a_bytes, b_bytes, meta_bytes;
+  size_t a_bytes, b_bytes, meta_bytes, part_bytes;
 };
 Layout2 layout_of(const Contraction& g) {
   const int D = digits_of(g);
@@ -760,6 +806,7 @@ Layout2 layout_of(const Contraction& g) {
   L.a_bytes = rup(static_cast<int64_t>(D * L.Mp * L.Kp), 1024);
   L.b_bytes = rup(static_cast<int64_t>(D * L.Np * L.Kp), 1024);
   L.meta_bytes = rup((L.Mp + L.Np) * (8 + 4), 1024);
+  L.part_bytes = part_bytes(g, L.Kp);
   return L;
 }
 
@@ -882,7 +929,7 @@ size_t gemm_split_scratch_bytes(const Contraction& g) {
   Contraction h = g;
   h.K = std::min(g.K, panel_len(g));
   const Layout2 L = layout_of(h);
-  return L.a_bytes + L.b_bytes + L.meta_bytes;
+  return L.a_bytes + L.b_bytes + L.meta_bytes + part_bound(g, L.Kp);
 }
 
 size_t split_packed_b_bytes(const Contraction& g) {
@@ -892,7 +939,7 @@ size_t split_packed_b_bytes(const Contraction& g) {
 
 size_t split_scratch_bytes_packed_b(const Contraction& g) {
   const Layout2 L = layout_of(g);
-  return L.a_bytes + L.meta_bytes;
+  return L.a_bytes + L.meta_bytes + part_bound(g, L.Kp);
 }
 
 bool split_single_panel(const Contraction& g) { return g.K <= panel_len(g) && g.batch == 1; }
@@ -936,7 +983,8 @@ void gemm_split(const Contraction& g, cudaStream_t s, SplitScratch& ws) {
 namespace {
 
 template <class F>
-void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, SplitParams sp, cudaStream_t s) {
+void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, SplitParams sp, double* part,
+                 cudaStream_t s) {
   static std::atomic<int> sms{0};
   int n = sms.load();
   if (!n) {
@@ -948,16 +996,37 @@ void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, SplitParams sp, c
     sms.store(n);
   }
   sp.nkb = static_cast<int>((sp.Kp + F::TK - 1) / F::TK);
-  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(sp.nMt * sp.nNt, n)));
+  sp.kb_len = sp.nkb;
+  sp.part_stride = 0;
+  SplitParams out = sp;
+  if (part) {
+    sp.kb_len = (sp.nkb + sp.nsplit - 1) / sp.nsplit;
+    sp.nsplit = (sp.nkb + sp.kb_len - 1) / sp.kb_len;
+    out.nsplit = sp.nsplit;
+    sp.part_stride = sp.M * sp.N;
+    sp.C = part;
+    sp.C2 = nullptr;
+    sp.Cm = mkax(sp.M, 0, sp.N);
+    sp.Cn = mkax(sp.N, 0, 1);
+    sp.beta = 0.0;
+  }
+  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(sp.nMt * sp.nNt * sp.nsplit, n)));
   split_kernel_persistent<F><<<grid, 320, smem_bytes<F>(), s>>>(ta, tb, sp);
   CC_LAUNCH_CHECK();
   g_split_launches.fetch_add(1);
+  if (part) {
+    split_k_sum_kernel<<<grid_for(out.M * out.N, 256), 256, 0, s>>>(out, part);
+    CC_LAUNCH_CHECK();
+    g_split_launches.fetch_add(1);
+  }
 }
 
-// The output side of a contraction and the runs of its packed rows -> one launch.
+// The output side of a contraction and the runs of its packed rows -> one launch, or with
+// room for partials (part_bytes) one launch over the k ranges and their sum.
 void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t Ap,
             const SplitRuns& ar, int64_t nra, void* Bpk, const int* eb, int64_t Bp,
-            const SplitRuns& br, int64_t nrb, int64_t Kp, cudaStream_t s, SplitScratch& ws) {
+            const SplitRuns& br, int64_t nrb, int64_t Kp, double* part, cudaStream_t s,
+            SplitScratch& ws) {
   const int tn = tile_n(digits), tk = digits == 7 ? Form<7>::TK : Form<4>::TK;
   const CUtensorMap ta = make_map(Apk, digits, Ap, Kp, tk, TM);
   const CUtensorMap tb = make_map(Bpk, digits, Bp, Kp, tk, tn);
@@ -972,6 +1041,7 @@ void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t 
   sp.alpha = g.alpha; sp.beta = g.beta;
   sp.ea = ea; sp.eb = eb;
   sp.error = ws.error;
+  sp.nsplit = part ? parts_of(g, Kp) : 1;
   sp.a_run = ar.run; sp.a_stride = ar.stride; sp.a_base = ar.base;
   sp.a_tiles = (ar.run + TM - 1) / TM; sp.nMt = nra * sp.a_tiles;
   sp.b_run = br.run; sp.b_stride = br.stride; sp.b_base = br.base;
@@ -979,16 +1049,17 @@ void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t 
   if (sp.nMt * sp.nNt >= (int64_t(1) << 31) || Ap >= (int64_t(1) << 31) ||
       Bp >= (int64_t(1) << 31) || Kp >= (int64_t(1) << 31))
     throw Error(ERR_BAD_SHAPE, "gemm_split: extent too large");
-  if (digits == 7) launch_form<Form<7>>(ta, tb, sp, s);
-  else launch_form<Form<4>>(ta, tb, sp, s);
+  if (digits == 7) launch_form<Form<7>>(ta, tb, sp, part, s);
+  else launch_form<Form<4>>(ta, tb, sp, part, s);
 }
 
 void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const SplitPackedB* pb) {
   const Layout2 L = layout_of(g);
   const int D = digits_of(g);
   // with a pre-packed B the scratch holds A and the metadata only
-  const size_t need = L.a_bytes + (pb ? 0 : L.b_bytes) + L.meta_bytes;
-  if (need > ws.bytes) throw Error(ERR_OUT_OF_MEMORY, "gemm_split: scratch too small");
+  const size_t base = L.a_bytes + (pb ? 0 : L.b_bytes) + L.meta_bytes;
+  if (base + L.part_bytes > ws.bytes)
+    throw Error(ERR_OUT_OF_MEMORY, "gemm_split: scratch too small");
   unsigned char* p = static_cast<unsigned char*>(ws.p);
   void* Apk = p;
   void* Bpk = p + L.a_bytes;
@@ -1012,7 +1083,8 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const S
   SplitRuns ar, br;
   ar.run = g.M;
   br.run = g.N;
-  launch(g, D, Apk, aexp, L.Mp, ar, 1, Bpk, bexp, L.Np, br, 1, L.Kp, s, ws);
+  double* part = L.part_bytes ? reinterpret_cast<double*>(p + base) : nullptr;
+  launch(g, D, Apk, aexp, L.Mp, ar, 1, Bpk, bexp, L.Np, br, 1, L.Kp, part, s, ws);
 }
 
 }  // namespace
@@ -1022,7 +1094,7 @@ namespace {
 struct ComplexLayout {
   int64_t Mp, Np, Kp;
   int na, nb;            // forms of A and of B
-  size_t a_bytes, b_bytes, meta_bytes;  // per form; all forms
+  size_t a_bytes, b_bytes, meta_bytes, part_bytes;  // slices per form, meta of all forms
 };
 ComplexLayout complex_layout(const Contraction& g, int64_t K) {
   const int D = digits_of(g);
@@ -1035,6 +1107,7 @@ ComplexLayout complex_layout(const Contraction& g, int64_t K) {
   L.a_bytes = rup(D * L.Mp * L.Kp, 1024);
   L.b_bytes = rup(D * L.Np * L.Kp, 1024);
   L.meta_bytes = rup((L.na * L.Mp + L.nb * L.Np) * (8 + 4), 1024);
+  L.part_bytes = part_bytes(g, L.Kp);
   return L;
 }
 int64_t complex_panel_len(const Contraction& g) {
@@ -1044,12 +1117,13 @@ int64_t complex_panel_len(const Contraction& g) {
   return std::max<int64_t>(KPAD, P / KPAD * KPAD);
 }
 size_t complex_bytes(const ComplexLayout& L) {
-  return L.na * L.a_bytes + L.nb * L.b_bytes + L.meta_bytes;
+  return L.na * L.a_bytes + L.nb * L.b_bytes + L.meta_bytes + L.part_bytes;
 }
 }  // namespace
 
 size_t gemm_split_complex_scratch_bytes(const Contraction& g) {
-  return complex_bytes(complex_layout(g, std::min(g.K, complex_panel_len(g))));
+  const ComplexLayout L = complex_layout(g, std::min(g.K, complex_panel_len(g)));
+  return complex_bytes(L) - L.part_bytes + part_bound(g, L.Kp);
 }
 
 void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
@@ -1101,6 +1175,9 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
       }
     }
     pack(ops, 3, rows, D, s);
+    double* part_mem = L.part_bytes ? reinterpret_cast<double*>(p + L.na * L.a_bytes +
+                                                                L.nb * L.b_bytes + L.meta_bytes)
+                                    : nullptr;
     SplitRuns ar, br;
     ar.run = h.M;
     br.run = h.N;
@@ -1113,7 +1190,8 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
         c.C.p = g.C.p + c_im;
         if (g.C2.p) c.C2.p = g.C2.p + c_im;
       }
-      launch(c, D, A.dst, A.rexp, L.Mp, ar, 1, B.dst, B.rexp, L.Np, br, 1, L.Kp, s, ws);
+      launch(c, D, A.dst, A.rexp, L.Mp, ar, 1, B.dst, B.rexp, L.Np, br, 1, L.Kp,
+             part_mem, s, ws);
     }
   }
 }
@@ -1166,8 +1244,8 @@ void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const Spl
     return nr;
   };
   const int64_t nra = check(ar, g.M, A.R, "A"), nrb = check(br, g.N, B.R, "B");
-  launch(g, A.digits, A.slices, A.exps, A.Rp, ar, nra, B.slices, B.exps, B.Rp, br, nrb, A.Kp, s,
-         ws);
+  launch(g, A.digits, A.slices, A.exps, A.Rp, ar, nra, B.slices, B.exps, B.Rp, br, nrb, A.Kp,
+         nullptr, s, ws);
 }
 
 }  // namespace cc4s_b200

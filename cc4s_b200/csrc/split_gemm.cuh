@@ -16,6 +16,8 @@
 // A row or column holding an Inf or NaN gives NaN in all its outputs.
 #pragma once
 
+#include <algorithm>
+
 #include "gemm_f64.cuh"
 
 namespace cc4s_b200 {
@@ -25,6 +27,26 @@ struct SplitScratch {
   size_t bytes = 0;
   int* error = nullptr;  // device flag: non-zero if a bounded wait gave up
 };
+
+// Ranges of k that share out the SMs when an output has few tiles (each range writes its
+// own FP64 partial, added in order afterwards): the number with the least time by waves of
+// 148 tiles, a k costing `per_k` microseconds and a tile 4 for its drain and store.
+inline int64_t split_k_most(int64_t M, int64_t N, int64_t K) {
+  return std::min<int64_t>(std::min<int64_t>(K / 1024, 40),
+                           (int64_t(1) << 23) / std::max<int64_t>(M * N, 1));
+}
+inline int split_k_parts(int64_t tiles, int64_t M, int64_t N, int64_t K, int digits) {
+  const double per_k = digits == 7 ? 0.019 : 0.012;
+  const int64_t most = split_k_most(M, N, K);
+  int best = 1;
+  double least = 0.0;
+  for (int n = 1; n <= std::max<int64_t>(most, 1); ++n) {
+    const double t = double((tiles * n + 147) / 148) * (per_k * double(K) / n + 4.0) +
+                     (n > 1 ? 6.0 : 0.0);
+    if (n == 1 || t < least) { best = n; least = t; }
+  }
+  return best;
+}
 
 // Same contraction semantics as gemm() (two-level index maps, optional C2).
 // The batch dimension must be 1.  Falls back to nothing: throws if the
