@@ -37,7 +37,7 @@ constexpr int KPAD = 32;                         // K step of one MMA: packed K 
 // |digit product| <= 2^14, at most 7 products per group and k: exact in S32 up to here
 constexpr int KCHUNK = 16384;
 constexpr uint32_t WAIT_LIMIT = 1u << 28;         // bounded mbarrier waits
-constexpr int64_t RASTER_M = 8;                  // tile rows per raster group
+constexpr uint32_t RASTER_M = 8;                 // tile rows per raster group
 constexpr int WBUF_DOUBLES = 32 * 16;            // transpose buffer of one epilogue warp
 constexpr int EXP_NONFINITE = INT_MAX;           // exponent of a row holding Inf or NaN
 
@@ -97,7 +97,7 @@ struct PackArgs {
 // forms in a complex one.
 struct PackSet {
   PackArgs op[3];
-  int64_t end[3];         // work items of the operands, cumulative; the last is the total
+  uint32_t end[3];        // work items of the operands, cumulative; the last is the total
 };
 
 // Packing works on tiles of 64 rows x 64 k staged in shared memory.  The row and
@@ -156,12 +156,13 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
 __global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackSet pp, int kstrip) {
   __shared__ unsigned long long part[8][PR];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int64_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
+  for (uint32_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
     const int which = it < pp.end[0] ? 0 : it < pp.end[1] ? 1 : 2;
     const PackArgs& a = pp.op[which];
-    const int64_t w = which ? it - pp.end[which - 1] : it;
-    const int64_t nks = (a.K + kstrip - 1) / kstrip;
-    const int64_t r0 = (w / nks) * PR, kbeg = (w % nks) * kstrip;
+    const uint32_t w = which ? it - pp.end[which - 1] : it;
+    const uint32_t nks = static_cast<uint32_t>(a.K + kstrip - 1) / static_cast<uint32_t>(kstrip);
+    const uint32_t wr = w / nks;
+    const int64_t r0 = int64_t(wr) * PR, kbeg = int64_t(w - wr * nks) * kstrip;
     const int64_t kend = min(a.K, kbeg + kstrip);
     if (a.r_contig) {  // lanes on rows; the eight warps take every eighth k
       unsigned long long m[2] = {0, 0};
@@ -239,12 +240,12 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
   __shared__ PackTile t;
   __shared__ double scale_s[2][PR];
   const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  for (int64_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
+  for (uint32_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
     const int which = it < pp.end[0] ? 0 : it < pp.end[1] ? 1 : 2;
     const PackArgs& a = pp.op[which];
-    const int64_t w = which ? it - pp.end[which - 1] : it;
-    const int64_t nk = (a.Kp + PKT - 1) / PKT, pl = a.Rp * a.Kp;
-    const int64_t r0 = (w / nk) * PR, k0 = (w % nk) * PKT;
+    const uint32_t w = which ? it - pp.end[which - 1] : it;
+    const uint32_t nk = static_cast<uint32_t>(a.Kp + PKT - 1) / PKT, wr = w / nk;
+    const int64_t pl = a.Rp * a.Kp, r0 = int64_t(wr) * PR, k0 = int64_t(w - wr * nk) * PKT;
     if (threadIdx.x < PR) {
       const int64_t r = r0 + threadIdx.x;
       double s1 = 0.0, s2 = 0.0;  // their product 2^(8 NS - 2 - e), each in the normal range
@@ -310,9 +311,10 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 // Bounded wait for the phase with the given parity: gives up after
-// WAIT_LIMIT polls or 2 seconds, whichever comes first; returns false then.
+// WAIT_LIMIT polls or 2 seconds, whichever comes first; returns false then.  The clock
+// is read only once 1024 polls have failed.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;
   for (uint32_t it = 0; it < WAIT_LIMIT; ++it) {
     uint32_t ok;
     asm volatile(
@@ -320,7 +322,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         " selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     if (ok) return true;
-    if ((it & 1023) == 1023 && global_ns() - t0 > 2000000000ull) return false;
+    if ((it & 1023) == 1023) {
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 2000000000ull) return false;
+    }
   }
   return false;
 }
@@ -467,22 +473,25 @@ struct TileAt {
   int kb0, nkb;     // k-blocks of the work item
   int64_t out;      // offset of its output
 };
+// (32-bit arithmetic: every role divides its way here once per tile, and a 64-bit division
+// is a call of some hundred instructions; tiles and work items stay below 2^31.)
 template <int TN>
-__device__ __forceinline__ TileAt tile_at(const SplitParams& p, int64_t t) {
+__device__ __forceinline__ TileAt tile_at(const SplitParams& p, uint32_t t) {
   TileAt a;
-  const int64_t tiles = p.nMt * p.nNt, part = t / tiles;
+  const uint32_t nM = static_cast<uint32_t>(p.nMt), nN = static_cast<uint32_t>(p.nNt);
+  const uint32_t tiles = nM * nN, part = p.nsplit > 1 ? t / tiles : 0;
   t -= part * tiles;
   a.kb0 = static_cast<int>(part) * p.kb_len;
   a.nkb = min(p.kb_len, p.nkb - a.kb0);
   a.out = part * p.part_stride;
-  const int64_t nM = p.nMt, nN = p.nNt;
-  const int64_t per_group = RASTER_M * nN, group = t / per_group;
-  const int64_t first = group * RASTER_M;
-  const int64_t rows = nM - first < RASTER_M ? nM - first : RASTER_M;
-  const int64_t in = t - group * per_group;
-  const int64_t tm = first + in % rows, tn = in / rows;
-  const int64_t rm = tm / p.a_tiles, om = (tm - rm * p.a_tiles) * TM;
-  const int64_t rn = tn / p.b_tiles, on = (tn - rn * p.b_tiles) * TN;
+  const uint32_t per_group = RASTER_M * nN, group = t / per_group;
+  const uint32_t first = group * RASTER_M;
+  const uint32_t rows = nM - first < RASTER_M ? nM - first : RASTER_M;
+  const uint32_t in = t - group * per_group;
+  const uint32_t tn = in / rows, tm = first + in - tn * rows;
+  const uint32_t at = static_cast<uint32_t>(p.a_tiles), bt = static_cast<uint32_t>(p.b_tiles);
+  const uint32_t rm = tm / at, om = (tm - rm * at) * TM;
+  const uint32_t rn = tn / bt, on = (tn - rn * bt) * TN;
   a.m0 = rm * p.a_run + om;
   a.n0 = rn * p.b_run + on;
   a.pa = p.a_base + rm * p.a_stride + om;
@@ -509,7 +518,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
   volatile int* abort_v = &abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ntiles = p.nMt * p.nNt * p.nsplit;
+  const uint32_t ntiles = static_cast<uint32_t>(p.nMt * p.nNt * p.nsplit);
   constexpr int KB_PER_CHUNK = KCHUNK / TK;
   auto chunks_of = [](int nkb) { return (nkb + KB_PER_CHUNK - 1) / KB_PER_CHUNK; };
 
@@ -536,7 +545,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
   if (warp == 0 && lane == 0) {
     // ---- TMA producer: every k-block of every tile of this CTA ----
     uint32_t it = 0;
-    for (int64_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
       const TileAt ta = tile_at<TN>(p, t);
       for (int kb = ta.kb0; kb < ta.kb0 + ta.nkb; ++kb, ++it) {
         const int s = it % NST;
@@ -555,7 +564,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer: chunks of all tiles, global stage and chunk counters ----
     uint32_t it = 0, q = 0;
-    for (int64_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < ntiles && !*abort_v; t += gridDim.x) {
       const TileAt ta = tile_at<TN>(p, t);
       const int nchunks = chunks_of(ta.nkb), kb_last = ta.kb0 + ta.nkb;
       int kb = ta.kb0;
@@ -590,7 +599,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
     double* wb = wbufs + (warp - 2) * WBUF_DOUBLES;
     const bool m_major = p.Cm.s_i == 1 && p.Cm.inner > 1;  // output contiguous along rows
     uint32_t q = 0;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
       if (__any_sync(0xffffffffu, *abort_v != 0)) break;
       const TileAt ta = tile_at<TN>(p, t);
       const int64_t m0 = ta.m0, n0 = ta.n0;
@@ -844,7 +853,8 @@ void pack(const PackArgs* const* ops, int n, int64_t rows, int digits, cudaStrea
   auto tiles = [](const PackArgs& x) { return (x.Rp / PR) * ((x.Kp + PKT - 1) / PKT); };
   auto items = [&](auto&& count) {
     int64_t t = 0;
-    for (int k = 0; k < 3; ++k) pp.end[k] = t += k < n ? count(pp.op[k]) : 0;
+    for (int k = 0; k < 3; ++k) pp.end[k] = static_cast<uint32_t>(t += k < n ? count(pp.op[k]) : 0);
+    if (t >= (int64_t(1) << 31)) throw Error(ERR_BAD_SHAPE, "gemm_split: operand too large");
     return t;
   };
   int64_t work = items(strips);
@@ -1046,7 +1056,7 @@ void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t 
   sp.a_tiles = (ar.run + TM - 1) / TM; sp.nMt = nra * sp.a_tiles;
   sp.b_run = br.run; sp.b_stride = br.stride; sp.b_base = br.base;
   sp.b_tiles = (br.run + tn - 1) / tn; sp.nNt = nrb * sp.b_tiles;
-  if (sp.nMt * sp.nNt >= (int64_t(1) << 31) || Ap >= (int64_t(1) << 31) ||
+  if (sp.nMt * sp.nNt * sp.nsplit >= (int64_t(1) << 31) || Ap >= (int64_t(1) << 31) ||
       Bp >= (int64_t(1) << 31) || Kp >= (int64_t(1) << 31))
     throw Error(ERR_BAD_SHAPE, "gemm_split: extent too large");
   if (digits == 7) launch_form<Form<7>>(ta, tb, sp, part, s);
