@@ -193,6 +193,15 @@ void triples_energy(const double* S, const double* S_im, const double* t1, const
                     const double* eps_p, const TriplesBlock& b, const double coef[6],
                     double* ws, double* out_dev, Stream s, const double* M = nullptr,
                     const double* M_im = nullptr);
+// The same sums of a block array that holds the connected part W alone: every (a, b, c)
+// cube of o^3 elements is staged in shared memory with its singles added there, so the
+// block array is read once and its singles are never written.  Available while the cube
+// fits (triples_cube_fits: o up to 29, 23 on the complex path).
+bool triples_cube_fits(int64_t o, bool cplx);
+void triples_energy_connected(const double* W, const double* W_im, const double* t1,
+                              const double* t1_im, const double* V, const double* V_im,
+                              const double* eps_h, const double* eps_p, const TriplesBlock& b,
+                              const double coef[6], double* ws, double* out_dev, Stream s);
 // The block-triple part of the CR-(T) denominator of the cT branch (ct::getDenominator,
 // CompleteTriples.cxx:138-162, reduced to sum y conj(Z) / D): out_dev[0] = sum Re y Re Z / D,
 // out_dev[1] = sum Im y Im Z / D over the block, with

@@ -1123,39 +1123,43 @@ __device__ __forceinline__ Cplx triples_singles_at(const TriplesArgs& a, int64_t
           t1r * v23m + t1m * v23r + t2r * v13m + t2m * v13r + t3r * v12m + t3m * v12r};
 }
 
-template <bool CPLX>
+// I: the index type of the block array (32 bits below 2^31 elements: a 64-bit division
+// costs more than the element's arithmetic).
+template <bool CPLX, class I>
 __global__ void triples_singles_kernel(TriplesArgs a) {
-  const int64_t L23 = a.L2 * a.L3;
+  const I L23 = static_cast<I>(a.L2 * a.L3), L3 = static_cast<I>(a.L3);
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < a.total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t q1 = e / L23, r = e - q1 * L23, q2 = r / a.L3, q3 = r - q2 * a.L3;
+    const I q1 = static_cast<I>(e) / L23, r = static_cast<I>(e) - q1 * L23, q2 = r / L3,
+            q3 = r - q2 * L3;
     const Cplx x = triples_singles_at<CPLX>(a, a.P1 + q1, a.P2 + q2, a.P3 + q3);
     a.Sw[e] = x.re;
     if (CPLX) a.Swi[e] = x.im;
   }
 }
 
-template <bool CPLX>
+template <bool CPLX, class I>
 __global__ void triples_energy_kernel(TriplesArgs a) {
-  const int64_t L23 = a.L2 * a.L3, o = a.o;
+  const I L23 = static_cast<I>(a.L2 * a.L3), L3 = static_cast<I>(a.L3), o = static_cast<I>(a.o);
   const int64_t X1 = a.P1 / o, X2 = a.P2 / o, X3 = a.P3 / o;
   double acc[2] = {0.0, 0.0};
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < a.total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t q1 = e / L23, r = e - q1 * L23, q2 = r / a.L3, q3 = r - q2 * a.L3;
-    const int64_t x1 = q1 / o, x2 = q2 / o, x3 = q3 / o;
-    const int64_t y0 = q1 - x1 * o, y1 = q2 - x2 * o, y2 = q3 - x3 * o;
+    const I q1 = static_cast<I>(e) / L23, r = static_cast<I>(e) - q1 * L23, q2 = r / L3,
+            q3 = r - q2 * L3;
+    const I x1 = q1 / o, x2 = q2 / o, x3 = q3 / o;
+    const I y0 = q1 - x1 * o, y1 = q2 - x2 * o, y2 = q3 - x3 * o;
     const Cplx sg = triples_singles_at<CPLX>(a, a.P1 + q1, a.P2 + q2, a.P3 + q3);
     const double d = a.eh[y0] + a.eh[y1] + a.eh[y2] - a.ep[X1 + x1] - a.ep[X2 + x2] -
                      a.ep[X3 + x3];
-    const int64_t b1 = x1 * o * L23, b2 = x2 * o * a.L3, b3 = x3 * o;
+    const I b1 = x1 * o * L23, b2 = x2 * o * L3, b3 = x3 * o;
     // the hole permutations 012, 021, 102, 120, 201, 210 of the pair (a, b, c)
-    const int64_t idx[6] = {e,
-                            b1 + y0 * L23 + b2 + y2 * a.L3 + b3 + y1,
-                            b1 + y1 * L23 + b2 + y0 * a.L3 + b3 + y2,
-                            b1 + y1 * L23 + b2 + y2 * a.L3 + b3 + y0,
-                            b1 + y2 * L23 + b2 + y0 * a.L3 + b3 + y1,
-                            b1 + y2 * L23 + b2 + y1 * a.L3 + b3 + y0};
+    const I idx[6] = {static_cast<I>(e),
+                            b1 + y0 * L23 + b2 + y2 * L3 + b3 + y1,
+                            b1 + y1 * L23 + b2 + y0 * L3 + b3 + y2,
+                            b1 + y1 * L23 + b2 + y2 * L3 + b3 + y0,
+                            b1 + y2 * L23 + b2 + y0 * L3 + b3 + y1,
+                            b1 + y2 * L23 + b2 + y1 * L3 + b3 + y0};
     double yr = 0.0, yi = 0.0;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -1167,6 +1171,99 @@ __global__ void triples_energy_kernel(TriplesArgs a) {
     const double wr = a.M ? a.M[e] : a.S[e] - sg.re;
     acc[0] += wr * yr * inv;
     if (CPLX) acc[1] += (a.M ? a.Mi[e] : a.Si[e] - sg.im) * yi * inv;
+  }
+  block_sum<2>(acc);
+  if (threadIdx.x == 0) {
+    a.ws[2 * blockIdx.x] = acc[0];
+    a.ws[2 * blockIdx.x + 1] = acc[1];
+  }
+}
+
+// Shared memory of one cube: the o^3 values S(y0, y1, y2) with odd strides (reads along any
+// of the three indices hit distinct banks), the three o x o blocks of V, the three rows of
+// t1 per plane, and eps_h.
+__host__ __device__ inline int cube_s1(int o) { return o | 1; }
+__host__ __device__ inline int cube_s0(int o) { return (o * cube_s1(o)) | 1; }
+inline size_t cube_smem(int64_t o, bool cplx) {
+  const size_t plane = o * cube_s0(static_cast<int>(o)) + 3 * o * o + 3 * o;
+  return ((cplx ? 2 : 1) * plane + o) * sizeof(double);
+}
+
+// One (a, b, c) cube per iteration of a block (triples_energy_connected in ops.h).  The
+// element-wise kernel above gathers six permuted elements of S and three of V per element
+// from L1 / L2 after five 64-bit divisions; here S and V are read coalesced and the
+// permutations come from shared memory ((T) block loop of 16/128 in FP64 174 -> 139 ms, of
+// 21/163 in the split form 542 -> 437 ms, with the singles pass that this makes needless).
+template <bool CPLX>
+__global__ void __launch_bounds__(512) triples_cube_kernel(TriplesArgs a, uint32_t n2, uint32_t n3,
+                                                           uint32_t ncubes) {
+  extern __shared__ double cube[];
+  const int o = static_cast<int>(a.o), s1 = cube_s1(o), s0 = cube_s0(o), o2 = o * o, o3 = o2 * o;
+  double* v = cube + o * s0;          // V23, V13, V12
+  double* t = v + 3 * o2;             // t1 of the three pairs
+  double* im = t + 3 * o;             // the imaginary plane, laid out alike
+  double* eh = cube + (CPLX ? 2 : 1) * (o * s0 + 3 * o2 + 3 * o);
+  const ptrdiff_t dv = v - cube, dt = t - cube;
+  for (int k = threadIdx.x; k < o; k += blockDim.x) eh[k] = a.eh[k];
+  double acc[2] = {0.0, 0.0};
+  for (uint32_t c = blockIdx.x; c < ncubes; c += gridDim.x) {
+    const uint32_t x3 = c % n3, c12 = c / n3, x2 = c12 % n2, x1 = c12 / n2;
+    const int64_t p1 = a.P1 + int64_t(x1) * o, p2 = a.P2 + int64_t(x2) * o,
+                  p3 = a.P3 + int64_t(x3) * o;
+    const int64_t base = (int64_t(x1) * o * a.L2 + int64_t(x2) * o) * a.L3 + int64_t(x3) * o;
+    const double ea = a.ep[p1 / o] + a.ep[p2 / o] + a.ep[p3 / o];
+    for (int k = threadIdx.x; k < o2; k += blockDim.x) {
+      const int y = k / o, z = k - y * o;
+      v[k] = a.V[(p2 + y) * a.n1 + p3 + z];
+      v[o2 + k] = a.V[(p1 + y) * a.n1 + p3 + z];
+      v[2 * o2 + k] = a.V[(p1 + y) * a.n1 + p2 + z];
+      if (CPLX) {
+        im[dv + k] = a.Vi[(p2 + y) * a.n1 + p3 + z];
+        im[dv + o2 + k] = a.Vi[(p1 + y) * a.n1 + p3 + z];
+        im[dv + 2 * o2 + k] = a.Vi[(p1 + y) * a.n1 + p2 + z];
+      }
+    }
+    for (int k = threadIdx.x; k < 3 * o; k += blockDim.x) {
+      const int64_t q = (k < o ? p1 : k < 2 * o ? p2 - o : p3 - 2 * o) + k;
+      t[k] = a.t1[q];
+      if (CPLX) im[dt + k] = a.t1i[q];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < o3; e += blockDim.x) {
+      const int y0 = e / o2, r = e - y0 * o2, y1 = r / o, y2 = r - y1 * o;
+      const int64_t g = base + (y0 * a.L2 + y1) * a.L3 + y2;
+      const int v23 = y1 * o + y2, v13 = o2 + y0 * o + y2, v12 = 2 * o2 + y0 * o + y1;
+      const double t1 = t[y0], t2 = t[o + y1], t3 = t[2 * o + y2];
+      double sr = t1 * v[v23] + t2 * v[v13] + t3 * v[v12];
+      if (CPLX) {
+        const double* vi = im + dv;
+        const double u1 = im[dt + y0], u2 = im[dt + o + y1], u3 = im[dt + 2 * o + y2];
+        sr -= u1 * vi[v23] + u2 * vi[v13] + u3 * vi[v12];
+        const double si = t1 * vi[v23] + u1 * v[v23] + t2 * vi[v13] + u2 * v[v13] +
+                          t3 * vi[v12] + u3 * v[v12];
+        im[y0 * s0 + y1 * s1 + y2] = a.Si[g] + si;
+      }
+      cube[y0 * s0 + y1 * s1 + y2] = a.S[g] + sr;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < o3; e += blockDim.x) {
+      const int y0 = e / o2, r = e - y0 * o2, y1 = r / o, y2 = r - y1 * o;
+      const int64_t g = base + (y0 * a.L2 + y1) * a.L3 + y2;
+      // the hole permutations 012, 021, 102, 120, 201, 210
+      const int idx[6] = {y0 * s0 + y1 * s1 + y2, y0 * s0 + y2 * s1 + y1, y1 * s0 + y0 * s1 + y2,
+                          y1 * s0 + y2 * s1 + y0, y2 * s0 + y0 * s1 + y1, y2 * s0 + y1 * s1 + y0};
+      double yr = 0.0, yi = 0.0;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        if (a.coef[k] == 0.0) continue;
+        yr += a.coef[k] * cube[idx[k]];
+        if (CPLX) yi += a.coef[k] * im[idx[k]];
+      }
+      const double inv = 1.0 / (eh[y0] + eh[y1] + eh[y2] - ea);
+      acc[0] += a.S[g] * yr * inv;
+      if (CPLX) acc[1] += a.Si[g] * yi * inv;
+    }
+    __syncthreads();
   }
   block_sum<2>(acc);
   if (threadIdx.x == 0) {
@@ -1238,10 +1335,13 @@ void triples_singles(double* S, double* S_im, const double* t1, const double* t1
   a.Sw = S; a.Swi = S_im;
   if (a.total <= 0) return;
   const unsigned grid = grid_for(a.total, 256, 148 * 16);
+  const bool small = a.total < (int64_t(1) << 31);
   if (S_im)
-    triples_singles_kernel<true><<<grid, 256, 0, s>>>(a);
+    small ? triples_singles_kernel<true, uint32_t><<<grid, 256, 0, s>>>(a)
+          : triples_singles_kernel<true, int64_t><<<grid, 256, 0, s>>>(a);
   else
-    triples_singles_kernel<false><<<grid, 256, 0, s>>>(a);
+    small ? triples_singles_kernel<false, uint32_t><<<grid, 256, 0, s>>>(a)
+          : triples_singles_kernel<false, int64_t><<<grid, 256, 0, s>>>(a);
   CC_LAUNCH_CHECK();
   count();
 }
@@ -1255,10 +1355,41 @@ void triples_energy(const double* S, const double* S_im, const double* t1, const
   a.S = S; a.Si = S_im; a.eh = eps_h; a.ep = eps_p; a.ws = ws;
   a.M = M; a.Mi = M_im;
   for (int k = 0; k < 6; ++k) a.coef[k] = coef[k];
+  const bool small = a.total < (int64_t(1) << 31);
   if (S_im)
-    triples_energy_kernel<true><<<RED_BLOCKS, RED_THREADS, 0, s>>>(a);
+    small ? triples_energy_kernel<true, uint32_t><<<RED_BLOCKS, RED_THREADS, 0, s>>>(a)
+          : triples_energy_kernel<true, int64_t><<<RED_BLOCKS, RED_THREADS, 0, s>>>(a);
   else
-    triples_energy_kernel<false><<<RED_BLOCKS, RED_THREADS, 0, s>>>(a);
+    small ? triples_energy_kernel<false, uint32_t><<<RED_BLOCKS, RED_THREADS, 0, s>>>(a)
+          : triples_energy_kernel<false, int64_t><<<RED_BLOCKS, RED_THREADS, 0, s>>>(a);
+  CC_LAUNCH_CHECK();
+  count();
+  finish_kernel<<<1, 256, 0, s>>>(out_dev, ws, RED_BLOCKS, 2, 1.0, 1.0, 1.0, 1.0);
+  CC_LAUNCH_CHECK();
+  count();
+}
+
+bool triples_cube_fits(int64_t o, bool cplx) { return o <= 64 && cube_smem(o, cplx) <= 227 * 1024; }
+
+void triples_energy_connected(const double* W, const double* W_im, const double* t1,
+                              const double* t1_im, const double* V, const double* V_im,
+                              const double* eps_h, const double* eps_p, const TriplesBlock& b,
+                              const double coef[6], double* ws, double* out_dev, Stream s) {
+  TriplesArgs a = triples_args(t1, t1_im, V, V_im, b);
+  a.S = W; a.Si = W_im; a.eh = eps_h; a.ep = eps_p; a.ws = ws;
+  for (int k = 0; k < 6; ++k) a.coef[k] = coef[k];
+  const uint32_t n1 = static_cast<uint32_t>(b.L[0] / b.o), n2 = static_cast<uint32_t>(b.L[1] / b.o),
+                 n3 = static_cast<uint32_t>(b.L[2] / b.o);
+  if (int64_t(n1) * n2 * n3 >= (int64_t(1) << 31))
+    throw Error(ERR_BAD_SHAPE, "triples: block too large");
+  const size_t smem = cube_smem(b.o, W_im != nullptr);
+  auto run = [&](auto kernel) {
+    CC_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)));
+    kernel<<<RED_BLOCKS, 512, smem, s>>>(a, n2, n3, n1 * n2 * n3);
+  };
+  if (W_im) run(triples_cube_kernel<true>);
+  else run(triples_cube_kernel<false>);
   CC_LAUNCH_CHECK();
   count();
   finish_kernel<<<1, 256, 0, s>>>(out_dev, ws, RED_BLOCKS, 2, 1.0, 1.0, 1.0, 1.0);

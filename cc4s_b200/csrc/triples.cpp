@@ -149,7 +149,7 @@ void Triples::residual(const double*, double*) {
 // writes the same elements of S with the same rows and columns (its transpose), so
 // rows of Ac hold [T | -V^h] and columns of Bc hold [V^p | T] along K.
 void Triples::connected(const ops::TriplesBlock& b, const int64_t X[3], const int64_t n[3],
-                        const double* Ac, const double* Bc, double* S) {
+                        const double* Ac, const double* Bc, double* S, bool fresh) {
   static const int PQR[6][3] = {{0, 1, 2}, {1, 0, 2}, {0, 2, 1}, {2, 1, 0}, {2, 0, 1}, {1, 2, 0}};
   const int64_t o = o_, n1 = n1_, kc = kc_;
   const int64_t sP[3] = {b.L[1] * b.L[2], b.L[2], 1};
@@ -168,7 +168,7 @@ void Triples::connected(const ops::TriplesBlock& b, const int64_t X[3], const in
       c.C = vw(S, sP[p], sP[q], o * sP[q], sP[r]);
     }
     c.B = vw(cp(Bc) + (X[q] * n1 + b.P[r]) * kc, 0, 1, n1 * kc, kc);
-    c.alpha = 1.0; c.beta = 1.0;
+    c.alpha = 1.0; c.beta = fresh && &t == PQR ? 0.0 : 1.0;
     zgemm(c, ai_, bi_, si_, false, false, true);
   }
 }
@@ -192,7 +192,7 @@ void Triples::pack_operands(int w, const double* Ac, const double* Bc) {
 }
 
 void Triples::connected_packed(const ops::TriplesBlock& b, const int64_t X[3], const int64_t n[3],
-                               int w, double* S) {
+                               int w, double* S, bool fresh) {
   static const int PQR[6][3] = {{0, 1, 2}, {1, 0, 2}, {0, 2, 1}, {2, 1, 0}, {2, 0, 1}, {1, 2, 0}};
   const int64_t o = o_, n1 = n1_;
   const int64_t sP[3] = {b.L[1] * b.L[2], b.L[2], 1};
@@ -212,7 +212,7 @@ void Triples::connected_packed(const ops::TriplesBlock& b, const int64_t X[3], c
       ar.base = b.P[p] * o; ar.run = c.M; ar.stride = 0;
     }
     br.base = X[q] * n1 + b.P[r]; br.run = b.L[r]; br.stride = n1;
-    c.alpha = 1.0; c.beta = 1.0;
+    c.alpha = 1.0; c.beta = fresh && &t == PQR ? 0.0 : 1.0;
     if (c.M < 64 || c.N < 64) {  // too small for the split form (a ragged last block): FP64
       const double* Ac = w ? AcM_ : Ac_;
       const double* Bc = w ? BcM_ : Bc_;
@@ -229,10 +229,12 @@ void Triples::connected_packed(const ops::TriplesBlock& b, const int64_t X[3], c
       const Sliced& im = sl_[w][1];
       Contraction d = c;
       d.alpha = -1.0;
+      d.beta = 1.0;
       tc_prepacked_(d, A(im), ar, im.B, br);
       d = c;
       d.C.p = S + si_;
       tc_prepacked_(d, A(re), ar, im.B, br);
+      d.beta = 1.0;
       tc_prepacked_(d, A(im), ar, re.B, br);
     }
   }
@@ -477,6 +479,9 @@ TriplesOutcome Triples::run(const double* T) {
   out.setup_seconds += ops::event_ms(e0, e1) * 1e-3;
   const int64_t Lm = nb * o;
   double* Mi = complete_ && cplx_ ? Mb_ + si_ : nullptr;
+  // The block array holds the connected terms alone where the energy adds the singles (the
+  // cT branch needs their sum in memory).
+  const bool cubes = !complete_ && ops::triples_cube_fits(o, cplx_);
   // profile: events around the four phases of every block triple
   std::vector<void*> pev;
   if (profile_) {
@@ -495,23 +500,27 @@ TriplesOutcome Triples::run(const double* T) {
         b.o = o; b.n1 = n1;
         for (int m = 0; m < 3; ++m) { b.P[m] = X[m] * o; b.L[m] = n[m] * o; }
         if (profile_) ops::event_record(pev[5 * t], s_);
-        ops::triples_singles(S_, Si, t1, t1i, Vpphh_, Vi, b, s_);
+        if (!cubes) ops::triples_singles(S_, Si, t1, t1i, Vpphh_, Vi, b, s_);
         if (complete_) zero_(Mb_, (cplx_ ? 2 : 1) * Lm * Lm * Lm);
         if (profile_) ops::event_record(pev[5 * t + 1], s_);
         if (packed) {
-          connected_packed(b, X, n, 0, S_);
-          if (complete_) connected_packed(b, X, n, 1, Mb_);
+          connected_packed(b, X, n, 0, S_, cubes);
+          if (complete_) connected_packed(b, X, n, 1, Mb_, false);
         } else {
-          connected(b, X, n, Ac_, Bc_, S_);
-          if (complete_) connected(b, X, n, AcM_, BcM_, Mb_);
+          connected(b, X, n, Ac_, Bc_, S_, cubes);
+          if (complete_) connected(b, X, n, AcM_, BcM_, Mb_, false);
         }
         if (profile_) ops::event_record(pev[5 * t + 2], s_);
         // (the hole terms ride in the contractions above: the hole phase stays empty)
         if (profile_) ops::event_record(pev[5 * t + 3], s_);
         double coef[6];
         coefficients(A, B, C, coef);
-        ops::triples_energy(S_, Si, t1, t1i, Vpphh_, Vi, sys_.eh, sys_.ep, b, coef, ws_,
-                            slots_ + 2 * t, s_, complete_ ? Mb_ : nullptr, Mi);
+        if (cubes)
+          ops::triples_energy_connected(S_, Si, t1, t1i, Vpphh_, Vi, sys_.eh, sys_.ep, b, coef,
+                                        ws_, slots_ + 2 * t, s_);
+        else
+          ops::triples_energy(S_, Si, t1, t1i, Vpphh_, Vi, sys_.eh, sys_.ep, b, coef, ws_,
+                              slots_ + 2 * t, s_, complete_ ? Mb_ : nullptr, Mi);
         if (complete_)
           ops::triples_cr_sums(S_, Si, t1, t1i, T + n1, cplx_ ? T + plane + n1 : nullptr, sys_.eh,
                                sys_.ep, b, coef, ws_, cr_slots_ + 2 * t, s_);

@@ -86,11 +86,11 @@ class Triples : public Schedule {
   // S += the six permutations of X = sum_d T V^p - sum_l T V^h through the
   // K-concatenated operands Ac (rows (pair, hole)) and Bc (columns (virtual, pair)).
   void connected(const ops::TriplesBlock& b, const int64_t X[3], const int64_t n[3],
-                 const double* Ac, const double* Bc, double* S);
+                 const double* Ac, const double* Bc, double* S, bool fresh);
   // The same six contractions in the split form from operands sliced once per
   // evaluation (w = 0: S from Ac_/Bc_, w = 1: M from AcM_/BcM_).
   void connected_packed(const ops::TriplesBlock& b, const int64_t X[3], const int64_t n[3],
-                        int w, double* S);
+                        int w, double* S, bool fresh);
   // Slices Ac (rows (pair, hole) and (hole, pair)) and Bc (rows (virtual, pair)) of
   // every plane for connected_packed.
   void pack_operands(int w, const double* Ac, const double* Bc);

@@ -775,6 +775,20 @@ void triples_energy(const double* S, const double* S_im, const double* t1, const
   out[1] = acc[1];
 }
 
+bool triples_cube_fits(int64_t, bool) { return true; }
+void triples_energy_connected(const double* W, const double* W_im, const double* t1,
+                              const double* t1_im, const double* V, const double* V_im,
+                              const double* eh, const double* ep, const TriplesBlock& b,
+                              const double coef[6], double* ws, double* out, Stream s) {
+  const int64_t n = b.L[0] * b.L[1] * b.L[2];
+  std::vector<double> S(n), Si(W_im ? n : 0);
+  triples_singles(S.data(), W_im ? Si.data() : nullptr, t1, t1_im, V, V_im, b, s);
+  for (int64_t k = 0; k < n; ++k) S[k] += W[k];
+  for (int64_t k = 0; k < (W_im ? n : 0); ++k) Si[k] += W_im[k];
+  triples_energy(S.data(), W_im ? Si.data() : nullptr, t1, t1_im, V, V_im, eh, ep, b, coef, ws, out,
+                 s, W, W_im);
+}
+
 void triples_cr_sums(const double* S, const double* S_im, const double* t1, const double* t1_im,
                      const double* T2, const double* T2_im, const double* eh, const double* ep,
                      const TriplesBlock& b, const double coef[6], double*, double* out, Stream) {
