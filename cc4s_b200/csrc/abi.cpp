@@ -16,67 +16,53 @@ int energy_noalloc(const double* T1, const double* T2, const double* V, int64_t 
 
 // Reference layout T1[a,i], T2[a,b,i,j] (first index fastest) -> amplitude vector.
 // Complex host buffers are interleaved (re, im); device vectors are planar.
-void Handle::upload_amplitudes(double* dst, const double* T1, const double* T2, double* st) {
+void Handle::upload_amplitudes(double* dst, const double* T1, const double* T2, double* st,
+                               bool check) {
   const int64_t o = shape.o, v = shape.v, n1 = v * o, pl = shape.plane();
-  std::vector<double> h1, h2;
-  for (int64_t p = 0; p < shape.planes; ++p) {
-    const double* s1 = T1;
-    const double* s2 = T2;
-    if (shape.planes > 1) {
-      h1.resize(n1);
-      h2.resize(n1 * n1);
-      for (int64_t k = 0; k < n1; ++k) h1[k] = T1[2 * k + p];
-      for (int64_t k = 0; k < n1 * n1; ++k) h2[k] = T2[2 * k + p];
-      s1 = h1.data();
-      s2 = h2.data();
-    }
-    ops::h2d(st, s1, n1, stream);
-    ops::h2d(st + n1, s2, n1 * n1, stream);
+  const int np = static_cast<int>(shape.planes);
+  for (int p = 0; p < np; ++p) {
+    ops::h2d_staged(st + p * pl, T1 + p, n1, np, stage, stream);
+    ops::h2d_staged(st + p * pl + n1, T2 + p, n1 * n1, np, stage, stream);
+  }
+  if (check && (ops::scan_vertex(st, np * pl, false, stream) & 1))
+    throw Error(ERR_NON_FINITE, "non-finite T2");  // T1 was checked on the host
+  for (int p = 0; p < np; ++p) {
     const int64_t d1[4] = {1, 1, o, v};
     const int p1[4] = {0, 1, 3, 2};
-    ops::permute4(dst + p * pl, st, d1, p1, 1.0, 0.0, stream);
+    ops::permute4(dst + p * pl, st + p * pl, d1, p1, 1.0, 0.0, stream);
     const int64_t d2[4] = {o, o, v, v};  // [j][i][b][a]
     const int p2[4] = {3, 1, 2, 0};      // -> [a][i][b][j]
-    ops::permute4(dst + p * pl + n1, st + n1, d2, p2, 1.0, 0.0, stream);
-    ops::sync(stream);
+    ops::permute4(dst + p * pl + n1, st + p * pl + n1, d2, p2, 1.0, 0.0, stream);
   }
+  ops::sync(stream);
 }
 
 void Handle::download_amplitudes(const double* src, double* T1, double* T2, double* st) {
   const int64_t o = shape.o, v = shape.v, n1 = v * o, pl = shape.plane();
-  std::vector<double> h1, h2;
-  for (int64_t p = 0; p < shape.planes; ++p) {
+  const int np = static_cast<int>(shape.planes);
+  for (int p = 0; p < np; ++p) {
     const int64_t d1[4] = {1, 1, v, o};
     const int p1[4] = {0, 1, 3, 2};
     ops::permute4(st, src + p * pl, d1, p1, 1.0, 0.0, stream);
     const int64_t d2[4] = {v, o, v, o};  // [a][i][b][j]
     const int p2[4] = {3, 1, 2, 0};      // -> [j][i][b][a]
     ops::permute4(st + n1, src + p * pl + n1, d2, p2, 1.0, 0.0, stream);
-    if (shape.planes == 1) {
-      if (T1) ops::d2h(T1, st, n1, stream);
-      if (T2) ops::d2h(T2, st + n1, n1 * n1, stream);
-      ops::sync(stream);
-    } else {
-      h1.resize(n1);
-      h2.resize(n1 * n1);
-      ops::d2h(h1.data(), st, n1, stream);
-      ops::d2h(h2.data(), st + n1, n1 * n1, stream);
-      ops::sync(stream);
-      if (T1) for (int64_t k = 0; k < n1; ++k) T1[2 * k + p] = h1[k];
-      if (T2) for (int64_t k = 0; k < n1 * n1; ++k) T2[2 * k + p] = h2[k];
-    }
+    if (T1) ops::d2h_staged(T1 + p, np, st, n1, stage, stream);
+    if (T2) ops::d2h_staged(T2 + p, np, st + n1, n1 * n1, stage, stream);
   }
 }
 
 void Handle::set_initial(const double* T1, const double* T2) {
   require_inputs();
   if (!T1 || !T2) throw Error(ERR_INVALID_ARGUMENT, "null amplitudes");
+  // small ones are checked here, large ones on the device once they are there
   const int64_t n1 = shape.n1(), np = shape.planes;
+  const bool large = n1 * n1 >= ops::STAGED_MIN;
   for (int64_t k = 0; k < n1 * np; ++k)
     if (!std::isfinite(T1[k])) throw Error(ERR_NON_FINITE, "non-finite T1");
-  for (int64_t k = 0; k < n1 * n1 * np; ++k)
+  for (int64_t k = 0; !large && k < n1 * n1 * np; ++k)
     if (!std::isfinite(T2[k])) throw Error(ERR_NON_FINITE, "non-finite T2");
-  upload_amplitudes(Tcur, T1, T2, Rbuf);
+  upload_amplitudes(Tcur, T1, T2, Rbuf, large);
   ops::sync(stream);
   have_T = true;
 }
@@ -319,28 +305,28 @@ Schedule* Handle::adjoint_schedule() {
 // interleaved complex when the input was complex; stacked Re/Im auxiliary rows
 // go to the two parts).  out is overwritten.
 void Handle::scatter_vertex_bar(const Schedule::VertexBar& vb, double* out) {
-  const int64_t o = shape.o, v = shape.v, G = sys.G, NG = in_NG, Np = in_Np;
+  const int64_t o = shape.o, v = shape.v, NG = in_NG, Np = in_Np;
   // planes of the device blocks: stacked Re/Im rows (real path) or the planar
   // real and imaginary parts (complex path) go to the two parts of the output
-  const int64_t es = in_complex ? 2 : 1, parts = (in_stacked || complex_path) ? 2 : 1;
-  const int64_t planes = complex_path ? 2 : 1;
-  std::memset(out, 0, sizeof(double) * NG * Np * Np * es);
+  // (a real input has no imaginary part to receive one)
+  const int64_t es = in_complex ? 2 : 1, parts = in_complex && (in_stacked || complex_path) ? 2 : 1;
+  const int64_t total = NG * Np * Np * es;
   struct Block { const double* d; int64_t row0, nx, col0, ny; };
   const Block blocks[4] = {{vb.Gpp, o, v, o, v}, {vb.Gph, o, v, 0, o}, {vb.Ghh, 0, o, 0, o},
                            {vb.Ghp, 0, o, o, v}};
-  std::vector<double> h;
-  for (const Block& b : blocks) {
-    if (!b.d) continue;
-    h.resize(planes * G * b.nx * b.ny);
-    ops::d2h(h.data(), b.d, h.size(), stream);
-    ops::sync(stream);
-    for (int64_t part = 0; part < parts; ++part)
-      for (int64_t k = 0; k < NG; ++k)
-        for (int64_t x = 0; x < b.nx; ++x)
-          for (int64_t y = 0; y < b.ny; ++y)
-            out[(k + NG * ((b.row0 + x) + Np * (b.col0 + y))) * es + part] +=
-                h[((part * NG + k) * b.nx + x) * b.ny + y];
+  double* dev = ops::alloc(total);
+  try {
+    ops::zero(dev, total, stream);
+    for (const Block& b : blocks)
+      for (int64_t part = 0; b.d && part < parts; ++part)
+        ops::scatter_vertex(dev, b.d + part * NG * b.nx * b.ny, es == 2, static_cast<int>(part), NG,
+                            Np, b.row0, b.nx, b.col0, b.ny, stream);
+    ops::d2h_staged(out, 1, dev, total, stage, stream);
+  } catch (...) {
+    ops::release(dev);
+    throw;
   }
+  ops::release(dev);
 }
 
 void Handle::residual_vjp(const double* T1, const double* T2, const double* R1b,

@@ -34,7 +34,9 @@ struct Handle {
   void require_inputs() const;
   // Layout change between the caller's column-major T1/T2 and the device
   // amplitude vector, through a full-size device staging vector st (not dst/src).
-  void upload_amplitudes(double* dst, const double* T1, const double* T2, double* st);
+  // check: a non-finite value throws before dst is written.
+  void upload_amplitudes(double* dst, const double* T1, const double* T2, double* st,
+                         bool check = false);
   void download_amplitudes(const double* src, double* T1, double* T2, double* st);
   void mix(double* A_new, double* dT_new, double* norm2_dev, double* out);
   std::string diis_failure(int status, int iteration, double energy, double norm);
@@ -57,6 +59,7 @@ struct Handle {
   void* ev0 = nullptr;
   void* ev1 = nullptr;
   std::string error;
+  ops::HostStage stage;  // pinned buffers of the large host transfers
 
   RealSystem sys;
   ComplexSystem csys;

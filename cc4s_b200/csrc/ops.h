@@ -20,6 +20,22 @@ void zero(double* p, size_t elems, Stream s);
 void h2d(double* dst, const double* src, size_t elems, Stream s);
 void d2h(double* dst, const double* src, size_t elems, Stream s);
 void d2d(double* dst, const double* src, size_t elems, Stream s);
+// Large transfers of pageable host memory: worker threads move the host side through
+// pinned buffers of their own while the copy engine moves the last pieces.  Element k of
+// the device vector is element k * stride of the host one (2: one plane of interleaved
+// complex values).  Both return when the host memory is done with.  The buffers (32 MiB)
+// belong to the HostStage, made by its first transfer of STAGED_MIN elements or more;
+// smaller ones go straight.
+struct HostStage {
+  HostStage() = default;
+  HostStage(const HostStage&) = delete;
+  HostStage& operator=(const HostStage&) = delete;
+  ~HostStage();
+  void* pinned = nullptr;
+};
+constexpr int64_t STAGED_MIN = int64_t(1) << 21;
+void h2d_staged(double* dst, const double* src, int64_t elems, int stride, HostStage& st, Stream s);
+void d2h_staged(double* dst, int stride, const double* src, int64_t elems, HostStage& st, Stream s);
 void sync(Stream s);
 Stream stream_create(int device);
 void stream_destroy(Stream s);
@@ -55,6 +71,11 @@ void symmetrize(double* R, int64_t n, Stream s);
 // or complex interleaved (part 0 = real, 1 = imaginary).
 void gather_vertex(double* out, const double* in, bool in_complex, int part, int64_t NG,
                    int64_t Np, int64_t row0, int64_t nx, int64_t col0, int64_t ny, Stream s);
+
+// The inverse: writes one row-major block in[G][nx][ny] into a column-major vertex
+// out[NG][Np][Np] (complex interleaved when out_complex, into part 0 or 1).
+void scatter_vertex(double* out, const double* in, bool out_complex, int part, int64_t NG,
+                    int64_t Np, int64_t row0, int64_t nx, int64_t col0, int64_t ny, Stream s);
 
 // Scans n doubles of a device vector (complex interleaved when complex_values):
 // returns bit 0 if any is not finite, bit 1 if any imaginary part is non-zero.

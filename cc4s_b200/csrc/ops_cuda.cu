@@ -7,8 +7,13 @@
 // partials in a fixed order.
 #include "ops.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
+#include <system_error>
+#include <thread>
+#include <vector>
 
 namespace cc4s_b200 {
 namespace ops {
@@ -196,6 +201,33 @@ __global__ void gather_vertex_kernel(double* out, const double* in, int cplx, in
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
       const int64_t g = bg * 32 + r, y = by * 32 + threadIdx.x;
       if (y < ny && g < NG) out[(g * nx + x) * ny + y] = tile[threadIdx.x][r];
+    }
+    __syncthreads();
+  }
+}
+
+// The inverse of gather_vertex_kernel, with its tiles (bound by memory: 16 B per element;
+// the strided host loop it takes the place of wrote one cache line per element).
+__global__ void scatter_vertex_kernel(double* out, const double* in, int cplx, int part,
+                                      int64_t NG, int64_t Np, int64_t row0, int64_t nx,
+                                      int64_t col0, int64_t ny) {
+  __shared__ double tile[32][33];
+  const int64_t tg = (NG + 31) / 32, tyn = (ny + 31) / 32;
+  const int64_t total = tg * tyn * nx;
+  const int64_t es = cplx ? 2 : 1;
+  for (int64_t blk = blockIdx.x; blk < total; blk += gridDim.x) {
+    const int64_t bg = blk % tg;
+    const int64_t by = (blk / tg) % tyn;
+    const int64_t x = blk / (tg * tyn);
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+      const int64_t g = bg * 32 + r, y = by * 32 + threadIdx.x;
+      if (y < ny && g < NG) tile[threadIdx.x][r] = in[(g * nx + x) * ny + y];
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+      const int64_t y = by * 32 + r, g = bg * 32 + threadIdx.x;
+      if (y < ny && g < NG)
+        out[(g + NG * (row0 + x + Np * (col0 + y))) * es + part] = tile[r][threadIdx.x];
     }
     __syncthreads();
   }
@@ -630,6 +662,128 @@ void d2d(double* d, const double* src, size_t elems, Stream s) {
   CC_CHECK(cudaMemcpyAsync(d, src, elems * sizeof(double), cudaMemcpyDeviceToDevice, s));
 }
 void sync(Stream s) { CC_CHECK(cudaStreamSynchronize(s)); }
+
+namespace {
+constexpr int STAGE_THREADS = 8;
+constexpr int64_t STAGE_PIECE = int64_t(1) << 18;  // doubles: 2 MiB, two per thread
+
+// Runs body(t) for t < STAGE_THREADS on threads of this device; the caller takes the ones
+// the system would not start.  The first CUDA error wins.
+template <class F>
+void stage_run(F&& body) {
+  int dev = 0;
+  CC_CHECK(cudaGetDevice(&dev));
+  std::atomic<int> status{cudaSuccess};
+  auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(dev);
+    if (e == cudaSuccess) e = body(t);
+    int none = cudaSuccess;
+    if (e != cudaSuccess) status.compare_exchange_strong(none, e);
+  };
+  std::thread th[STAGE_THREADS];
+  int started = 0;
+  try {
+    for (; started < STAGE_THREADS - 1; ++started) th[started] = std::thread(work, started);
+  } catch (const std::system_error&) {
+  }
+  for (int t = started; t < STAGE_THREADS; ++t) work(t);
+  for (int t = 0; t < started; ++t) th[t].join();
+  CC_CHECK(static_cast<cudaError_t>(status.load()));
+}
+
+double* stage_buffers(HostStage& st) {
+  if (!st.pinned && cudaHostAlloc(&st.pinned, 2 * STAGE_THREADS * STAGE_PIECE * sizeof(double),
+                                  cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    st.pinned = nullptr;
+  }
+  return static_cast<double*>(st.pinned);
+}
+
+// One thread's pieces t, t + STAGE_THREADS, ... through its two buffers; `begin` and `end`
+// are called for piece i (at element lo, n of them) with its buffer and event, `end`
+// once per piece in order, at the latest before the buffer is taken again.
+template <class Begin, class End>
+cudaError_t stage_pieces(int t, double* pinned, int64_t elems, Begin&& begin, End&& end) {
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+    e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+  const int64_t step = STAGE_THREADS * STAGE_PIECE;
+  auto at = [&](int64_t i) { return t * STAGE_PIECE + i * step; };
+  auto len = [&](int64_t i) { return std::min(STAGE_PIECE, elems - at(i)); };
+  auto buf = [&](int64_t i) { return pinned + (2 * t + (i & 1)) * STAGE_PIECE; };
+  int64_t i = 0, done = 0;
+  for (; e == cudaSuccess && at(i) < elems; ++i) {
+    if (i - done == 2) { e = end(buf(done), ev[done & 1], at(done), len(done)); ++done; }
+    if (e == cudaSuccess) e = begin(buf(i), ev[i & 1], at(i), len(i));
+  }
+  for (; e == cudaSuccess && done < i; ++done) e = end(buf(done), ev[done & 1], at(done), len(done));
+  for (int k = 0; k < 2; ++k) {
+    if (ev[k]) {
+      cudaEventSynchronize(ev[k]);  // no copy of this thread's buffers outlives the call
+      cudaEventDestroy(ev[k]);
+    }
+  }
+  return e;
+}
+}  // namespace
+
+HostStage::~HostStage() {
+  if (pinned) cudaFreeHost(pinned);
+}
+
+void h2d_staged(double* dst, const double* src, int64_t elems, int stride, HostStage& st, Stream s) {
+  double* pinned = elems >= STAGED_MIN ? stage_buffers(st) : nullptr;
+  if (!pinned) {
+    std::vector<double> h;
+    if (stride != 1) {
+      h.resize(elems);
+      for (int64_t k = 0; k < elems; ++k) h[k] = src[k * stride];
+      src = h.data();
+    }
+    h2d(dst, src, elems, s);
+    sync(s);
+    return;
+  }
+  stage_run([&](int t) {
+    return stage_pieces(
+        t, pinned, elems,
+        [&](double* b, cudaEvent_t ev, int64_t lo, int64_t n) {
+          if (stride == 1) std::memcpy(b, src + lo, n * sizeof(double));
+          else for (int64_t k = 0; k < n; ++k) b[k] = src[(lo + k) * stride];
+          const cudaError_t e = cudaMemcpyAsync(dst + lo, b, n * sizeof(double), cudaMemcpyHostToDevice, s);
+          return e != cudaSuccess ? e : cudaEventRecord(ev, s);
+        },
+        [&](double*, cudaEvent_t ev, int64_t, int64_t) { return cudaEventSynchronize(ev); });
+  });
+}
+
+void d2h_staged(double* dst, int stride, const double* src, int64_t elems, HostStage& st, Stream s) {
+  double* pinned = elems >= STAGED_MIN ? stage_buffers(st) : nullptr;
+  if (!pinned) {
+    std::vector<double> h(stride != 1 ? elems : 0);
+    d2h(stride != 1 ? h.data() : dst, src, elems, s);
+    sync(s);
+    for (int64_t k = 0; k < static_cast<int64_t>(h.size()); ++k) dst[k * stride] = h[k];
+    return;
+  }
+  stage_run([&](int t) {
+    return stage_pieces(
+        t, pinned, elems,
+        [&](double* b, cudaEvent_t ev, int64_t lo, int64_t n) {
+          const cudaError_t e = cudaMemcpyAsync(b, src + lo, n * sizeof(double), cudaMemcpyDeviceToHost, s);
+          return e != cudaSuccess ? e : cudaEventRecord(ev, s);
+        },
+        [&](double* b, cudaEvent_t ev, int64_t lo, int64_t n) {
+          const cudaError_t e = cudaEventSynchronize(ev);
+          if (e != cudaSuccess) return e;
+          if (stride == 1) std::memcpy(dst + lo, b, n * sizeof(double));
+          else for (int64_t k = 0; k < n; ++k) dst[(lo + k) * stride] = b[k];
+          return cudaSuccess;
+        });
+  });
+}
 Stream stream_create(int device) {
   CC_CHECK(cudaSetDevice(device));
   cudaStream_t s;
@@ -762,6 +916,15 @@ void jacobi(double* Tnew, double* dT, const double* R, const double* Told, const
             const double* ep, const AmpShape& sh, double shift, Stream s) {
   JacobiArgs a{Tnew, dT, R, Told, eh, ep, sh.o, sh.v, sh.plane(), sh.total(), shift};
   jacobi_kernel<<<grid_for(sh.total(), 256), 256, 0, s>>>(a);
+  CC_LAUNCH_CHECK();
+  count();
+}
+
+void scatter_vertex(double* out, const double* in, bool out_complex, int part, int64_t NG,
+                    int64_t Np, int64_t row0, int64_t nx, int64_t col0, int64_t ny, Stream s) {
+  const int64_t work = ((NG + 31) / 32) * ((ny + 31) / 32) * nx;
+  scatter_vertex_kernel<<<grid_for(work, 1), dim3(32, 8), 0, s>>>(out, in, out_complex ? 1 : 0, part,
+                                                                NG, Np, row0, nx, col0, ny);
   CC_LAUNCH_CHECK();
   count();
 }

@@ -512,6 +512,22 @@ void sum_partials_to(double* dst, const double* ws, int nparts, int nvals, Strea
   }
 }
 
+HostStage::~HostStage() {}
+void h2d_staged(double* dst, const double* src, int64_t n, int stride, HostStage&, Stream) {
+  for (int64_t k = 0; k < n; ++k) dst[k] = src[k * stride];
+}
+void d2h_staged(double* dst, int stride, const double* src, int64_t n, HostStage&, Stream) {
+  for (int64_t k = 0; k < n; ++k) dst[k * stride] = src[k];
+}
+void scatter_vertex(double* out, const double* in, bool cplx, int part, int64_t NG, int64_t Np,
+                    int64_t row0, int64_t nx, int64_t col0, int64_t ny, Stream) {
+  ++g_ops;
+  for (int64_t g = 0; g < NG; ++g)
+    for (int64_t x = 0; x < nx; ++x)
+      for (int64_t y = 0; y < ny; ++y)
+        out[(g + NG * (row0 + x + Np * (col0 + y))) * (cplx ? 2 : 1) + part] =
+            in[(g * nx + x) * ny + y];
+}
 int scan_vertex(const double* p, int64_t n, bool complex_values, Stream) {
   ++g_ops;
   int f = 0;
