@@ -95,7 +95,7 @@ class Schedule {
     double gemm_seconds = 0, gemm_flops = 0;  // all contractions of the last residual
     double top_seconds = 0, top_flops = 0;    // the most expensive single launch
     int launches = 0;
-    // split-precision launches only (FP64-equivalent flops; 6 FP16 products each)
+    // split-precision launches only (FP64-equivalent flops; ten digit products each)
     double split_seconds = 0, split_flops = 0;
     int split_launches = 0;
   };
