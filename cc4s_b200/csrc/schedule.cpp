@@ -65,7 +65,10 @@ constexpr size_t kSplitDataOffset = 128;  // doubles: 1 KiB
 }  // namespace
 
 // FP64 contractions: the seven-digit form where its time (slicing, then the integer
-// tensor cores) is below the FP64 tensor pipe's.
+// tensor cores) is below the FP64 tensor pipe's.  The constants follow measured shapes
+// (FP64 pipe, seven digits): 512^3 37 and 41 us, 1024 x 1024 x 256 46 and 35 us,
+// 128 x 32768 x 128 61 and 83 us (slicing of an operand used 128 times),
+// 2048 x 2048 x 512 251 and 93 us, 8192^3 37.4 and 13.0 ms.
 static bool digits7_pays(const Contraction& c) {
   if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K < 64) return false;
   const double M = double(c.M), N = double(c.N), K = double(c.K);
