@@ -100,48 +100,7 @@ struct PackSet {
   uint32_t end[3];        // work items of the operands, cumulative; the last is the total
 };
 
-// Packing works on tiles of 64 rows x 64 k staged in shared memory.  The row and
-// k offsets of a tile are computed once per tile (two-level index maps need an
-// integer division each), every thread keeps 16 loads in flight, and the digits
-// leave as 16-byte vector stores along k.
-constexpr int PR = 64, PKT = 64, PTHREADS = 256;
-
-struct PackTile {
-  double v[PR][PKT + 1];
-  int64_t roff[PR];
-  int64_t koff[PKT];
-};
-
-// Loads the tile (r0, k0) of the operand into t.v (zero outside R x K).
-__device__ __forceinline__ void pack_load_tile(const PackArgs& a, int64_t r0, int64_t k0,
-                                               PackTile& t) {
-  for (int q = threadIdx.x; q < PR + PKT; q += PTHREADS) {
-    if (q < PR) {
-      const int64_t r = r0 + q;
-      t.roff[q] = r < a.R ? a.ar.off(static_cast<uint32_t>(r)) : -1;
-    } else {
-      const int64_t k = k0 + (q - PR);
-      t.koff[q - PR] = k < a.K ? a.koff(k) : -1;
-    }
-  }
-  __syncthreads();
-  const int lo = threadIdx.x & 63, hi = threadIdx.x >> 6;  // lanes along the contiguous index
-  double x[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int rr = a.r_contig ? lo : hi + 4 * j;
-    const int kk = a.r_contig ? hi + 4 * j : lo;
-    const int64_t ro = t.roff[rr], ko = t.koff[kk];
-    x[j] = (ro >= 0 && ko >= 0) ? a.src[ro + ko] : 0.0;
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int rr = a.r_contig ? lo : hi + 4 * j;
-    const int kk = a.r_contig ? hi + 4 * j : lo;
-    t.v[rr][kk] = x[j];
-  }
-  __syncthreads();
-}
+constexpr int PR = 64, PTHREADS = 256;  // rows of a work item
 
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
   return static_cast<unsigned long long>(__double_as_longlong(fabs(x)));
@@ -231,63 +190,163 @@ __device__ __forceinline__ double pow2i(int e) {
   return ldexp(1.0, e);
 }
 
+// Digits of four elements: word q holds digit q of each, element 0 in the lowest byte.
+// With 128 added to every digit but the top one, the bytes of the integer are the digits
+// plus 128 (the carries of a balanced representation happen in the one addition).
+template <int NS>
+__device__ __forceinline__ void digits4(const double (&x)[4], double s1, double s2,
+                                        uint32_t (&w)[NS]) {
+  uint32_t lo[4], hi[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if constexpr (NS == 4) {
+      lo[j] = (static_cast<uint32_t>(__double2int_rn(x[j] * s1 * s2)) + 0x00808080u) ^ 0x00808080u;
+      hi[j] = 0;
+    } else {
+      const unsigned long long X =
+          (static_cast<unsigned long long>(__double2ll_rn(x[j] * s1 * s2)) + 0x0000808080808080ull) ^
+          0x0000808080808080ull;
+      lo[j] = static_cast<uint32_t>(X);
+      hi[j] = static_cast<uint32_t>(X >> 32);
+    }
+  }
+  auto planes = [&](const uint32_t (&v)[4], int byte) {  // byte pair (byte, byte + 1) of each
+    const uint32_t a = __byte_perm(v[0], v[1], byte ? 0x7362 : 0x5140);
+    const uint32_t b = __byte_perm(v[2], v[3], byte ? 0x7362 : 0x5140);
+    return make_uint2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
+  };
+  const uint2 l0 = planes(lo, 0), l2 = planes(lo, 2);
+  w[NS - 1] = l0.x;
+  w[NS - 2] = l0.y;
+  w[NS - 3] = l2.x;
+  w[NS - 4] = l2.y;
+  if constexpr (NS == 7) {
+    const uint2 h0 = planes(hi, 0), h2 = planes(hi, 2);
+    w[2] = h0.x;
+    w[1] = h0.y;
+    w[0] = h2.x;
+  }
+}
+
 // The digits of every element (row-padded to Rp, k-padded to Kp) and the per-row
 // exponent: x = 2^e X 2^-(8 NS - 2) with |X| <= 2^(8 NS - 2) rounded to an integer and
-// written in balanced base 256, lowest digit first (each in [-128, 127], the top one in
-// [-64, 65]).  Memory bound: 8 B read and NS B written per element.
+// written in balanced base 256 (each digit in [-128, 127], the top one in [-64, 65]).
+// A work item is 64 rows x 128 k (lanes on four k each, a warp per row, nothing staged, so
+// 16 loads per thread stay in flight without a barrier) or, where the rows are contiguous
+// in memory, 64 rows x 64 k through a shared-memory tile (stores of 16 bytes per row and
+// lane straight from such loads were slower: 1.14 against 0.99 ms for 256 x 262144 x 256).
+// Memory bound: 8 B read, NS B written per element.  Against tiles for both and digits
+// extracted one by one, whole contractions of 2048^3 0.291 -> 0.275 ms in seven digits,
+// 4096 x 256 x 16384 0.92 -> 0.87 ms, 4096 x 1024 x 65536 8.06 -> 7.83 ms.
+constexpr int PK_K = 128, PK_R = 64;  // k per item, by the contiguous index
 template <int NS>
 __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
-  __shared__ PackTile t;
-  __shared__ double scale_s[2][PR];
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
+  __shared__ double tile[PR][81];  // k at k + k / 4: both directions free of bank conflicts
+  __shared__ int64_t rows_off[PR], ks_off[PK_R];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (uint32_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
     const int which = it < pp.end[0] ? 0 : it < pp.end[1] ? 1 : 2;
     const PackArgs& a = pp.op[which];
     const uint32_t w = which ? it - pp.end[which - 1] : it;
-    const uint32_t nk = static_cast<uint32_t>(a.Kp + PKT - 1) / PKT, wr = w / nk;
-    const int64_t pl = a.Rp * a.Kp, r0 = int64_t(wr) * PR, k0 = int64_t(w - wr * nk) * PKT;
-    if (threadIdx.x < PR) {
-      const int64_t r = r0 + threadIdx.x;
-      double s1 = 0.0, s2 = 0.0;  // their product 2^(8 NS - 2 - e), each in the normal range
-      if (r < a.R) {
-        const unsigned long long mb = a.rmax[r];
-        int e = 0;
-        if (mb >= 0x7ff0000000000000ull) {
-          e = EXP_NONFINITE;
-        } else if (mb != 0) {
-          frexp(__longlong_as_double(static_cast<long long>(mb)), &e);
-          const int sh = 8 * NS - 2 - e;
-          s1 = pow2i(sh / 2);
-          s2 = pow2i(sh - sh / 2);
-        }
-        if (k0 == 0) a.rexp[r] = e;
+    const int kw = a.r_contig ? PK_R : PK_K;
+    const uint32_t nk = static_cast<uint32_t>(a.Kp + kw - 1) / kw, wr = w / nk;
+    const int64_t pl = a.Rp * a.Kp, r0 = int64_t(wr) * PR, k0 = int64_t(w - wr * nk) * kw;
+    // the row this lane answers for: its exponent, scale and offset
+    const int64_t lr = r0 + 8 * warp + (lane & 7);
+    double s1 = 0.0, s2 = 0.0;  // their product 2^(8 NS - 2 - e), each in the normal range
+    int64_t roff = -1;
+    if (lr < a.R) {
+      const unsigned long long mb = a.rmax[lr];
+      int e = 0;
+      if (mb >= 0x7ff0000000000000ull) {
+        e = EXP_NONFINITE;
+      } else if (mb != 0) {
+        frexp(__longlong_as_double(static_cast<long long>(mb)), &e);
+        const int sh = 8 * NS - 2 - e;
+        s1 = pow2i(sh / 2);
+        s2 = pow2i(sh - sh / 2);
       }
-      scale_s[0][threadIdx.x] = s1;
-      scale_s[1][threadIdx.x] = s2;
+      if (k0 == 0) a.rexp[lr] = e;
+      roff = a.ar.off(static_cast<uint32_t>(lr));
     }
-    pack_load_tile(a, r0, k0, t);   // its first barrier also publishes scale_s
-    const int64_t r = r0 + row, kb = k0 + 16 * part;
-    if (kb < a.Kp) {
-      const double s1 = scale_s[0][row], s2 = scale_s[1][row];
-      __align__(16) int8_t h[NS][16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const double v = t.v[row][16 * part + j] * a.sign[kb + j < a.K1 ? 0 : 1];
-        long long X = s1 != 0.0 ? __double2ll_rn(v * s1 * s2) : 0;
-#pragma unroll
-        for (int q = NS - 1; q > 0; --q) {
-          const int8_t d = static_cast<int8_t>(X & 255);
-          h[q][j] = d;
-          X = (X - d) >> 8;
-        }
-        h[0][j] = static_cast<int8_t>(X);
+    if (a.r_contig) {
+      if (lane < 8) rows_off[8 * warp + lane] = roff;
+      else if (lane < 16) {
+        const int64_t k = k0 + 8 * warp + (lane - 8);
+        ks_off[8 * warp + lane - 8] = k < a.K ? a.koff(k) : -1;
       }
-      const int64_t o = r * a.Kp + kb;
-#pragma unroll
-      for (int q = 0; q < NS; ++q)
-        *reinterpret_cast<uint4*>(a.dst + q * pl + o) = *reinterpret_cast<const uint4*>(h[q]);
+      __syncthreads();
     }
-    __syncthreads();
+    if (a.r_contig) {  // lanes on rows for the loads, on k for the stores
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int64_t ro = rows_off[32 * h + lane];
+        double x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int64_t ko = ks_off[8 * warp + j];
+          x[j] = (ro >= 0 && ko >= 0) ? a.src[ro + ko] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int k = 8 * warp + j;
+          tile[32 * h + lane][k + (k >> 2)] = x[j];
+        }
+      }
+      __syncthreads();
+      const int64_t kb = k0 + 4 * (lane & 15);
+      double sg[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sg[j] = a.sign[kb + j < a.K1 ? 0 : 1];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {  // two rows at a time, half a warp each
+        const int r = 2 * h + (lane >> 4);
+        const double t1 = __shfl_sync(0xffffffffu, s1, r), t2 = __shfl_sync(0xffffffffu, s2, r);
+        double y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = tile[8 * warp + r][5 * (lane & 15) + j] * sg[j];
+        uint32_t q[NS];
+        digits4<NS>(y, t1, t2, q);
+        if (kb < a.Kp) {
+          int8_t* d = a.dst + (r0 + 8 * warp + r) * a.Kp + kb;
+#pragma unroll
+          for (int n = 0; n < NS; ++n) *reinterpret_cast<uint32_t*>(d + n * pl) = q[n];
+        }
+      }
+      __syncthreads();
+    } else {
+      const int64_t kb = k0 + 4 * lane;
+      int64_t ko[4];
+      double sg[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        ko[j] = kb + j < a.K ? a.koff(kb + j) : -1;
+        sg[j] = a.sign[kb + j < a.K1 ? 0 : 1];
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {  // four rows at a time
+        double x[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int64_t ro = __shfl_sync(0xffffffffu, roff, 4 * h + r);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            x[r][j] = (ro >= 0 && ko[j] >= 0) ? a.src[ro + ko[j]] * sg[j] : 0.0;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const double t1 = __shfl_sync(0xffffffffu, s1, 4 * h + r);
+          const double t2 = __shfl_sync(0xffffffffu, s2, 4 * h + r);
+          uint32_t q[NS];
+          digits4<NS>(x[r], t1, t2, q);
+          if (kb < a.Kp) {
+            int8_t* d = a.dst + (r0 + 8 * warp + 4 * h + r) * a.Kp + kb;
+#pragma unroll
+            for (int n = 0; n < NS; ++n) *reinterpret_cast<uint32_t*>(d + n * pl) = q[n];
+          }
+        }
+      }
+    }
   }
 }
 
@@ -850,7 +909,10 @@ void pack(const PackArgs* const* ops, int n, int64_t rows, int digits, cudaStrea
   // strips of k for the maxima: the longest of 128 .. 1024 that gives 148 x 6 work items
   int64_t kstrip = 1024;
   auto strips = [&](const PackArgs& x) { return (x.Rp / PR) * ((x.K + kstrip - 1) / kstrip); };
-  auto tiles = [](const PackArgs& x) { return (x.Rp / PR) * ((x.Kp + PKT - 1) / PKT); };
+  auto tiles = [](const PackArgs& x) {
+    const int kw = x.r_contig ? PK_R : PK_K;
+    return (x.Rp / PR) * ((x.Kp + kw - 1) / kw);
+  };
   auto items = [&](auto&& count) {
     int64_t t = 0;
     for (int k = 0; k < 3; ++k) pp.end[k] = static_cast<uint32_t>(t += k < n ? count(pp.op[k]) : 0);
