@@ -161,13 +161,12 @@ int Handle::run(cc4s_cc_result* out) {
     double st = 0.0;
     if (opt.mixer == CC4S_MIXER_DIIS) ops::d2h(&st, reinterpret_cast<double*>(status_dev), 1, stream);
     ops::sync(stream);
+    solver->check_device();
     const float ms = ops::event_ms(ev0, ev1);
     int status_int;
     std::memcpy(&status_int, &st, sizeof(int));
     if (opt.mixer == CC4S_MIXER_DIIS && status_int != 0)
       throw Error(ERR_DIIS_SINGULAR, diis_failure(status_int, i, prev.real(), i > 0 && i <= CC4S_MAX_HISTORY ? out->residuum_norm[i - 1] : 0.0));
-    if (opt.precision != CC4S_PRECISION_FP64 && solver->device_error())
-      throw Error(ERR_TIMEOUT, "a tensor-core kernel gave up a bounded wait");
     Dr = host[0]; Xr = host[1];
     e = std::complex<double>(host[0] + host[1], host[2] + host[3]);
     const double norm = std::sqrt(host[4]);
@@ -228,6 +227,7 @@ void Handle::residual(const double* T1, const double* T2, double* R1, double* R2
   try {
     if (!first) upload_amplitudes(Tin, T1, T2, Rbuf);
     solver->residual(first ? nullptr : Tin, Rbuf);
+    solver->check_device();
     download_amplitudes(Rbuf, R1, R2, Tin);
   } catch (...) {
     ops::release(Tin);
@@ -250,6 +250,7 @@ void Handle::backward(double* S_of_G, double* dE_dGamma) {
   try {
     if (dE_dGamma) dG = ops::alloc(G * n1);
     solver->structure_factor(Tcur, Sd, dG);
+    solver->check_device();
     std::vector<double> S(G), g;
     ops::d2h(S.data(), Sd, G, stream);
     if (dG) {
@@ -353,6 +354,7 @@ void Handle::residual_vjp(const double* T1, const double* T2, const double* R1b,
       ops::zero(vb.Ghh, pl * G * o * o, stream); ops::zero(vb.Ghp, pl * G * o * v, stream);
     }
     adjs->vjp(Rb, Tb, dGamma ? &vb : nullptr, nullptr);
+    adjs->check_device();
     download_amplitudes(Tb, T1b, T2b, Rbuf);
     if (dGamma) scatter_vertex_bar(vb, dGamma);
   } catch (...) {
@@ -411,6 +413,7 @@ void Handle::relaxed_gradient(int max_iterations, double convergence, double* dE
       double st = 0.0;
       if (diis) ops::d2h(&st, reinterpret_cast<double*>(status_dev), 1, stream);
       ops::sync(stream);
+      adjs->check_device();
       int status_int;
       std::memcpy(&status_int, &st, sizeof(int));
       if (diis && status_int != 0)
@@ -431,6 +434,7 @@ void Handle::relaxed_gradient(int max_iterations, double convergence, double* dE
     ops::event_record(ev0, stream);
     adjs->vjp(lam, Jt, &vb, VdB);
     ops::event_record(ev1, stream);
+    adjs->check_device();
     out->gradient_seconds = 1e-3 * ops::event_ms(ev0, ev1);
     if (dE_dGamma) scatter_vertex_bar(vb, dE_dGamma);
   } catch (...) {
@@ -563,7 +567,7 @@ void Handle::finite_size_correction(const double* U, int64_t NGG, const double* 
     ops::event_record(ev1, stream);
     out->seconds = ops::event_ms(ev0, ev1) * 1e-3;
     ops::sync(stream);
-    if (solver->device_error()) throw Error(ERR_TIMEOUT, "tensor-core kernel wait expired");
+    solver->check_device();
     const double N3 = double(g.N) * g.N * g.N;
     out->uncorrected = h[0];
     out->corrected = h[1] / N3 / 8.0;

@@ -183,6 +183,12 @@ void Handle::allocate_state() {
   status_dev = reinterpret_cast<int*>(take(4));
   reset_mixer();
   ops::sync(stream);
+  try {
+    solver->check_device();  // the integrals were built above
+  } catch (...) {
+    free_state();
+    throw;
+  }
 }
 
 void Handle::reset_mixer() {

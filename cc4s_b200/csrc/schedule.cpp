@@ -2,7 +2,6 @@
 
 #include <algorithm>
 #include <array>
-#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -18,7 +17,8 @@ void Schedule::release_all() {
   for (void* e : ev_) ops::event_destroy(e);
   ev_.clear();
   if (split_mem_) ops::release(split_mem_);
-  split_mem_ = nullptr;
+  if (split_error_) ops::release(split_error_);
+  split_mem_ = split_error_ = nullptr;
   split_ = SplitScratch();
   split_extra_ = nullptr;
   split_extra_bytes_ = 0;
@@ -60,28 +60,6 @@ void Schedule::gemm_(const Contraction& c) {
   fp64_exec(c);
 }
 
-namespace {
-constexpr size_t kSplitDataOffset = 128;  // doubles: 1 KiB
-}  // namespace
-
-// FP64 contractions: the seven-digit form where its time (slicing, then the integer
-// tensor cores) is below the FP64 tensor pipe's.  The constants follow measured shapes
-// (FP64 pipe, seven digits): 512^3 37 and 41 us, 1024 x 1024 x 256 46 and 35 us,
-// 128 x 32768 x 128 61 and 83 us (slicing of an operand used 128 times),
-// 2048 x 2048 x 512 251 and 93 us, 8192^3 37.4 and 13.0 ms.
-static bool digits7_pays(const Contraction& c) {
-  if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K < 64) return false;
-  const double M = double(c.M), N = double(c.N), K = double(c.K);
-  auto up = [](double x, double t) { return std::ceil(x / t) * t; };
-  // microseconds: launches, slicing, waves of one tile per SM
-  const double tiles7 = up(M, 128) * up(N, 64) / (128 * 64);
-  const int parts = split_k_parts(static_cast<int64_t>(tiles7), c.M, c.N, c.K, 7);
-  const double d7 = 20.0 + 24.0 * (M + N) * K / 3.5e6 + (parts > 1 ? 6.0 : 0.0) +
-                    std::ceil(tiles7 * parts / 148.0) * (3.3 + 0.021 * up(K, 32) / parts);
-  const double dmma = 12.0 + 2.0 * up(M, 128) * up(N, 128) * K / 22e6;
-  return d7 < dmma;
-}
-
 int Schedule::digits_for(const Contraction& c, bool big) const {
   if (big && precision_ != 0 && c.batch == 1 && c.K >= 64 && c.M >= 64 && c.N >= 64) return 4;
   return digits7_pays(c) ? 7 : 0;
@@ -96,22 +74,30 @@ void Schedule::split_reserve(size_t regular, size_t extra) {
   ops::sync(s_);
   if (split_mem_) ops::release(split_mem_);
   split_mem_ = nullptr;
-  split_ = SplitScratch();  // nothing is left if the allocation fails
+  split_.p = nullptr;  // nothing is left if the allocation fails
+  split_.bytes = 0;
   split_extra_ = nullptr;
   split_extra_bytes_ = 0;
-  // The error word sits in the first double; the packed slices start 1 KiB in,
-  // so every TMA row request of the contraction kernel begins on a sector and
-  // line boundary (a 16-byte offset made each 64-byte row touch three sectors).
-  const size_t doubles = (regular + extra) / 8 + kSplitDataOffset;
-  split_mem_ = ops::alloc(doubles);
-  split_.p = split_mem_ + kSplitDataOffset;
+  error_word();
+  // Allocations start on a 256-byte boundary, so every TMA row request of the contraction
+  // kernel begins on a sector and line boundary (a 16-byte offset made each 64-byte row
+  // touch three sectors).
+  split_mem_ = ops::alloc((regular + extra) / 8);
+  split_.p = split_mem_;
   split_.bytes = regular;
-  split_.error = reinterpret_cast<int*>(split_mem_);
   if (extra) {
     split_extra_ = static_cast<unsigned char*>(split_.p) + regular;
     split_extra_bytes_ = extra;
   }
-  ops::zero(split_mem_, 2, s_);
+}
+
+// The word in which a kernel records an expired wait: in memory of its own, so that it
+// outlives the growing of the scratch, and never cleared.
+void Schedule::error_word() {
+  if (split_error_) return;
+  split_error_ = ops::alloc(2);
+  ops::zero(split_error_, 2, s_);
+  split_.error = reinterpret_cast<int*>(split_error_);
 }
 
 void Schedule::split_exec(const Contraction& c) {
@@ -163,7 +149,7 @@ void Schedule::tc_packed_b_(const Contraction& c, const SplitPackedB& b) {
 void Schedule::tc_prepacked_(const Contraction& c, const SplitOperand& A, const SplitRuns& ar,
                              const SplitOperand& B, const SplitRuns& br) {
   if (taping_) throw Error(ERR_STATE, "pre-packed split operands are not recorded");
-  if (!split_.error) split_reserve(size_t(1) << 16, split_extra_bytes_);  // the error word
+  error_word();
   const double f = 2.0 * double(c.M) * double(c.N) * double(c.K);
   if (count_flops_) flops_ += f;
   if (profile_ && count_flops_) {
@@ -540,11 +526,15 @@ void Schedule::structure_factor_pw(const double* T, const double* Uw, int64_t NG
 int Schedule::device_error() {
   if (!split_.error) return 0;
   double v = 0.0;
-  ops::d2h(&v, split_mem_, 1, s_);
+  ops::d2h(&v, split_error_, 1, s_);
   ops::sync(s_);
   int e;
   std::memcpy(&e, &v, sizeof(int));
   return e;
+}
+
+void Schedule::check_device() {
+  if (device_error()) throw Error(ERR_TIMEOUT, "a tensor-core kernel gave up a bounded wait");
 }
 
 void Schedule::profile_finish() {

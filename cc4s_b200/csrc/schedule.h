@@ -46,8 +46,12 @@ class Schedule {
   // mode also the recorded forward pass and the large contractions of the
   // reverse sweep).
   void set_precision(int slices) { precision_ = slices; }
-  // Non-zero if a bounded wait inside a tensor-core kernel expired (synchronises).
+  // Non-zero if a bounded wait inside a tensor-core kernel of this schedule has ever expired
+  // (synchronises).  What the kernel was to write is then incomplete, the integrals made
+  // once per input among it, so the word stays set: the inputs have to be set again.
   int device_error();
+  // Throws ERR_TIMEOUT if so: for every entry point, before its results are used.
+  void check_device();
 
   // Adjoint of the energy at frozen amplitudes T (amplitude-vector layout):
   //   S_dev[G]    = Re sum conj(G^ph_Gai) G^hp_Gjb (2 X_abij - X_abji), the transition
@@ -159,6 +163,7 @@ class Schedule {
   // reallocate (synchronises).  A later split_exec that needs more than `regular`
   // reallocates with an extra region of the same size (its contents are lost).
   void split_reserve(size_t regular, size_t extra);
+  void error_word();
   // One split contraction whose B was sliced by split_pack_b (recorded like tc_).
   void tc_packed_b_(const Contraction& c, const SplitPackedB& b);
   // One split contraction with both operands sliced beforehand (split_pack_operand);
@@ -195,6 +200,7 @@ class Schedule {
   int precision_ = 0;
   SplitScratch split_;
   double* split_mem_ = nullptr;
+  double* split_error_ = nullptr;
   void* split_extra_ = nullptr;
   size_t split_extra_bytes_ = 0;
   // vertex description for the adjoint (set by each schedule)

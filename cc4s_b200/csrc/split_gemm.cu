@@ -994,6 +994,24 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws,
 
 }  // namespace
 
+// FP64 contractions: the seven-digit form where its time (slicing, then the integer
+// tensor cores) is below the FP64 tensor pipe's.  The constants follow measured shapes
+// (FP64 pipe, seven digits): 512^3 37 and 41 us, 1024 x 1024 x 256 46 and 35 us,
+// 128 x 32768 x 128 61 and 83 us (slicing of an operand used 128 times),
+// 2048 x 2048 x 512 251 and 93 us, 8192^3 37.4 and 13.0 ms.
+bool digits7_pays(const Contraction& c) {
+  if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K < 64) return false;
+  const double M = double(c.M), N = double(c.N), K = double(c.K);
+  auto up = [](double x, double t) { return std::ceil(x / t) * t; };
+  // microseconds: launches, slicing, waves of one tile per SM
+  const double tiles7 = up(M, 128) * up(N, 64) / (128 * 64);
+  const int parts = split_k_parts(static_cast<int64_t>(tiles7), c.M, c.N, c.K, 7);
+  const double d7 = 20.0 + 24.0 * (M + N) * K / 3.5e6 + (parts > 1 ? 6.0 : 0.0) +
+                    std::ceil(tiles7 * parts / 148.0) * (3.3 + 0.021 * up(K, 32) / parts);
+  const double dmma = 12.0 + 2.0 * up(M, 128) * up(N, 128) * K / 22e6;
+  return d7 < dmma;
+}
+
 uint64_t split_launch_count() { return g_split_launches.load(); }
 uint64_t split_pack_launch_count() { return g_pack_launches.load(); }
 

@@ -48,6 +48,9 @@ inline int split_k_parts(int64_t tiles, int64_t M, int64_t N, int64_t K, int dig
   return best;
 }
 
+// True where an FP64 contraction runs faster in seven digits than on the FP64 tensor pipe.
+bool digits7_pays(const Contraction& c);
+
 // Same contraction semantics as gemm() (two-level index maps, optional C2).
 // The batch dimension must be 1.  Falls back to nothing: throws if the
 // contraction cannot be expressed (the caller then uses gemm()).

@@ -544,7 +544,7 @@ TriplesOutcome Triples::run(const double* T) {
   double sums[2];
   ops::d2h(sums, slots_ + 2 * ntri_, 2, s_);
   ops::sync(s_);
-  if (device_error()) throw Error(ERR_TIMEOUT, "tensor-core kernel wait expired in (T)");
+  check_device();
   // Re conj(W) Z = ReW ReZ + ImW ImZ;  Re conj(W) conj(Z) = ReW ReZ - ImW ImZ;
   // cT: Re M conj(Z) = ReM ReZ + ImM ImZ
   out.energy = reference_form_ && !complete_ ? sums[0] - sums[1] : sums[0] + sums[1];

@@ -41,7 +41,7 @@ extern "C" {
 #define CC4S_WARN_NOT_CONVERGED 4 /* warning: results are valid */
 #define CC4S_ERR_DIIS_SINGULAR 5
 #define CC4S_ERR_CUDA 6
-#define CC4S_ERR_TIMEOUT 7
+#define CC4S_ERR_TIMEOUT 7 /* a kernel gave up a bounded wait: set the inputs again */
 #define CC4S_ERR_STATE 8
 #define CC4S_ERR_NON_FINITE 9
 #define CC4S_ERR_UNSUPPORTED 10

@@ -65,12 +65,25 @@ void gemm(const Contraction& g, cudaStream_t, const GemmScratch&) {
 // base-256 digits and digit products (p + q < 4 of four digits, p + q < 8 of seven), each
 // weight summed exactly as on the device.
 static uint64_t g_split = 0, g_pack = 0;
+// Test controls: every eligible FP64 contraction in the digit form, and the n-th digit
+// contraction from now (0: the next) recording an expired wait.
+static int g_force_digits = 0, g_fail_in = -1;
+extern "C" void emu_force_digits(int on) { g_force_digits = on; }
+extern "C" void emu_fail_split_in(int n) { g_fail_in = n; }
+extern "C" uint64_t emu_split_count() { return g_split; }
+bool digits7_pays(const Contraction& c) {
+  return g_force_digits && c.batch == 1 && c.M >= 64 && c.N >= 64 && c.K >= 64;
+}
 uint64_t split_launch_count() { return g_split; }
 uint64_t split_pack_launch_count() { return g_pack; }
-size_t gemm_split_scratch_bytes(const Contraction&) { return 64; }
+size_t gemm_split_scratch_bytes(const Contraction& g) { return size_t(g.digits) * (g.M + g.N) * g.K; }
 
-void gemm_split(const Contraction& g, cudaStream_t, SplitScratch&) {
+void gemm_split(const Contraction& g, cudaStream_t, SplitScratch& ws) {
   ++g_split;
+  if (g_fail_in >= 0 && g_fail_in-- == 0) {
+    *ws.error = 1;
+    return;
+  }
   g_pack += 2;  // the device slices both operands together (two launches)
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
   const int64_t Ki = g.Ki > 0 ? g.Ki : std::max<int64_t>(g.K, 1);
@@ -130,7 +143,7 @@ void gemm_split(const Contraction& g, cudaStream_t, SplitScratch&) {
 }
 
 // The complex form: the emulation runs the four real contractions it stands for.
-size_t gemm_split_complex_scratch_bytes(const Contraction&) { return 64; }
+size_t gemm_split_complex_scratch_bytes(const Contraction& g) { return 4 * gemm_split_scratch_bytes(g); }
 void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
                         bool conjB, cudaStream_t s, SplitScratch& ws) {
   const double sA = conjA ? -1.0 : 1.0, sB = conjB ? -1.0 : 1.0;
@@ -153,7 +166,7 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
 // Pre-packed B: the emulation keeps a dense copy B[n][k] of the operand's values
 // and slices it again in gemm_split (same values, same slices).
 size_t split_packed_b_bytes(const Contraction& g) { return size_t(g.N) * g.K * 8 + 64; }
-size_t split_scratch_bytes_packed_b(const Contraction&) { return 64; }
+size_t split_scratch_bytes_packed_b(const Contraction& g) { return size_t(g.digits) * g.M * g.K; }
 bool split_single_panel(const Contraction& g) { return g.batch == 1; }
 
 SplitPackedB split_pack_b(const Contraction& g, void* dst, cudaStream_t) {
