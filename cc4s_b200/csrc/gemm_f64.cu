@@ -53,6 +53,16 @@ struct KParams {
   double* A; double* B; double* C; double* C2;
   double alpha, beta;
   double* partial;  // split-K partials [nsplit][batch][M][N] or nullptr
+  const unsigned char* only;  // Contraction::only, only_any, ...
+  const int* only_any;
+  int64_t only_ld, only_bs;
+  double alpha1;
+  __device__ __forceinline__ bool nothing() const { return only && *only_any == 0; }
+  // Whether the 64 x 64 block that holds (m, n) is computed.
+  __device__ __forceinline__ bool wanted(int64_t b, int64_t m, int64_t n) const {
+    return m < M && n < N && (!only || only[b * only_bs + (m >> 6) * only_ld + (n >> 6)] != 0);
+  }
+  __device__ __forceinline__ double factor(int64_t b) const { return only && (b & 1) ? alpha1 : alpha; }
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
@@ -146,6 +156,7 @@ __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[8], con
 // A_KC: A tile stored [m][k]; otherwise [k][m].  B_NC: B tile stored [k][n]; otherwise [n][k].
 template <class T, bool A_KC, bool B_NC, int VA, int VB>
 __global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
+  if (p.nothing()) return;
   extern __shared__ __align__(16) double smem[];
   constexpr int BM = T::BM, BN = T::BN, BK = T::BK, STAGES = T::STAGES;
   constexpr int MT = T::WM / 16, NT = T::WN / 8;  // MMA tiles of a warp
@@ -179,6 +190,10 @@ __global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
   }
   const int64_t z = blockIdx.z;
   const int64_t b = z % p.batch;
+  // (no tile and no warp's part of one straddles a block of the map without covering it)
+  if (!(p.wanted(b, m0, n0) || (BM > 64 && p.wanted(b, m0 + 64, n0)) ||
+        (BN > 64 && (p.wanted(b, m0, n0 + 64) || (BM > 64 && p.wanted(b, m0 + 64, n0 + 64))))))
+    return;
   const int split = static_cast<int>(z / p.batch);
   const int64_t kbeg = split * p.ksplit_len;
   const int64_t kend = min(p.K, kbeg + p.ksplit_len);
@@ -253,6 +268,8 @@ __global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
   cp_wait<0>();
 
   // Epilogue.
+  if (!p.wanted(b, m0 + wm, n0 + wn)) return;
+  const double alpha = p.factor(b);
   if (p.partial) {
     double* P = p.partial + (static_cast<int64_t>(split) * p.batch + b) * p.M * p.N;
 #pragma unroll
@@ -291,7 +308,7 @@ __global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
 #pragma unroll
       for (int h = 0; h < 2 * NT; ++h) {
         const int64_t n = n0 + wn + (h >> 1) * 8 + 2 * t + (h & 1);
-        val[h] = p.alpha * acc[mt][h >> 1][hh * 2 + (h & 1)];
+        val[h] = alpha * acc[mt][h >> 1][hh * 2 + (h & 1)];
         old[h] = (p.beta != 0.0 && n < p.N) ? Cb[ro + co[h]] : 0.0;
       }
 #pragma unroll
@@ -320,6 +337,7 @@ __global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
 // chain of 512 loads).
 template <int GROUPS>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(KParams p) {
+  if (p.nothing()) return;
   constexpr int PER = 256 / GROUPS;  // elements per block
   __shared__ double part[GROUPS][PER];
   const int64_t total = p.batch * p.M * p.N;
@@ -328,7 +346,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(KParams p) {
        e0 += static_cast<int64_t>(gridDim.x) * PER) {
     const int64_t e = e0 + lane;
     double s = 0.0;
-    if (e < total) {
+    const bool mine = e < total && (!p.only || p.wanted(e / (p.M * p.N), e / p.N % p.M, e % p.N));
+    if (mine) {
 #pragma unroll 8
       for (int q = warp; q < p.nsplit; q += GROUPS) s += p.partial[q * total + e];
     }
@@ -336,13 +355,13 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(KParams p) {
       part[warp][lane] = s;
       __syncthreads();
     }
-    if (warp == 0 && e < total) {
+    if (warp == 0 && mine) {
 #pragma unroll
       for (int q = 1; q < GROUPS; ++q) s += part[q][lane];
       const int64_t b = e / (p.M * p.N);
       const int64_t r = e - b * p.M * p.N;
       const int64_t m = r / p.N, n = r - (r / p.N) * p.N;
-      const double v = p.alpha * s;
+      const double v = p.factor(b) * s;
       double* c = p.C + p.Cb.off(static_cast<uint32_t>(b)) + p.Cm.off(static_cast<uint32_t>(m)) +
                   p.Cn.off(static_cast<uint32_t>(n));
       *c = (p.beta != 0.0) ? v + p.beta * *c : v;
@@ -407,7 +426,7 @@ Contraction transposed(const Contraction& g) {
 void gemm(const Contraction& g0, cudaStream_t s, const GemmScratch& ws) {
   Contraction g = g0;
   // a narrow M becomes a narrow N (not where the M tiles would exceed the grid)
-  if (g.M <= 32 && g.N > g.M && g.N < 65535 * 64) g = transposed(g0);
+  if (g.M <= 32 && g.N > g.M && g.N < 65535 * 64 && !g.only) g = transposed(g0);
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return;
   if (g.K < 0) throw Error(ERR_INVALID_ARGUMENT, "gemm: negative K");
   const int64_t lim = int64_t(1) << 31;
@@ -434,6 +453,8 @@ void gemm(const Contraction& g0, cudaStream_t s, const GemmScratch& ws) {
   p.C2b = axis(Bi, g.C2.s_bo, g.C2.s_bi);
   p.A = g.A.p; p.B = g.B.p; p.C = g.C.p; p.C2 = g.C2.p;
   p.alpha = g.alpha; p.beta = g.beta;
+  p.only = g.only; p.only_any = g.only_any; p.only_ld = g.only_ld; p.only_bs = g.only_bs;
+  p.alpha1 = g.alpha1;
   if (!p.C || (g.K > 0 && (!p.A || !p.B)))
     throw Error(ERR_INVALID_ARGUMENT, "gemm: null operand");
 

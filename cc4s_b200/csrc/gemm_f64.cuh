@@ -44,8 +44,15 @@ struct Contraction {
   View C;   // rows m, cols n
   View C2;  // optional second output (C2.p == nullptr: none): C2 = alpha*AB + beta*C2
   double alpha = 1.0, beta = 0.0;
-  // Digit form of the tensor-core contractions (split_gemm.cuh): 7 is the FP64 one.
+  // Digit form of the tensor-core contractions (split_gemm.cuh): 8 is the FP64 one.
   int digits = 4;
+  // Device map of the 64 x 64 blocks of the output, [batch][ceil(M / 64)][only_ld] bytes:
+  // gemm() computes the blocks whose byte is non-zero and leaves the others (null: all).
+  // *only_any is zero where none is.  With a map, odd batches take alpha1.
+  const unsigned char* only = nullptr;
+  const int* only_any = nullptr;
+  int64_t only_ld = 0, only_bs = 0;
+  double alpha1 = 1.0;
 };
 
 // Scratch memory used by split-K partial sums.

@@ -60,9 +60,9 @@ void Schedule::gemm_(const Contraction& c) {
   fp64_exec(c);
 }
 
-int Schedule::digits_for(const Contraction& c, bool big) const {
+int Schedule::digits_for(const Contraction& c, bool big, bool cplx) const {
   if (big && precision_ != 0 && c.batch == 1 && c.K >= 64 && c.M >= 64 && c.N >= 64) return 4;
-  return digits7_pays(c) ? 7 : 0;
+  return !fp64_pipe_ && digits8_pays(c, cplx) ? 8 : 0;
 }
 
 void Schedule::split_reserve(size_t regular, size_t extra) {
@@ -91,6 +91,11 @@ void Schedule::split_reserve(size_t regular, size_t extra) {
   }
 }
 
+SplitScratch& Schedule::split_ws() {
+  split_.fp64 = scratch_;
+  return split_;
+}
+
 // The word in which a kernel records an expired wait: in memory of its own, so that it
 // outlives the growing of the scratch, and never cleared.
 void Schedule::error_word() {
@@ -105,13 +110,13 @@ void Schedule::split_exec(const Contraction& c) {
   // growing keeps the size of the extra region (not its contents: no pre-packed
   // operand is live across a contraction that needs more than the reserved part)
   if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
-  gemm_split(c, s_, split_);
+  gemm_split(c, s_, split_ws());
 }
 
 void Schedule::fp64_exec(const Contraction& c) {
-  if (digits_for(c, false) == 7) {
+  if (digits_for(c, false) == 8) {
     Contraction d = c;
-    d.digits = 7;
+    d.digits = 8;
     bool fits = true;
     try {
       const size_t need = gemm_split_scratch_bytes(d);
@@ -121,7 +126,7 @@ void Schedule::fp64_exec(const Contraction& c) {
       fits = false;  // no room for the digits: the FP64 tensor pipe needs none
     }
     if (fits) {
-      gemm_split(d, s_, split_);
+      gemm_split(d, s_, split_ws());
       return;
     }
   }
@@ -139,11 +144,11 @@ void Schedule::tc_packed_b_(const Contraction& c, const SplitPackedB& b) {
     ev_split_.push_back(1);
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
-    gemm_split_packed_b(c, b, s_, split_);
+    gemm_split_packed_b(c, b, s_, split_ws());
     ops::event_record(ev_[2 * k + 1], s_);
     return;
   }
-  gemm_split_packed_b(c, b, s_, split_);
+  gemm_split_packed_b(c, b, s_, split_ws());
 }
 
 void Schedule::tc_prepacked_(const Contraction& c, const SplitOperand& A, const SplitRuns& ar,
@@ -159,11 +164,11 @@ void Schedule::tc_prepacked_(const Contraction& c, const SplitOperand& A, const 
     ev_split_.push_back(1);
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
-    gemm_split_prepacked(c, A, ar, B, br, s_, split_);
+    gemm_split_prepacked(c, A, ar, B, br, s_, split_ws());
     ops::event_record(ev_[2 * k + 1], s_);
     return;
   }
-  gemm_split_prepacked(c, A, ar, B, br, s_, split_);
+  gemm_split_prepacked(c, A, ar, B, br, s_, split_ws());
 }
 
 // A contraction of the reverse sweep (or a recomputed forward one): split
@@ -205,18 +210,13 @@ bool Schedule::zgemm_split(const Contraction& c, int64_t a_im, int64_t b_im, int
                            bool conjA, bool conjB, bool big) {
   if (taping_) return false;  // reverse mode records the four real contractions
   Contraction d = c;
-  d.digits = digits_for(c, big);
-  if (d.digits != 4) {
-    Contraction k2 = c;
-    k2.K = 2 * c.K;
-    d.digits = digits_for(k2, false);
-  }
+  d.digits = digits_for(c, big, true);
   if (!d.digits) return false;
   try {
     const size_t need = gemm_split_complex_scratch_bytes(d);
     if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
   } catch (const Error& e) {
-    if (e.status != ERR_OUT_OF_MEMORY || d.digits != 7) throw;
+    if (e.status != ERR_OUT_OF_MEMORY || d.digits != 8) throw;
     return false;
   }
   const double f = 8.0 * double(c.M) * double(c.N) * double(c.K);
@@ -230,7 +230,7 @@ bool Schedule::zgemm_split(const Contraction& c, int64_t a_im, int64_t b_im, int
     ev_shape_.push_back({c.M, c.N, 2 * c.K, 2});
     ops::event_record(ev_[2 * k], s_);
   }
-  gemm_split_complex(d, a_im, b_im, c_im, conjA, conjB, s_, split_);
+  gemm_split_complex(d, a_im, b_im, c_im, conjA, conjB, s_, split_ws());
   if (prof) ops::event_record(ev_[2 * k + 1], s_);
   return true;
 }

@@ -152,9 +152,9 @@ class Schedule {
   // A large contraction: split precision when enabled (batch 1), else FP64.
   // Recorded on the tape when taping, like gemm_.
   void tc_(const Contraction& c);
-  // The digit form a contraction runs in: 4 (a large one in split precision), 7 (FP64 on
-  // the integer tensor cores) or 0 (the FP64 tensor pipe).
-  int digits_for(const Contraction& c, bool big) const;
+  // The digit form a contraction runs in: 4 (a large one in split precision), 8 (FP64 on
+  // the integer tensor cores, rows permitting) or 0 (the FP64 tensor pipe).
+  int digits_for(const Contraction& c, bool big, bool cplx = false) const;
   void split_exec(const Contraction& c);
   // One contraction in FP64, in the faster of its two forms.
   void fp64_exec(const Contraction& c);
@@ -164,6 +164,7 @@ class Schedule {
   // reallocates with an extra region of the same size (its contents are lost).
   void split_reserve(size_t regular, size_t extra);
   void error_word();
+  SplitScratch& split_ws();  // split_ with the partial-sum scratch of the FP64 pipe
   // One split contraction whose B was sliced by split_pack_b (recorded like tc_).
   void tc_packed_b_(const Contraction& c, const SplitPackedB& b);
   // One split contraction with both operands sliced beforehand (split_pack_operand);
@@ -198,6 +199,7 @@ class Schedule {
            bool big = false);
   void profile_finish();
   int precision_ = 0;
+  bool fp64_pipe_ = false;  // FP64 contractions keep to the FP64 tensor pipe
   SplitScratch split_;
   double* split_mem_ = nullptr;
   double* split_error_ = nullptr;

@@ -1,7 +1,7 @@
 // FP64 contraction in signed 8-bit digits on the tcgen05 tensor cores (kind::i8).
 //
 // Kernel layout (persistent, one CTA of 320 threads per SM, 128 x TN output tiles,
-// TN = 128 with 4 digits, 64 with 7):
+// TN = 128 with 4 digits, 64 with 8):
 //   warp 0      TMA producer: per k-block all digit planes of the A rows and of the
 //               B rows (two 3-D boxes, swizzled) into a shared-memory ring, completion
 //               tracked by mbarriers;
@@ -34,28 +34,29 @@ namespace {
 
 constexpr int TM = 128;
 constexpr int KPAD = 32;                         // K step of one MMA: packed K granularity
-// |digit product| <= 2^14, at most 7 products per group and k: exact in S32 up to here
+// |digit product| <= 2^14, and 65 * 128 where the top digit takes part: at most 114944 per
+// group and k (six products and two with the top digit), exact in S32 up to here
 constexpr int KCHUNK = 16384;
 constexpr uint32_t WAIT_LIMIT = 1u << 28;         // bounded mbarrier waits
 constexpr uint32_t RASTER_M = 8;                 // tile rows per raster group
 constexpr int WBUF_DOUBLES = 32 * 16;            // transpose buffer of one epilogue warp
 constexpr int EXP_NONFINITE = INT_MAX;           // exponent of a row holding Inf or NaN
 
-// Geometry of the two forms: NS digits, groups p + q < NG, TN columns per tile (TN NG =
+// Geometry of the two forms: NS digits, groups p + q < NG = NS, TN columns per tile (TN NG =
 // the 512 TMEM columns), k-blocks of TK bytes (= the swizzle width), NST ring stages.
 template <int NS_> struct Form;
 template <> struct Form<4> {
   static constexpr int NS = 4, NG = 4, TN = 128, TK = 64, NST = 3;
 };
-template <> struct Form<7> {
-  static constexpr int NS = 7, NG = 8, TN = 64, TK = 64, NST = 2;
+template <> struct Form<8> {
+  static constexpr int NS = 8, NG = 8, TN = 64, TK = 64, NST = 2;
 };
 template <class F> __host__ __device__ constexpr int a_bytes() { return F::NS * TM * F::TK; }
 template <class F> __host__ __device__ constexpr int stage_bytes() { return F::NS * (TM + F::TN) * F::TK; }
 template <class F> constexpr int smem_bytes() {
   return F::NST * stage_bytes<F>() + 8 * WBUF_DOUBLES * 8 + 1024 + 256;
 }
-int tile_n(int digits) { return digits == 7 ? Form<7>::TN : Form<4>::TN; }
+int tile_n(int digits) { return digits == 8 ? Form<8>::TN : Form<4>::TN; }
 
 std::atomic<uint64_t> g_split_launches{0};
 std::atomic<uint64_t> g_pack_launches{0};
@@ -83,6 +84,7 @@ struct PackArgs {
   int* rexp;              // per-row exponent
   int8_t* dst;            // [NS][Rp][Kp]
   int r_contig;           // 1: the row index is the contiguous one in memory
+  float* prof;            // [Rp / 64][Kp] profiles (eight digits)
   // Two planes of a complex operand side by side along k: k < K1 reads at offset off[0]
   // with sign[0], the others at off[1] with sign[1] (K1 = K: one plane).
   int64_t K1;
@@ -110,7 +112,7 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
 // number).  A work item is 64 rows x `kstrip` k, read straight from memory with the lanes
 // along the contiguous index and 16 loads in flight per thread; one atomicMax per row.
 // Bound by latency until a few hundred items are in flight, which sets kstrip: strips of
-// 1024 k left two 1024 x 1024 operands to 32 blocks (whole seven-digit contraction 79 us,
+// 1024 k left two 1024 x 1024 operands to 32 blocks (whole contraction 79 us,
 // 63 us with strips of 128).
 __global__ void __launch_bounds__(PTHREADS) pack_max_kernel(PackSet pp, int kstrip) {
   __shared__ unsigned long long part[8][PR];
@@ -192,10 +194,11 @@ __device__ __forceinline__ double pow2i(int e) {
 
 // Digits of four elements: word q holds digit q of each, element 0 in the lowest byte.
 // With 128 added to every digit but the top one, the bytes of the integer are the digits
-// plus 128 (the carries of a balanced representation happen in the one addition).
+// plus 128 (the carries of a balanced representation happen in the one addition).  Eight
+// digits also add the magnitudes, in units of 2^-27 of the row's power of two, to sum.
 template <int NS>
 __device__ __forceinline__ void digits4(const double (&x)[4], double s1, double s2,
-                                        uint32_t (&w)[NS]) {
+                                        uint32_t (&w)[NS], uint32_t (&sum)[4]) {
   uint32_t lo[4], hi[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -203,9 +206,10 @@ __device__ __forceinline__ void digits4(const double (&x)[4], double s1, double 
       lo[j] = (static_cast<uint32_t>(__double2int_rn(x[j] * s1 * s2)) + 0x00808080u) ^ 0x00808080u;
       hi[j] = 0;
     } else {
+      const long long v = __double2ll_rn(x[j] * s1 * s2);
+      sum[j] += static_cast<uint32_t>(abs(static_cast<int>(v >> 32))) >> 3;
       const unsigned long long X =
-          (static_cast<unsigned long long>(__double2ll_rn(x[j] * s1 * s2)) + 0x0000808080808080ull) ^
-          0x0000808080808080ull;
+          (static_cast<unsigned long long>(v) + 0x0080808080808080ull) ^ 0x0080808080808080ull;
       lo[j] = static_cast<uint32_t>(X);
       hi[j] = static_cast<uint32_t>(X >> 32);
     }
@@ -220,11 +224,12 @@ __device__ __forceinline__ void digits4(const double (&x)[4], double s1, double 
   w[NS - 2] = l0.y;
   w[NS - 3] = l2.x;
   w[NS - 4] = l2.y;
-  if constexpr (NS == 7) {
+  if constexpr (NS == 8) {
     const uint2 h0 = planes(hi, 0), h2 = planes(hi, 2);
-    w[2] = h0.x;
-    w[1] = h0.y;
-    w[0] = h2.x;
+    w[3] = h0.x;
+    w[2] = h0.y;
+    w[1] = h2.x;
+    w[0] = h2.y;
   }
 }
 
@@ -236,13 +241,32 @@ __device__ __forceinline__ void digits4(const double (&x)[4], double s1, double 
 // in memory, 64 rows x 64 k through a shared-memory tile (stores of 16 bytes per row and
 // lane straight from such loads were slower: 1.14 against 0.99 ms for 256 x 262144 x 256).
 // Memory bound: 8 B read, NS B written per element.  Against tiles for both and digits
-// extracted one by one, whole contractions of 2048^3 0.291 -> 0.275 ms in seven digits,
+// extracted one by one, whole contractions (seven digits) of 2048^3 0.291 -> 0.275 ms,
 // 4096 x 256 x 16384 0.92 -> 0.87 ms, 4096 x 1024 x 65536 8.06 -> 7.83 ms.
+// Eight digits also leave the profile of the item's rows (the header says what for): sums
+// over the 8 rows of a warp in registers, from the integers that are there, then the least
+// of the eight warps' means through shared memory, which costs the unstaged items their
+// only barrier.
 constexpr int PK_K = 128, PK_R = 64;  // k per item, by the contiguous index
+// Mean magnitudes over `live` rows (all-zero rows are exact and do not count).
+__device__ __forceinline__ float4 means(const uint32_t (&s)[4], int live) {
+  const float w = live ? 0x1p-27f / static_cast<float>(live) : 0.0f;
+  const float none = live ? 0.0f : 1.0f;
+  return make_float4(s[0] * w + none, s[1] * w + none, s[2] * w + none, s[3] * w + none);
+}
+// The least of the eight warps' means.
+__device__ __forceinline__ float least(const float* part, int stride, bool odd) {
+  float v = part[0];
+#pragma unroll
+  for (int q = 1; q < 8; ++q) v = fminf(v, part[q * stride]);
+  return odd ? __int_as_float(0x7fc00000) : v;
+}
 template <int NS>
 __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
   __shared__ double tile[PR][81];  // k at k + k / 4: both directions free of bank conflicts
   __shared__ int64_t rows_off[PR], ks_off[PK_R];
+  __shared__ float cpart[8][PK_R];
+  int flip = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (uint32_t it = blockIdx.x; it < pp.end[2]; it += gridDim.x) {
     const int which = it < pp.end[0] ? 0 : it < pp.end[1] ? 1 : 2;
@@ -255,6 +279,7 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
     const int64_t lr = r0 + 8 * warp + (lane & 7);
     double s1 = 0.0, s2 = 0.0;  // their product 2^(8 NS - 2 - e), each in the normal range
     int64_t roff = -1;
+    bool live = false, odd = false;  // not all zero; neither finite nor within the exponents
     if (lr < a.R) {
       const unsigned long long mb = a.rmax[lr];
       int e = 0;
@@ -267,8 +292,13 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
         s2 = pow2i(sh - sh / 2);
       }
       if (k0 == 0) a.rexp[lr] = e;
+      live = mb != 0;
+      odd = e > kSplitMaxExponent || e < -kSplitMaxExponent;
       roff = a.ar.off(static_cast<uint32_t>(lr));
     }
+    uint32_t sum[4] = {0, 0, 0, 0};  // magnitudes of the warp's rows, per k of the lane
+    const int nlive = NS == 8 ? __popc(__ballot_sync(0xffffffffu, live) & 0xff) : 0;
+    int any_odd = odd;
     if (a.r_contig) {
       if (lane < 8) rows_off[8 * warp + lane] = roff;
       else if (lane < 16) {
@@ -306,12 +336,21 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) y[j] = tile[8 * warp + r][5 * (lane & 15) + j] * sg[j];
         uint32_t q[NS];
-        digits4<NS>(y, t1, t2, q);
+        digits4<NS>(y, t1, t2, q, sum);
         if (kb < a.Kp) {
           int8_t* d = a.dst + (r0 + 8 * warp + r) * a.Kp + kb;
 #pragma unroll
           for (int n = 0; n < NS; ++n) *reinterpret_cast<uint32_t*>(d + n * pl) = q[n];
         }
+      }
+      if (NS == 8) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 16);
+        if (lane < 16)
+          *reinterpret_cast<float4*>(&cpart[warp][4 * lane]) = means(sum, nlive);
+        any_odd = __syncthreads_or(any_odd);
+        if (threadIdx.x < PK_R && k0 + threadIdx.x < a.Kp)
+          a.prof[int64_t(wr) * a.Kp + k0 + threadIdx.x] = least(&cpart[0][threadIdx.x], PK_R, any_odd);
       }
       __syncthreads();
     } else {
@@ -338,7 +377,7 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
           const double t1 = __shfl_sync(0xffffffffu, s1, 4 * h + r);
           const double t2 = __shfl_sync(0xffffffffu, s2, 4 * h + r);
           uint32_t q[NS];
-          digits4<NS>(x[r], t1, t2, q);
+          digits4<NS>(x[r], t1, t2, q, sum);
           if (kb < a.Kp) {
             int8_t* d = a.dst + (r0 + 8 * warp + 4 * h + r) * a.Kp + kb;
 #pragma unroll
@@ -346,7 +385,57 @@ __global__ void __launch_bounds__(PTHREADS) pack_digits_kernel(PackSet pp) {
           }
         }
       }
+      if (NS == 8) {  // two buffers in turn, so that one barrier per item is enough
+        float* part = reinterpret_cast<float*>(tile) + flip * 8 * PK_K;
+        *reinterpret_cast<float4*>(part + warp * PK_K + 4 * lane) = means(sum, nlive);
+        any_odd = __syncthreads_or(any_odd);
+        if (threadIdx.x < PK_K && k0 + threadIdx.x < a.Kp)
+          a.prof[int64_t(wr) * a.Kp + k0 + threadIdx.x] = least(part + threadIdx.x, PK_K, any_odd);
+      }
     }
+    if (NS == 8) flip ^= 1;
+  }
+}
+
+// Product sums of the profiles of nI blocks of A and nJ of B: map[I][J] (and *any) tell the
+// ones below `least`, or NaN.  A block takes one I and four J, its warps share k.  Small: 20
+// flops per 64 x 64 x 4 products; the launch is most of it.
+__global__ void profile_kernel(const float* A, const float* B, int64_t nI, int64_t nJ, int64_t Kp,
+                               float least, unsigned char* map, int* any) {
+  __shared__ float part[32][4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t nq = (nJ + 3) / 4;
+  for (int64_t b = blockIdx.x; b < nI * nq; b += gridDim.x) {
+    const int64_t I = b / nq, J = (b - I * nq) * 4;
+    const float* a = A + I * Kp;
+    const float* bs[4];
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) bs[q] = B + min(J + q, nJ - 1) * Kp;
+#pragma unroll 2
+    for (int64_t k = 4 * threadIdx.x; k < Kp; k += 4 * blockDim.x) {
+      const float4 x = *reinterpret_cast<const float4*>(a + k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 y = *reinterpret_cast<const float4*>(bs[q] + k);
+        s[q] += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], d);
+      if (lane == 0) part[warp][q] = s[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 && J + threadIdx.x < nJ) {
+      float v = 0.f;
+      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) v += part[w][threadIdx.x];
+      const bool refused = !(v >= least);
+      if (map) map[I * nJ + J + threadIdx.x] = refused;
+      if (refused) *any = 1;
+    }
+    __syncthreads();
   }
 }
 
@@ -433,23 +522,13 @@ __device__ __forceinline__ void umma_row(uint32_t d, uint64_t da, uint32_t b, ui
   }
 }
 // All digit products with p + q < NG of one K step of 32: A digit p against B digits
-// 0 .. min(NS, NG - p) - 1, into groups p and up.  `init` starts the accumulators: group
-// g is first written by p = 0, or by p = 1 where g = NS.
+// 0 .. NG - p - 1, into groups p and up.  `init` starts the accumulators: every group is
+// first written by p = 0.
 template <class F, int P>
 __device__ __forceinline__ void umma_digits(uint32_t tmem, uint32_t a, uint32_t b, bool init) {
   if constexpr (P < F::NS) {
-    constexpr int CNT = F::NS < F::NG - P ? F::NS : F::NG - P;
-    const uint64_t da = sdesc<F::TK>(a + P * TM * F::TK);
-    if constexpr (P == 1 && F::NG > F::NS) {
-      if (init) {
-        umma_row<(CNT - 1) * F::TN, F::TK>(tmem + F::TN, da, b, 1u);
-        umma_row<F::TN, F::TK>(tmem + CNT * F::TN, da, b + (CNT - 1) * F::TN * F::TK, 0u);
-      } else {
-        umma_row<CNT * F::TN, F::TK>(tmem + F::TN, da, b, 1u);
-      }
-    } else {
-      umma_row<CNT * F::TN, F::TK>(tmem + P * F::TN, da, b, P == 0 && init ? 0u : 1u);
-    }
+    umma_row<(F::NG - P) * F::TN, F::TK>(tmem + P * F::TN, sdesc<F::TK>(a + P * TM * F::TK), b,
+                                         P == 0 && init ? 0u : 1u);
     umma_digits<F, P + 1>(tmem, a, b, init);
   }
 }
@@ -513,6 +592,12 @@ struct SplitParams {
   double alpha, beta;
   const int* ea; const int* eb;    // exponents of the packed rows of A and of B
   int* error;
+  const unsigned char* map;  // refused 64 x 64 blocks of the output, [ceil(M / 64)][map_ld]
+  const int* any;            // (null: none), and whether there are some
+  int64_t map_ld;
+  __device__ __forceinline__ bool refused(int64_t m, int64_t n) const {
+    return map && m < M && map[(m >> 6) * map_ld + (n >> 6)] != 0;
+  }
   // nsplit ranges of kb_len k-blocks; range q stores at C + q part_stride.
   int nsplit, kb_len;
   int64_t part_stride;
@@ -529,7 +614,7 @@ struct SplitParams {
 struct TileAt {
   int64_t m0, n0, pa, pb;
   int mlim, nlim;
-  int kb0, nkb;     // k-blocks of the work item
+  int kb0, nkb;     // k-blocks of the work item (none if the whole tile is refused)
   int64_t out;      // offset of its output
 };
 // (32-bit arithmetic: every role divides its way here once per tile, and a 64-bit division
@@ -558,6 +643,7 @@ __device__ __forceinline__ TileAt tile_at(const SplitParams& p, uint32_t t) {
   const int64_t ml = min(p.a_run - om, p.M - a.m0), nl = min(p.b_run - on, p.N - a.n0);
   a.mlim = static_cast<int>(ml < 0 ? 0 : (ml > TM ? TM : ml));
   a.nlim = static_cast<int>(nl < 0 ? 0 : (nl > TN ? TN : nl));
+  if (p.refused(a.m0, a.n0) && (a.m0 + 64 >= p.M || p.refused(a.m0 + 64, a.n0))) a.nkb = 0;
   return a;
 }
 
@@ -578,6 +664,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t ntiles = static_cast<uint32_t>(p.nMt * p.nNt * p.nsplit);
+  if (p.map && *p.any == 0) p.map = nullptr;
   constexpr int KB_PER_CHUNK = KCHUNK / TK;
   auto chunks_of = [](int nkb) { return (nkb + KB_PER_CHUNK - 1) / KB_PER_CHUNK; };
 
@@ -696,6 +783,7 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
       // power-of-two scale of a column are computed by one lane per group of 32 (or 16)
       // columns; both reach the lanes that store an element through warp shuffles
       // (offset -1: outside the output).
+      if (nchunks == 0 || p.refused(m0 + (row & 64), n0)) continue;
       const int64_t m = m0 + row;
       const bool mv = row < ta.mlim;
       // acc counts 2^-36: digit 0 weighs 2^-6 in each operand, the fourth group 2^-24 of the first
@@ -786,13 +874,15 @@ split_kernel_persistent(const __grid_constant__ CUtensorMap tmA,
 
 // C = sum over the k ranges, in order, + beta C (C2 likewise).
 __global__ void __launch_bounds__(256) split_k_sum_kernel(SplitParams p, const double* part) {
+  if (p.map && *p.any == 0) p.map = nullptr;
   const int64_t total = p.M * p.N;
   for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const uint32_t m = static_cast<uint32_t>(e / p.N), n = static_cast<uint32_t>(e - m * p.N);
+    if (p.refused(m, n)) continue;
     double v = 0.0;
 #pragma unroll 4
     for (int q = 0; q < p.nsplit; ++q) v += part[q * total + e];
-    const uint32_t m = static_cast<uint32_t>(e / p.N), n = static_cast<uint32_t>(e - m * p.N);
     double* c = p.C + p.Cm.off(m) + p.Cn.off(n);
     *c = p.beta != 0.0 ? v + p.beta * *c : v;
     if (p.C2) {
@@ -844,7 +934,7 @@ CUtensorMap make_map(void* base, int digits, int64_t Rp, int64_t Kp, int tk, int
 
 inline int64_t rup(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
-int digits_of(const Contraction& g) { return g.digits == 7 ? 7 : 4; }
+int digits_of(const Contraction& g) { return g.digits == 8 ? 8 : 4; }
 
 // Partials of the k ranges of a contraction packed over Kp.
 int parts_of(const Contraction& g, int64_t Kp) {
@@ -861,9 +951,36 @@ size_t part_bound(const Contraction& g, int64_t Kp) {
   return n > 1 ? rup(n * g.M * g.N * 8, 1024) : 0;
 }
 
+// Metadata of `rows` packed rows: whether a block is refused and the maxima (cleared by every
+// slicing), exponents and, in eight digits, profiles.
+struct Meta {
+  int* any;
+  unsigned long long* rmax;
+  int* exps;
+  float* prof;
+};
+size_t meta_clear_bytes(int64_t rows) { return 8 + rows * 8; }
+size_t meta_head_bytes(int64_t rows) { return rup(meta_clear_bytes(rows) + rows * 4, 1024); }
+size_t meta_bytes(int64_t rows, int64_t Kp, int digits) {
+  return meta_head_bytes(rows) + (digits == 8 ? rup(rows / PR * Kp * 4, 1024) : 0);
+}
+Meta meta_at(void* p, int64_t rows) {
+  unsigned char* b = static_cast<unsigned char*>(p);
+  Meta m;
+  m.any = reinterpret_cast<int*>(b);
+  m.rmax = reinterpret_cast<unsigned long long*>(b + 8);
+  m.exps = reinterpret_cast<int*>(b + meta_clear_bytes(rows));
+  m.prof = reinterpret_cast<float*>(b + meta_head_bytes(rows));
+  return m;
+}
+// The map of refused blocks of an M x N output.
+size_t map_bytes(int64_t M, int64_t N, int digits) {
+  return digits == 8 ? rup(rup(M, PR) / PR * (rup(N, PR) / PR), 1024) : 0;
+}
+
 struct Layout2 {
   int64_t Mp, Np, Kp;
-  size_t a_bytes, b_bytes, meta_bytes, part_bytes;
+  size_t a_bytes, b_bytes, meta, map, part_bytes;
 };
 Layout2 layout_of(const Contraction& g) {
   const int D = digits_of(g);
@@ -873,13 +990,14 @@ Layout2 layout_of(const Contraction& g) {
   L.Kp = rup(std::max<int64_t>(g.K, 1), KPAD);
   L.a_bytes = rup(static_cast<int64_t>(D * L.Mp * L.Kp), 1024);
   L.b_bytes = rup(static_cast<int64_t>(D * L.Np * L.Kp), 1024);
-  L.meta_bytes = rup((L.Mp + L.Np) * (8 + 4), 1024);
+  L.meta = meta_bytes(L.Mp + L.Np, L.Kp, D);
+  L.map = map_bytes(g.M, g.N, D);
   L.part_bytes = part_bytes(g, L.Kp);
   return L;
 }
 
 PackArgs pack_args(const View& v, bool rows_are_m, const Contraction& g, int64_t R, int64_t Rp,
-                   int64_t Kp, void* dst, unsigned long long* rmax, int* rexp) {
+                   int64_t Kp, void* dst, const Meta& m, int64_t row0) {
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
   const int64_t Ki = g.Ki > 0 ? g.Ki : std::max<int64_t>(g.K, 1);
   PackArgs a;
@@ -894,16 +1012,18 @@ PackArgs pack_args(const View& v, bool rows_are_m, const Contraction& g, int64_t
     a.r_contig = (v.s_ci == 1 && v.s_ri != 1) ? 1 : 0;
   }
   a.R = R; a.K = g.K; a.Rp = Rp; a.Kp = Kp;
-  a.rmax = rmax; a.rexp = rexp; a.dst = static_cast<int8_t*>(dst);
+  a.rmax = m.rmax + row0; a.rexp = m.exps + row0; a.dst = static_cast<int8_t*>(dst);
+  a.prof = m.prof + row0 / PR * Kp;
   a.K1 = a.K; a.off[0] = a.off[1] = 0; a.sign[0] = a.sign[1] = 1.0;
   if (Rp % PR || Kp % 16) throw Error(ERR_BAD_SHAPE, "gemm_split: packed extents not tiled");
   return a;
 }
 
-// Row maxima and digits of one to three operands.  Their rmax arrays are one block of
-// `rows` entries starting at that of the first (cleared here).
-void pack(const PackArgs* const* ops, int n, int64_t rows, int digits, cudaStream_t s) {
-  CC_CHECK(cudaMemsetAsync(ops[0]->rmax, 0, rows * sizeof(unsigned long long), s));
+// Row maxima and digits of one to three operands, whose rows share one block of metadata of
+// `rows` rows (cleared here).
+void pack(const PackArgs* const* ops, int n, const Meta& m, int64_t rows, int digits,
+          cudaStream_t s) {
+  CC_CHECK(cudaMemsetAsync(m.any, 0, meta_clear_bytes(rows), s));
   PackSet pp;
   for (int k = 0; k < 3; ++k) pp.op[k] = *ops[std::min(k, n - 1)];
   // strips of k for the maxima: the longest of 128 .. 1024 that gives 148 x 6 work items
@@ -929,14 +1049,26 @@ void pack(const PackArgs* const* ops, int n, int64_t rows, int digits, cudaStrea
   CC_LAUNCH_CHECK();
   work = items(tiles);
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(work, 148 * 8));
-  if (digits == 7) pack_digits_kernel<7><<<grid, PTHREADS, 0, s>>>(pp);
+  if (digits == 8) pack_digits_kernel<8><<<grid, PTHREADS, 0, s>>>(pp);
   else pack_digits_kernel<4><<<grid, PTHREADS, 0, s>>>(pp);
   CC_LAUNCH_CHECK();
   g_pack_launches.fetch_add(2);
 }
-void pack_one(const PackArgs& a, int64_t rows, int digits, cudaStream_t s) {
+void pack_one(const PackArgs& a, const Meta& m, int64_t rows, int digits, cudaStream_t s) {
   const PackArgs* op = &a;
-  pack(&op, 1, rows, digits, s);
+  pack(&op, 1, m, rows, digits, s);
+}
+
+// The refused blocks of an M x N output from the profiles of its operands.
+void profiles(const float* A, const float* B, int64_t M, int64_t N, int64_t K, int64_t Kp,
+              unsigned char* map, int* any, cudaStream_t s) {
+  const int64_t nI = rup(M, PR) / PR, nJ = rup(N, PR) / PR, work = nI * ((nJ + 3) / 4);
+  int threads = 32;  // more warps share k where there are few pairs of blocks
+  while (threads < 1024 && work * threads < 148 * 2048 && threads * 4 < Kp) threads *= 2;
+  profile_kernel<<<static_cast<unsigned>(std::min<int64_t>(work, 148 * 32)), threads, 0, s>>>(
+      A, B, nI, nJ, Kp, split_profile_least(K), map, any);
+  CC_LAUNCH_CHECK();
+  g_pack_launches.fetch_add(1);
 }
 
 // Packed slices of both operands are limited to this many bytes: a longer K is
@@ -994,22 +1126,28 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws,
 
 }  // namespace
 
-// FP64 contractions: the seven-digit form where its time (slicing, then the integer
-// tensor cores) is below the FP64 tensor pipe's.  The constants follow measured shapes
-// (FP64 pipe, seven digits): 512^3 37 and 41 us, 1024 x 1024 x 256 46 and 35 us,
-// 128 x 32768 x 128 61 and 83 us (slicing of an operand used 128 times),
-// 2048 x 2048 x 512 251 and 93 us, 8192^3 37.4 and 13.0 ms.
-bool digits7_pays(const Contraction& c) {
+// FP64 contractions: the eight-digit form where its time (launches, slicing at 24 bytes per
+// element, waves of one tile per SM) is below the FP64 tensor pipe's.  The constants follow
+// measured contractions that accumulate (FP64 pipe, eight digits, us): 512 x 512 x 512 30 and 55,
+// 1024 x 1024 x 256 47 and 51, x 1024 107 and 70; 128 x 8192 x 1024 108 and 135,
+// 64 x 32768 x 1024 184 and 376 (slicing of an operand used 64 times), 1067 x 1067 x 512 68
+// and 70, 2048 x 2048 x 256 160 and 82, 256 x 256 x 16384 111 and 142; complex, four real
+// ones and the digit form: 512 x 512 x 256 82 and 91, 512 x 512 x 512 122 and 114,
+// 1024 x 1024 x 64 62 and 67, x 256 187 and 86, 64 x 32768 x 1024 737 and 939.
+bool digits8_pays(const Contraction& c, bool cplx) {
   if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K < 64) return false;
-  const double M = double(c.M), N = double(c.N), K = double(c.K);
+  const double M = double(c.M), N = double(c.N), K = double(c.K), P = cplx ? 2.0 : 1.0;
   auto up = [](double x, double t) { return std::ceil(x / t) * t; };
-  // microseconds: launches, slicing, waves of one tile per SM
-  const double tiles7 = up(M, 128) * up(N, 64) / (128 * 64);
-  const int parts = split_k_parts(static_cast<int64_t>(tiles7), c.M, c.N, c.K, 7);
-  const double d7 = 20.0 + 24.0 * (M + N) * K / 3.5e6 + (parts > 1 ? 6.0 : 0.0) +
-                    std::ceil(tiles7 * parts / 148.0) * (3.3 + 0.021 * up(K, 32) / parts);
-  const double dmma = 12.0 + 2.0 * up(M, 128) * up(N, 128) * K / 22e6;
-  return d7 < dmma;
+  const double tiles = up(M, 128) * up(N, 64) / (128 * 64);
+  const double rows = cplx ? M + N + std::min(M, N) : M + N;
+  const int parts = split_k_parts(static_cast<int64_t>(tiles), c.M, c.N, c.K * (cplx ? 2 : 1), 8);
+  const double d8 = (cplx ? 58.0 : 38.0) + 24.0 * rows * P * K / 3.5e6 +
+                    P * ((parts > 1 ? 6.0 : 0.0) +
+                         std::ceil(tiles * parts / 148.0) * (3.3 + 0.021 * up(P * K, 32) / parts));
+  // (outputs beyond 2^22 elements no longer stay in L2 between their load and their store)
+  const double dmma = P * P * (15.0 + 2.0 * up(M, 64) * up(N, 64) * K / 24.5e6 +
+                               std::max(0.0, M * N - 4194304.0) / 1.6e5);
+  return d8 < dmma;
 }
 
 uint64_t split_launch_count() { return g_split_launches.load(); }
@@ -1019,17 +1157,17 @@ size_t gemm_split_scratch_bytes(const Contraction& g) {
   Contraction h = g;
   h.K = std::min(g.K, panel_len(g));
   const Layout2 L = layout_of(h);
-  return L.a_bytes + L.b_bytes + L.meta_bytes + part_bound(g, L.Kp);
+  return L.a_bytes + L.b_bytes + L.meta + L.map + part_bound(g, L.Kp);
 }
 
 size_t split_packed_b_bytes(const Contraction& g) {
   const Layout2 L = layout_of(g);
-  return L.b_bytes + rup(L.Np * 8, 1024) + rup(L.Np * 4, 1024);
+  return L.b_bytes + meta_bytes(L.Np, L.Kp, digits_of(g));
 }
 
 size_t split_scratch_bytes_packed_b(const Contraction& g) {
   const Layout2 L = layout_of(g);
-  return L.a_bytes + L.meta_bytes + part_bound(g, L.Kp);
+  return L.a_bytes + L.meta + L.map + part_bound(g, L.Kp);
 }
 
 bool split_single_panel(const Contraction& g) { return g.K <= panel_len(g) && g.batch == 1; }
@@ -1040,10 +1178,11 @@ SplitPackedB split_pack_b(const Contraction& g, void* dst, cudaStream_t s) {
   unsigned char* p = static_cast<unsigned char*>(dst);
   SplitPackedB b;
   b.slices = p;
-  auto* bmax = reinterpret_cast<unsigned long long*>(p + L.b_bytes);
-  b.exps = reinterpret_cast<int*>(p + L.b_bytes + rup(L.Np * 8, 1024));
+  const Meta m = meta_at(p + L.b_bytes, L.Np);
+  b.exps = m.exps;
   b.N = g.N; b.K = g.K; b.Np = L.Np; b.Kp = L.Kp; b.digits = digits_of(g);
-  pack_one(pack_args(g.B, false, g, g.N, L.Np, L.Kp, b.slices, bmax, b.exps), g.N, b.digits, s);
+  b.prof = m.prof;
+  pack_one(pack_args(g.B, false, g, g.N, L.Np, L.Kp, b.slices, m, 0), m, L.Np, b.digits, s);
   return b;
 }
 
@@ -1112,12 +1251,13 @@ void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, SplitParams sp, d
 }
 
 // The output side of a contraction and the runs of its packed rows -> one launch, or with
-// room for partials (part_bytes) one launch over the k ranges and their sum.
+// room for partials (part_bytes) one launch over the k ranges and their sum; of the
+// blocks that the contraction's map does not leave to gemm().
 void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t Ap,
             const SplitRuns& ar, int64_t nra, void* Bpk, const int* eb, int64_t Bp,
             const SplitRuns& br, int64_t nrb, int64_t Kp, double* part, cudaStream_t s,
             SplitScratch& ws) {
-  const int tn = tile_n(digits), tk = digits == 7 ? Form<7>::TK : Form<4>::TK;
+  const int tn = tile_n(digits), tk = digits == 8 ? Form<8>::TK : Form<4>::TK;
   const CUtensorMap ta = make_map(Apk, digits, Ap, Kp, tk, TM);
   const CUtensorMap tb = make_map(Bpk, digits, Bp, Kp, tk, tn);
   const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N;
@@ -1131,6 +1271,8 @@ void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t 
   sp.alpha = g.alpha; sp.beta = g.beta;
   sp.ea = ea; sp.eb = eb;
   sp.error = ws.error;
+  sp.map = g.only; sp.any = g.only_any;
+  sp.map_ld = g.only_ld;
   sp.nsplit = part ? parts_of(g, Kp) : 1;
   sp.a_run = ar.run; sp.a_stride = ar.stride; sp.a_base = ar.base;
   sp.a_tiles = (ar.run + TM - 1) / TM; sp.nMt = nra * sp.a_tiles;
@@ -1139,7 +1281,7 @@ void launch(const Contraction& g, int digits, void* Apk, const int* ea, int64_t 
   if (sp.nMt * sp.nNt * sp.nsplit >= (int64_t(1) << 31) || Ap >= (int64_t(1) << 31) ||
       Bp >= (int64_t(1) << 31) || Kp >= (int64_t(1) << 31))
     throw Error(ERR_BAD_SHAPE, "gemm_split: extent too large");
-  if (digits == 7) launch_form<Form<7>>(ta, tb, sp, part, s);
+  if (digits == 8) launch_form<Form<8>>(ta, tb, sp, part, s);
   else launch_form<Form<4>>(ta, tb, sp, part, s);
 }
 
@@ -1147,34 +1289,43 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws, const S
   const Layout2 L = layout_of(g);
   const int D = digits_of(g);
   // with a pre-packed B the scratch holds A and the metadata only
-  const size_t base = L.a_bytes + (pb ? 0 : L.b_bytes) + L.meta_bytes;
+  const size_t base = L.a_bytes + (pb ? 0 : L.b_bytes) + L.meta + L.map;
   if (base + L.part_bytes > ws.bytes)
     throw Error(ERR_OUT_OF_MEMORY, "gemm_split: scratch too small");
   unsigned char* p = static_cast<unsigned char*>(ws.p);
   void* Apk = p;
   void* Bpk = p + L.a_bytes;
   unsigned char* meta = p + L.a_bytes + (pb ? 0 : L.b_bytes);
-  auto* amax = reinterpret_cast<unsigned long long*>(meta);
-  auto* bmax = amax + L.Mp;
-  int* aexp = reinterpret_cast<int*>(bmax + L.Np);
-  int* bexp = aexp + L.Mp;
-  const PackArgs pa = pack_args(g.A, true, g, g.M, L.Mp, L.Kp, Apk, amax, aexp);
+  const Meta m = meta_at(meta, L.Mp + L.Np);
+  const int* bexp = m.exps + L.Mp;
+  const float* bprof = m.prof + L.Mp / PR * L.Kp;
+  const PackArgs pa = pack_args(g.A, true, g, g.M, L.Mp, L.Kp, Apk, m, 0);
   if (pb) {   // B sliced before, by split_pack_b, for this N, K and padding
     if (pb->N != g.N || pb->K != g.K || pb->Np != L.Np || pb->Kp != L.Kp || pb->digits != D)
       throw Error(ERR_INVALID_ARGUMENT, "gemm_split: pre-packed B of another shape");
     Bpk = pb->slices;
     bexp = pb->exps;
-    pack_one(pa, L.Mp, D, s);
+    bprof = pb->prof;
+    pack_one(pa, m, L.Mp, D, s);
   } else {
-    const PackArgs pbk = pack_args(g.B, false, g, g.N, L.Np, L.Kp, Bpk, bmax, bexp);
+    const PackArgs pbk = pack_args(g.B, false, g, g.N, L.Np, L.Kp, Bpk, m, L.Mp);
     const PackArgs* both[2] = {&pa, &pbk};
-    pack(both, 2, L.Mp + L.Np, D, s);
+    pack(both, 2, m, L.Mp + L.Np, D, s);
+  }
+  Contraction h = g;
+  if (D == 8) {
+    unsigned char* map = meta + L.meta;
+    profiles(m.prof, bprof, g.M, g.N, g.K, L.Kp, map, m.any, s);
+    h.only = map;
+    h.only_any = m.any;
+    h.only_ld = rup(g.N, PR) / PR;
   }
   SplitRuns ar, br;
   ar.run = g.M;
   br.run = g.N;
   double* part = L.part_bytes ? reinterpret_cast<double*>(p + base) : nullptr;
-  launch(g, D, Apk, aexp, L.Mp, ar, 1, Bpk, bexp, L.Np, br, 1, L.Kp, part, s, ws);
+  launch(h, D, Apk, m.exps, L.Mp, ar, 1, Bpk, bexp, L.Np, br, 1, L.Kp, part, s, ws);
+  if (D == 8) gemm(h, s, ws.fp64);
 }
 
 }  // namespace
@@ -1184,7 +1335,7 @@ namespace {
 struct ComplexLayout {
   int64_t Mp, Np, Kp;
   int na, nb;            // forms of A and of B
-  size_t a_bytes, b_bytes, meta_bytes, part_bytes;  // slices per form, meta of all forms
+  size_t a_bytes, b_bytes, meta, map, part_bytes;  // slices per form, meta of all, map per plane
 };
 ComplexLayout complex_layout(const Contraction& g, int64_t K) {
   const int D = digits_of(g);
@@ -1196,7 +1347,8 @@ ComplexLayout complex_layout(const Contraction& g, int64_t K) {
   L.nb = 3 - L.na;
   L.a_bytes = rup(D * L.Mp * L.Kp, 1024);
   L.b_bytes = rup(D * L.Np * L.Kp, 1024);
-  L.meta_bytes = rup((L.na * L.Mp + L.nb * L.Np) * (8 + 4), 1024);
+  L.meta = meta_bytes(L.na * L.Mp + L.nb * L.Np, L.Kp, D);
+  L.map = map_bytes(g.M, g.N, D);
   L.part_bytes = part_bytes(g, L.Kp);
   return L;
 }
@@ -1207,7 +1359,7 @@ int64_t complex_panel_len(const Contraction& g) {
   return std::max<int64_t>(KPAD, P / KPAD * KPAD);
 }
 size_t complex_bytes(const ComplexLayout& L) {
-  return L.na * L.a_bytes + L.nb * L.b_bytes + L.meta_bytes + L.part_bytes;
+  return L.na * L.a_bytes + L.nb * L.b_bytes + L.meta + 2 * L.map + L.part_bytes;
 }
 }  // namespace
 
@@ -1234,9 +1386,8 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
     if (complex_bytes(L) > ws.bytes)
       throw Error(ERR_OUT_OF_MEMORY, "gemm_split_complex: scratch too small");
     unsigned char* p = static_cast<unsigned char*>(ws.p);
-    auto* rmax = reinterpret_cast<unsigned long long*>(p + L.na * L.a_bytes + L.nb * L.b_bytes);
     const int64_t rows = L.na * L.Mp + L.nb * L.Np;
-    int* rexp = reinterpret_cast<int*>(rmax + rows);
+    const Meta m = meta_at(p + L.na * L.a_bytes + L.nb * L.b_bytes, rows);
     PackArgs op[3];
     const PackArgs* ops[3] = {&op[0], &op[1], &op[2]};
     int64_t r = 0;
@@ -1245,7 +1396,7 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
       const int form = isA ? k : k - L.na;
       void* dst = isA ? p + k * L.a_bytes : p + L.na * L.a_bytes + form * L.b_bytes;
       op[k] = pack_args(isA ? h.A : h.B, isA, h, isA ? h.M : h.N, isA ? L.Mp : L.Np, L.Kp, dst,
-                        rmax + r, rexp + r);
+                        m, r);
       r += isA ? L.Mp : L.Np;
       const int64_t im = isA ? a_im : b_im;
       op[k].K = 2 * h.K;
@@ -1264,10 +1415,10 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
         }
       }
     }
-    pack(ops, 3, rows, D, s);
-    double* part_mem = L.part_bytes ? reinterpret_cast<double*>(p + L.na * L.a_bytes +
-                                                                L.nb * L.b_bytes + L.meta_bytes)
-                                    : nullptr;
+    pack(ops, 3, m, rows, D, s);
+    unsigned char* maps = p + L.na * L.a_bytes + L.nb * L.b_bytes + L.meta;
+    const int64_t map1 = static_cast<int64_t>(L.map);
+    double* part_mem = L.part_bytes ? reinterpret_cast<double*>(maps + 2 * L.map) : nullptr;
     SplitRuns ar, br;
     ar.run = h.M;
     br.run = h.N;
@@ -1280,16 +1431,40 @@ void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_
         c.C.p = g.C.p + c_im;
         if (g.C2.p) c.C2.p = g.C2.p + c_im;
       }
+      if (D == 8) {
+        c.only = maps + part * map1;
+        c.only_any = m.any;
+        c.only_ld = rup(h.N, PR) / PR;
+        profiles(A.prof, B.prof, h.M, h.N, c.K, L.Kp, maps + part * map1, m.any, s);
+      }
       launch(c, D, A.dst, A.rexp, L.Mp, ar, 1, B.dst, B.rexp, L.Np, br, 1, L.Kp,
              part_mem, s, ws);
+    }
+    // The refused blocks: Re A and then Im A on both planes of B, the planes of the output
+    // as a batch of two.
+    for (int term = 0; D == 8 && term < 2; ++term) {
+      Contraction c = h;
+      c.batch = 2;
+      c.A.s_bi = c.A.s_bo = 0;
+      if (term) c.A.p += a_im;
+      if (term) c.B.p += b_im;
+      c.B.s_bi = term ? -b_im : b_im;
+      c.C.s_bi = c.C2.s_bi = c_im;
+      c.alpha1 = c.alpha * (term ? sA : sB);
+      if (term) c.alpha *= -sA * sB;
+      if (term) c.beta = 1.0;
+      c.only = maps;
+      c.only_any = m.any;
+      c.only_ld = rup(h.N, PR) / PR;
+      c.only_bs = map1;
+      gemm(c, s, ws.fp64);
     }
   }
 }
 
 size_t split_operand_bytes(int64_t R, int64_t K, int digits) {
   const int64_t Rp = rup(std::max<int64_t>(R, 1), TM), Kp = rup(std::max<int64_t>(K, 1), KPAD);
-  return static_cast<size_t>(rup(digits * Rp * Kp, 1024) + rup(Rp * 8, 1024) +
-                             rup(Rp * 4, 1024));
+  return static_cast<size_t>(rup(digits * Rp * Kp, 1024)) + meta_bytes(Rp, Kp, digits);
 }
 
 SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_t s_ro,
@@ -1305,14 +1480,22 @@ SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_
   unsigned char* p = static_cast<unsigned char*>(dst);
   const int64_t sb = rup(digits * o.Rp * o.Kp, 1024);
   o.slices = p;
-  auto* rmax = reinterpret_cast<unsigned long long*>(p + sb);
-  o.exps = reinterpret_cast<int*>(p + sb + rup(o.Rp * 8, 1024));
+  const Meta m = meta_at(p + sb, o.Rp);
+  o.exps = m.exps;
+  o.prof = m.prof;
   Contraction g;
   g.M = R; g.Mi = Ri; g.K = K;
   g.A.p = const_cast<double*>(src);
   g.A.s_ro = s_ro; g.A.s_ri = s_ri; g.A.s_co = 0; g.A.s_ci = s_k;
-  pack_one(pack_args(g.A, true, g, R, o.Rp, o.Kp, o.slices, rmax, o.exps), R, digits, s);
+  pack_one(pack_args(g.A, true, g, R, o.Rp, o.Kp, o.slices, m, 0), m, o.Rp, digits, s);
   return o;
+}
+
+void split_refused(const SplitOperand& A, const SplitOperand& B, int* word, cudaStream_t s) {
+  if (A.digits != 8 || B.digits != 8 || A.K != B.K)
+    throw Error(ERR_INVALID_ARGUMENT, "split_refused: operands of another form");
+  CC_CHECK(cudaMemsetAsync(word, 0, 8, s));
+  profiles(A.prof, B.prof, A.R, B.R, A.K, A.Kp, nullptr, word, s);
 }
 
 void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const SplitRuns& ar,

@@ -9,14 +9,29 @@
 // combined in exact 64-bit integers before the one conversion to FP64.
 //   digits = 4 (30 bits of each operand relative to its row / column maximum): the ten
 //     products p + q < 4; the split-precision form.
-//   digits = 7 (54 bits, i.e. FP64's 53 for the largest element of a row): the 34
-//     products p + q < 8.  What is left out is below 2^-63 of the row times the column
-//     maximum, and the sum over k adds no rounding, so the result is at least as close
-//     to the exact one as an FP64 accumulation of more than a few terms.
-// A row or column holding an Inf or NaN gives NaN in all its outputs.
+//   digits = 8 (62 bits): the 36 products p + q < 8; the FP64 form.
+//
+// The error of a digit form is relative to the row and column maxima: with the row of A
+// below 2^ea and the column of B below 2^eb it is about 2^-61 sqrt(K) 2^(ea+eb) in eight
+// digits, while an FP64 accumulation is off by about 2^-54 sum_k |a_k b_k|.  Where the large
+// elements of a row of A meet small ones of a column of B, that sum is far below
+// K 2^(ea+eb), and a digit form loses what FP64 keeps.  So eight digits hold only where the
+// sum is large enough.  The slicing pass takes a profile over k of every 64 rows of an
+// operand (the least, over its groups of 8 rows, of their mean of |x| 2^-e); the product
+// sum of two profiles stands for sum_k |a_k b_k| 2^-(ea+eb) of that 64 x 64 block of the
+// output, and a block below 2^-10 sqrt(K), or with a non-finite element or a row maximum
+// outside 2^+-400, is refused: gemm() computes it on the FP64 tensor pipe, all decided on
+// the device.  Measured on 64 x 64 outputs, K = 64 .. 4096, largest error over sum |a b| in
+// 2^-53 (FP64 chain, eight digits), by the product sum over sqrt(K): even Gaussian rows 0.1
+// .. 0.8: 3, 0.4 .. 0.04; one element 300 times the others 1e-3 .. 7e-3: 14, 2 .. 0.5; A
+// falling and B rising along k over a factor of 300 2e-3 .. 3e-3: 3, 4 .. 0.7, over 1000
+// 7e-4 .. 1e-3: 3, 12 .. 2 (refused up to K = 2048), over 1e6 1e-6: 3, 14000 .. 2000.
+// (Seven digits of 34 products were at 17 on the factor of 100 that eight hold at 1.)
+// In four digits, a row or column holding an Inf or NaN gives NaN in all its outputs.
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 
 #include "gemm_f64.cuh"
 
@@ -26,7 +41,14 @@ struct SplitScratch {
   void* p = nullptr;     // device scratch for the packed slices
   size_t bytes = 0;
   int* error = nullptr;  // device flag: non-zero if a bounded wait gave up
+  GemmScratch fp64;      // split-K partials of the blocks that eight digits refuse
 };
+
+// The rule above: what the product sum of two profiles has to reach.
+inline float split_profile_least(int64_t K) {
+  return static_cast<float>(std::sqrt(static_cast<double>(K)) * 0x1p-9);
+}
+constexpr int kSplitMaxExponent = 400;
 
 // Ranges of k that share out the SMs when an output has few tiles (each range writes its
 // own FP64 partial, added in order afterwards): the number with the least time by waves of
@@ -36,7 +58,7 @@ inline int64_t split_k_most(int64_t M, int64_t N, int64_t K) {
                            (int64_t(1) << 23) / std::max<int64_t>(M * N, 1));
 }
 inline int split_k_parts(int64_t tiles, int64_t M, int64_t N, int64_t K, int digits) {
-  const double per_k = digits == 7 ? 0.019 : 0.012;
+  const double per_k = digits == 8 ? 0.020 : 0.012;
   const int64_t most = split_k_most(M, N, K);
   int best = 1;
   double least = 0.0;
@@ -48,8 +70,9 @@ inline int split_k_parts(int64_t tiles, int64_t M, int64_t N, int64_t K, int dig
   return best;
 }
 
-// True where an FP64 contraction runs faster in seven digits than on the FP64 tensor pipe.
-bool digits7_pays(const Contraction& c);
+// True where an FP64 contraction (planar complex: one of gemm_split_complex) runs faster in
+// eight digits than on the FP64 tensor pipe.
+bool digits8_pays(const Contraction& c, bool cplx);
 
 // Same contraction semantics as gemm() (two-level index maps, optional C2).
 // The batch dimension must be 1.  Falls back to nothing: throws if the
@@ -73,6 +96,7 @@ size_t gemm_split_complex_scratch_bytes(const Contraction& g);
 struct SplitPackedB {
   void* slices = nullptr;  // [digits][Np][Kp] signed bytes
   int* exps = nullptr;     // [Np] power-of-two column scales
+  float* prof = nullptr;   // [Np / 64][Kp] profiles (eight digits)
   int64_t N = 0, K = 0, Np = 0, Kp = 0;
   int digits = 4;
 };
@@ -95,6 +119,7 @@ void gemm_split_packed_b(const Contraction& g, const SplitPackedB& b, cudaStream
 struct SplitOperand {
   void* slices = nullptr;
   int* exps = nullptr;   // [Rp]
+  float* prof = nullptr;   // [Rp / 64][Kp] profiles (eight digits)
   int64_t R = 0, K = 0, Rp = 0, Kp = 0;
   int digits = 4;
 };
@@ -113,10 +138,14 @@ struct SplitRuns {
 // C = alpha A B + beta C (g gives M, N, K, the output views, alpha, beta) with the rows
 // m of A and the columns n of B taken from sliced operands (B sliced by its columns,
 // i.e. its rows are n).  Tiles never straddle a run, so a run shorter than a tile
-// costs a partial tile.
+// costs a partial tile.  Nothing is refused here: see split_refused.
 void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const SplitRuns& ar,
                           const SplitOperand& B, const SplitRuns& br, cudaStream_t s,
                           SplitScratch& ws);
+
+// Whether eight digits refuse any block of the products of these two operands' rows: *word
+// (8 bytes of device memory, cleared here) is non-zero if so.
+void split_refused(const SplitOperand& A, const SplitOperand& B, int* word, cudaStream_t s);
 
 uint64_t split_launch_count();
 // Number of operand-slicing kernel launches issued so far (two per

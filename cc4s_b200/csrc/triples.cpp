@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cstring>
 #include <set>
 #include <vector>
 
@@ -189,6 +190,26 @@ void Triples::pack_operands(int w, const double* Ac, const double* Bc) {
     s.A2 = split_pack_operand(A, o * n1, n1, kc, o * kc, kc, 1, p + ba, s_, digits_);
     s.B = split_pack_operand(B, v * n1, 0, 0, kc, kc, 1, p + 2 * ba, s_, digits_);
   }
+}
+
+// Whether eight digits refuse a block of the sliced operands' products.
+bool Triples::operands_refused() {
+  double word[16] = {};
+  int n = 0;
+  for (int w = 0; w < (complete_ ? 2 : 1); ++w)
+    for (int pa = 0; pa < (cplx_ ? 2 : 1); ++pa)
+      for (int pb = 0; pb < (cplx_ ? 2 : 1); ++pb)
+        for (const SplitOperand* A : {&sl_[w][pa].A, &sl_[w][pa].A2}) {
+          split_refused(*A, sl_[w][pb].B, reinterpret_cast<int*>(slots_), s_);
+          ops::d2h(&word[n++], slots_, 1, s_);
+        }
+  ops::sync(s_);
+  for (double v : word) {
+    int any;
+    std::memcpy(&any, &v, sizeof(int));
+    if (any) return true;
+  }
+  return false;
 }
 
 void Triples::connected_packed(const ops::TriplesBlock& b, const int64_t X[3], const int64_t n[3],
@@ -463,17 +484,21 @@ TriplesOutcome Triples::run(const double* T) {
   concat_operands(T, Vppph_, Vhhhp_, Ac_, Bc_);
   if (complete_) concat_operands(T, Ip_, Ih_, AcM_, BcM_);
   // Both operands sliced once here where the contractions' K = v + o is long enough: in
-  // four digits (split precision), or in seven (FP64) once a block of pairs fills tiles (the
+  // four digits (split precision), or in eight (FP64) once a block of pairs fills tiles (the
   // block loop of 16/128, 224 pairs, 260 -> 184 ms; below a tile's 128 rows most of it is
   // padding).
-  digits_ = kc_ < 64 ? 0 : precision_ == 3 ? 4 : nb * o >= 128 ? 7 : 0;
+  digits_ = kc_ < 64 ? 0 : precision_ == 3 ? 4 : nb * o >= 128 ? 8 : 0;
   if (digits_) {
     try {
       pack_operands(0, Ac_, Bc_);
       if (complete_) pack_operands(1, AcM_, BcM_);
     } catch (const Error& e) {
-      if (e.status != ERR_OUT_OF_MEMORY || digits_ != 7) throw;
+      if (e.status != ERR_OUT_OF_MEMORY || digits_ != 8) throw;
       digits_ = 0;  // no room for the digits: the FP64 tensor pipe needs none
+    }
+    if (digits_ == 8 && operands_refused()) {
+      digits_ = 0;
+      fp64_pipe_ = true;
     }
   }
   const bool packed = digits_ != 0;

@@ -94,6 +94,7 @@ class Triples : public Schedule {
   // Slices Ac (rows (pair, hole) and (hole, pair)) and Bc (rows (virtual, pair)) of
   // every plane for connected_packed.
   void pack_operands(int w, const double* Ac, const double* Bc);
+  bool operands_refused();
   // Ac[(a,i)][j][k] = T_adij (k = d < v), -V^h_jail^* (k = v + l);
   // Bc[b][(c,k)][k'] = V^p_bcdk (k' = d < v), T_cbkl (k' = v + l); V^p in the layout of
   // Vppph_, V^h in that of Vhhhp_.

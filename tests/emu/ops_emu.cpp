@@ -46,6 +46,7 @@ void gemm(const Contraction& g, cudaStream_t, const GemmScratch&) {
     for (int64_t m = 0; m < g.M; ++m) {
       const int64_t am = Am.off(m);
       for (int64_t n = 0; n < g.N; ++n) {
+        if (g.only && !g.only[b * g.only_bs + (m / 64) * g.only_ld + n / 64]) continue;
         const int64_t bn = Bn.off(n);
         double s = 0.0;
         for (int64_t k = 0; k < g.K; ++k) s += A[am + ak[k]] * B[bk[k] + bn];
@@ -62,23 +63,72 @@ void gemm(const Contraction& g, cudaStream_t, const GemmScratch&) {
 }
 
 // Emulation of the digit-form contraction: the same row/column scaling, balanced
-// base-256 digits and digit products (p + q < 4 of four digits, p + q < 8 of seven), each
-// weight summed exactly as on the device.
+// base-256 digits and digit products (p + q < 4 of four digits, p + q < 8 of eight), each
+// weight summed exactly as on the device, and the same blocks refused by eight digits.
 static uint64_t g_split = 0, g_pack = 0;
 // Test controls: every eligible FP64 contraction in the digit form, and the n-th digit
 // contraction from now (0: the next) recording an expired wait.
 static int g_force_digits = 0, g_fail_in = -1;
+static uint64_t g_refused = 0;
 extern "C" void emu_force_digits(int on) { g_force_digits = on; }
 extern "C" void emu_fail_split_in(int n) { g_fail_in = n; }
 extern "C" uint64_t emu_split_count() { return g_split; }
-bool digits7_pays(const Contraction& c) {
+bool digits8_pays(const Contraction& c, bool) {
   return g_force_digits && c.batch == 1 && c.M >= 64 && c.N >= 64 && c.K >= 64;
 }
 uint64_t split_launch_count() { return g_split; }
 uint64_t split_pack_launch_count() { return g_pack; }
 size_t gemm_split_scratch_bytes(const Contraction& g) { return size_t(g.digits) * (g.M + g.N) * g.K; }
 
-void gemm_split(const Contraction& g, cudaStream_t, SplitScratch& ws) {
+extern "C" uint64_t emu_refused_count() { return g_refused; }
+
+// The profiles of split_gemm.cuh: rows [R][K] -> [ceil(R / 64)][K].
+static std::vector<float> profile(const std::vector<std::vector<double>>& rows, int64_t K) {
+  const int64_t R = rows.size(), nI = (R + 63) / 64;
+  std::vector<float> p(nI * K);
+  for (int64_t I = 0; I < nI; ++I) {
+    std::vector<double> least(K, 1.0);
+    bool odd = false;
+    for (int64_t g0 = 64 * I; g0 < std::min(R, 64 * I + 64); g0 += 8) {
+      std::vector<double> sum(K, 0.0);
+      int live = 0;
+      for (int64_t r = g0; r < std::min(R, g0 + 8); ++r) {
+        double m = 0.0;
+        bool finite = true;
+        for (double v : rows[r]) {
+          finite = finite && std::isfinite(v);
+          m = std::max(m, std::fabs(v));
+        }
+        if (!finite) { odd = true; continue; }
+        if (m == 0.0) continue;
+        int e;
+        std::frexp(m, &e);
+        odd = odd || std::abs(e) > kSplitMaxExponent;
+        ++live;
+        for (int64_t k = 0; k < K; ++k) sum[k] += std::ldexp(std::fabs(rows[r][k]), -e);
+      }
+      for (int64_t k = 0; live && k < K; ++k) least[k] = std::min(least[k], sum[k] / live);
+    }
+    for (int64_t k = 0; k < K; ++k) p[I * K + k] = odd ? NAN : static_cast<float>(least[k]);
+  }
+  return p;
+}
+// The blocks that eight digits refuse.
+static std::vector<unsigned char> refused(const std::vector<std::vector<double>>& A,
+                                          const std::vector<std::vector<double>>& B, int64_t K) {
+  const std::vector<float> a = profile(A, K), b = profile(B, K);
+  const int64_t nI = a.size() / K, nJ = b.size() / K;
+  std::vector<unsigned char> map(nI * nJ);
+  for (int64_t I = 0; I < nI; ++I)
+    for (int64_t J = 0; J < nJ; ++J) {
+      double v = 0.0;
+      for (int64_t k = 0; k < K; ++k) v += double(a[I * K + k]) * b[J * K + k];
+      map[I * nJ + J] = !(v >= split_profile_least(K));
+    }
+  return map;
+}
+
+void gemm_split(const Contraction& g, cudaStream_t s, SplitScratch& ws) {
   ++g_split;
   if (g_fail_in >= 0 && g_fail_in-- == 0) {
     *ws.error = 1;
@@ -91,7 +141,7 @@ void gemm_split(const Contraction& g, cudaStream_t, SplitScratch& ws) {
   Ax Bk = ax(Ki, g.B.s_ro, g.B.s_ri), Bn = ax(Ni, g.B.s_co, g.B.s_ci);
   Ax Cm = ax(Mi, g.C.s_ro, g.C.s_ri), Cn = ax(Ni, g.C.s_co, g.C.s_ci);
   Ax C2m = ax(Mi, g.C2.s_ro, g.C2.s_ri), C2n = ax(Ni, g.C2.s_co, g.C2.s_ci);
-  const int D = g.digits == 7 ? 7 : 4, NG = D == 7 ? 8 : 4;
+  const int D = g.digits == 8 ? 8 : 4, NG = D;
   using Digits = std::vector<std::vector<double>>;  // [digit][k]
   auto split = [&](const std::vector<double>& x, Digits& s, int& e) {
     double m = 0.0;
@@ -111,17 +161,20 @@ void gemm_split(const Contraction& g, cudaStream_t, SplitScratch& ws) {
   };
   std::vector<Digits> as(g.M), bs(g.N);
   std::vector<int> ea(g.M), eb(g.N);
-  std::vector<double> row(g.K);
+  std::vector<std::vector<double>> Ar(g.M, std::vector<double>(g.K)), Br(g.N, Ar[0]);
   for (int64_t m = 0; m < g.M; ++m) {
-    for (int64_t k = 0; k < g.K; ++k) row[k] = g.A.p[Am.off(m) + Ak.off(k)];
-    split(row, as[m], ea[m]);
+    for (int64_t k = 0; k < g.K; ++k) Ar[m][k] = g.A.p[Am.off(m) + Ak.off(k)];
+    split(Ar[m], as[m], ea[m]);
   }
   for (int64_t n = 0; n < g.N; ++n) {
-    for (int64_t k = 0; k < g.K; ++k) row[k] = g.B.p[Bk.off(k) + Bn.off(n)];
-    split(row, bs[n], eb[n]);
+    for (int64_t k = 0; k < g.K; ++k) Br[n][k] = g.B.p[Bk.off(k) + Bn.off(n)];
+    split(Br[n], bs[n], eb[n]);
   }
+  std::vector<unsigned char> map((g.M + 63) / 64 * ((g.N + 63) / 64), 0);
+  if (D == 8) map = refused(Ar, Br, g.K);
   for (int64_t m = 0; m < g.M; ++m)
     for (int64_t n = 0; n < g.N; ++n) {
+      if (map[(m / 64) * ((g.N + 63) / 64) + n / 64]) continue;
       double sum = 0.0;
       for (int w = NG - 1; w >= 0; --w) {  // smallest weight first
         double grp = 0.0;
@@ -140,27 +193,46 @@ void gemm_split(const Contraction& g, cudaStream_t, SplitScratch& ws) {
         *c2 = g.beta != 0.0 ? v + g.beta * *c2 : v;
       }
     }
+  if (std::count(map.begin(), map.end(), 0) < static_cast<int64_t>(map.size())) {
+    ++g_refused;
+    Contraction h = g;
+    h.only = map.data();
+    h.only_ld = (g.N + 63) / 64;
+    gemm(h, s, ws.fp64);
+  }
 }
 
-// The complex form: the emulation runs the four real contractions it stands for.
+// The complex form: two real contractions over the planes side by side along k.
 size_t gemm_split_complex_scratch_bytes(const Contraction& g) { return 4 * gemm_split_scratch_bytes(g); }
 void gemm_split_complex(const Contraction& g, int64_t a_im, int64_t b_im, int64_t c_im, bool conjA,
                         bool conjB, cudaStream_t s, SplitScratch& ws) {
   const double sA = conjA ? -1.0 : 1.0, sB = conjB ? -1.0 : 1.0;
-  for (int part = 0; part < 2; ++part)
-    for (int term = 0; term < 2; ++term) {
-      Contraction c = g;
-      const bool ai = term == 1, bi = part == 0 ? term == 1 : term == 0;
-      if (ai) c.A.p += a_im;
-      if (bi) c.B.p += b_im;
-      if (part) {
-        c.C.p += c_im;
-        if (c.C2.p) c.C2.p += c_im;
-      }
-      c.alpha = g.alpha * (part == 0 ? (term ? -sA * sB : 1.0) : (term ? sA : sB));
-      if (term) c.beta = 1.0;
-      gemm_split(c, s, ws);
+  const int64_t Mi = g.Mi > 0 ? g.Mi : g.M, Ni = g.Ni > 0 ? g.Ni : g.N, K = g.K;
+  const int64_t Ki = g.Ki > 0 ? g.Ki : std::max<int64_t>(K, 1);
+  const Ax Am = ax(Mi, g.A.s_ro, g.A.s_ri), Ak = ax(Ki, g.A.s_co, g.A.s_ci);
+  const Ax Bk = ax(Ki, g.B.s_ro, g.B.s_ri), Bn = ax(Ni, g.B.s_co, g.B.s_ci);
+  for (int part = 0; part < 2; ++part) {  // [Ar | Ai] on [Br ; -sA sB Bi] or [sB Bi ; sA Br]
+    std::vector<double> A(g.M * 2 * K), B(2 * K * g.N);
+    for (int64_t m = 0; m < g.M; ++m)
+      for (int64_t k = 0; k < K; ++k)
+        for (int h = 0; h < 2; ++h)
+          A[m * 2 * K + h * K + k] = g.A.p[Am.off(m) + Ak.off(k) + h * a_im];
+    for (int64_t n = 0; n < g.N; ++n)
+      for (int64_t k = 0; k < K; ++k)
+        for (int h = 0; h < 2; ++h) {
+          const double w = part == 0 ? (h ? -sA * sB : 1.0) : (h ? sA : sB);
+          B[n * 2 * K + h * K + k] = w * g.B.p[Bk.off(k) + Bn.off(n) + (h != part ? b_im : 0)];
+        }
+    Contraction c = g;
+    c.K = 2 * K; c.Ki = 0;
+    c.A.p = A.data(); c.A.s_ro = Mi * 2 * K; c.A.s_ri = 2 * K; c.A.s_co = 0; c.A.s_ci = 1;
+    c.B.p = B.data(); c.B.s_ro = 0; c.B.s_ri = 1; c.B.s_co = Ni * 2 * K; c.B.s_ci = 2 * K;
+    if (part) {
+      c.C.p += c_im;
+      if (c.C2.p) c.C2.p += c_im;
     }
+    gemm_split(c, s, ws);
+  }
 }
 
 // Pre-packed B: the emulation keeps a dense copy B[n][k] of the operand's values
@@ -207,6 +279,18 @@ SplitOperand split_pack_operand(const double* src, int64_t R, int64_t Ri, int64_
   o.slices = dst; o.R = R; o.K = K; o.Rp = R; o.Kp = K; o.digits = digits;
   g_pack += 2;
   return o;
+}
+
+void split_refused(const SplitOperand& A, const SplitOperand& B, int* word, cudaStream_t) {
+  auto rows = [](const SplitOperand& o) {
+    const double* d = static_cast<const double*>(o.slices);
+    std::vector<std::vector<double>> r;
+    for (int64_t i = 0; i < o.R; ++i) r.emplace_back(d + i * o.K, d + (i + 1) * o.K);
+    return r;
+  };
+  const std::vector<unsigned char> map = refused(rows(A), rows(B), A.K);
+  std::memset(word, 0, 8);
+  *word = std::count(map.begin(), map.end(), 0) < static_cast<int64_t>(map.size());
 }
 
 void gemm_split_prepacked(const Contraction& g, const SplitOperand& A, const SplitRuns& ar,
@@ -859,3 +943,17 @@ void triples_cr_sums(const double* S, const double* S_im, const double* t1, cons
 
 }  // namespace ops
 }  // namespace cc4s_b200
+
+// Test-only entry: C = A B of row-major host operands in a digit form (0: the plain chain).
+extern "C" void emu_gemm_split(const double* A, const double* B, double* C, int64_t M, int64_t N,
+                               int64_t K, int digits) {
+  using namespace cc4s_b200;
+  Contraction c;
+  c.M = M; c.N = N; c.K = K; c.digits = digits;
+  c.A = rm(const_cast<double*>(A), K);
+  c.B = rm(const_cast<double*>(B), N);
+  c.C = rm(C, N);
+  SplitScratch ws;
+  if (digits) gemm_split(c, nullptr, ws);
+  else gemm(c, nullptr, ws.fp64);
+}

@@ -119,3 +119,118 @@ def test_expired_wait_while_the_integrals_are_built(emu):
     with pytest.raises(CoupledClusterError) as e:
         _solver(emu)
     assert e.value.status == TIMEOUT
+
+
+def _product(emu, A, B, digits):
+    M, K = A.shape
+    C = np.zeros((M, B.shape[1]))
+    P = ctypes.POINTER(ctypes.c_double)
+    A, B = np.ascontiguousarray(A), np.ascontiguousarray(B)
+    emu.emu_gemm_split(A.ctypes.data_as(P), B.ctypes.data_as(P), C.ctypes.data_as(P),
+                       ctypes.c_int64(M), ctypes.c_int64(C.shape[1]), ctypes.c_int64(K), digits)
+    return C
+
+
+def _graded(kind, rng, M, N, K):
+    """Operands that the eight-digit form (62 bits below the largest element of a row) must
+    not lose against FP64, and some on which it holds anyway."""
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    name, _, x = kind.partition(" ")
+    x = float(x or 0)
+    if name == "opposed":    # A falls along k, B rises
+        w = x ** (-np.arange(K) / (K - 1))
+        A, B = A * w, B * w[::-1, None]
+    elif name == "alike":    # both fall
+        w = x ** (-np.arange(K) / (K - 1))
+        A, B = A * w, B * w[:, None]
+    elif name == "rows":     # eight rows of A against a rising B, the others even
+        w = x ** (-np.arange(K) / (K - 1))
+        A[16:24] *= w
+        B = B * w[::-1, None]
+    elif name == "blocks":   # the large elements of either meet tiny ones of the other
+        q = K // 4
+        A *= x
+        B *= x
+        A[:, :q], B[:q] = rng.uniform(.5, 1, (M, q)), 1e-13
+        A[:, -q:], B[-q:] = 1e-13, rng.uniform(.5, 1, (q, N))
+    elif name == "spike":    # one element per column far above the others
+        B[rng.integers(K, size=N), np.arange(N)] = x
+    elif name == "scaled":   # rows of very different magnitude, which a row scale absorbs
+        A *= x ** rng.uniform(-1, 1, (M, 1))
+    elif name == "extreme":  # beyond the exponents that the scaling is used for
+        A[5] *= x
+    elif name == "zeros":
+        A[3], B[:, 7] = 0.0, 0.0
+        A[rng.random(A.shape) < 0.5] = 0.0
+    return A, B
+
+
+@pytest.mark.parametrize("kind,refuses", [
+    ("even", False), ("opposed 30", False), ("opposed 1e3", True), ("opposed 1e6", True),
+    ("opposed 1e12", True), ("alike 1e8", False), ("rows 1e8", True), ("blocks 1e-3", True),
+    ("spike 100", False), ("scaled 1e30", False), ("extreme 1e-150", True), ("zeros", False)])
+@pytest.mark.parametrize("shape", [(64, 64, 64), (96, 130, 256)])
+def test_eight_digits_are_no_less_precise_than_fp64(emu, kind, refuses, shape):
+    """Against 80-bit sums: the error relative to sum |a b| of each output and the 2-norm of
+    all errors stay within what the plain FP64 chain shows on the same operands (1.25 times
+    its largest, and not below one rounding of the result)."""
+    rng = np.random.default_rng(11)
+    A, B = _graded(kind, rng, *shape)
+    Al = A.astype(np.longdouble)
+    ref, total = Al @ B.astype(np.longdouble), np.abs(Al) @ np.abs(B)
+    before = emu.emu_refused_count()
+    eight, chain = _product(emu, A, B, 8), _product(emu, A, B, 0)
+    assert (emu.emu_refused_count() > before) == refuses
+
+    def worst(C):
+        return float((np.abs(C - ref) / np.where(total > 0, total, 1)).max())
+
+    def norm(C):
+        return float(np.linalg.norm(((C - ref) / np.where(total > 0, total, 1)).astype(float)))
+    u = 2.0 ** -53
+    assert worst(eight) <= max(1.25 * worst(chain), u)
+    assert norm(eight) <= max(1.1 * norm(chain), u)
+
+
+def test_eight_digits_keep_non_finite_elements_to_their_outputs(emu):
+    """An Inf or NaN shows where the FP64 chain shows it, and nowhere else."""
+    rng = np.random.default_rng(2)
+    A, B = rng.standard_normal((70, 64)), rng.standard_normal((64, 66))
+    A[3, 5], A[40, 7], B[9, 2] = np.inf, np.nan, -np.inf
+    B[5, 60] = 0.0
+    eight, chain = _product(emu, A, B, 8), _product(emu, A, B, 0)
+    np.testing.assert_array_equal(np.isnan(eight), np.isnan(chain))
+    np.testing.assert_array_equal(np.isinf(eight), np.isinf(chain))
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("slice_size", [0, 8])
+def test_residual_in_eight_digits_matches_oracle(emu, cplx, slice_size):
+    """Every eligible contraction of the FP64 residual in the digit form (ladder with its
+    shared X panel, planar complex contractions of both kinds): within rounding of the
+    oracle's, and different from the FP64 pipe's (the digit form really ran)."""
+    from oracle import ccsd
+    rng = np.random.default_rng(5)
+    n = NO + NV
+    if cplx:
+        g = rng.standard_normal((NG, n, n)) + 1j * rng.standard_normal((NG, n, n))
+        g = 0.1 * (g + g.conj().transpose(0, 2, 1))
+    else:
+        g = rng.standard_normal((NG, n, n)) * 0.1
+        g = g + g.transpose(0, 2, 1)
+    s = inputs.System(np.sort(rng.uniform(-1.5, -.5, NO)), np.sort(rng.uniform(.2, 3, NV)), g,
+                      half_grid=not cplx)
+    T = _amplitudes(cplx)
+    out = []
+    for forced in (1, 0):
+        from cc4s_b200 import Solver
+        emu.emu_force_digits(forced)
+        sol = Solver({"integralsSliceSize": slice_size} if slice_size else {}, lib=emu._name)
+        sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=not cplx)
+        out.append(sol.residual(T))
+        sol.close()
+    kw = dict(slice_size=slice_size) if slice_size and cplx else {}
+    Q = ccsd.residuum(T, ccsd.CcsdInputs(s), **kw)
+    for q in range(2):
+        assert np.abs(out[0][q] - Q[q]).max() < 1e-13 * np.abs(Q[q]).max()
+    assert np.abs(out[0][1] - out[1][1]).max() > 0.0

@@ -1,7 +1,8 @@
-"""The digit-form contraction kernels (four digits: split precision, seven: FP64) at the
+"""The digit-form contraction kernels (four digits: split precision, eight: FP64) at the
 edges of their tiles (128 x 128 and 128 x 64), of the K step of 32 and of the K blocks of
-64, beyond one S32 accumulation span (K > 16384), and with a non-finite input, against
-128-bit dot products with a derived bound (tests/kernels/digits_check.cu)."""
+64, beyond one S32 accumulation span (K > 16384), on rows graded along k and with a
+non-finite input, against 128-bit dot products with a derived bound, relative to
+sum |a b| where the form stands for FP64 (tests/kernels/digits_check.cu)."""
 import os
 import subprocess
 import sys
@@ -21,4 +22,4 @@ def test_digit_forms(shape):
     r = subprocess.run([exe] + [str(x) for x in shape], capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
-    assert r.stdout.count("errflag=0") == 8
+    assert r.stdout.count("errflag=0") == 12
