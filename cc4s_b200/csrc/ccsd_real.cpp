@@ -510,7 +510,7 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
   // by all block pairs: B depends on N = o^2, K = c_n v and the X view only) is
   // sliced once per c range into a region kept beside the per-contraction scratch.
   const Contraction c_first = contraction(0, std::min(s, v), 0, std::min(s, v), 0, std::min(cn, v));
-  const bool prepack = !taping_ && c_first.digits && split_single_panel(c_first) && nb > 1;
+  bool prepack = !taping_ && c_first.digits && split_single_panel(c_first) && nb > 1;
   if (prepack) {
     size_t regular = 0;
     for (int64_t c0 = 0; c0 < v; c0 += cn) {
@@ -526,7 +526,9 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
         }
       }
     }
-    split_reserve(regular, split_packed_b_bytes(c_first));
+    const size_t extra = split_packed_b_bytes(c_first);
+    if (c_first.digits == 8) prepack = split_room(regular, extra);
+    else split_reserve(regular, extra);
   }
   for (int64_t c0 = 0; c0 < v; c0 += cn) {
     const int64_t nc = std::min(cn, v - c0);

@@ -71,29 +71,51 @@ void Schedule::split_reserve(size_t regular, size_t extra) {
   if (regular <= split_.bytes && extra <= split_extra_bytes_) return;
   regular = std::max(regular, split_.bytes);
   extra = std::max(extra, split_extra_bytes_);
-  ops::sync(s_);
-  if (split_mem_) ops::release(split_mem_);
-  split_mem_ = nullptr;
-  split_.p = nullptr;  // nothing is left if the allocation fails
-  split_.bytes = 0;
-  split_extra_ = nullptr;
-  split_extra_bytes_ = 0;
   error_word();
-  // Allocations start on a 256-byte boundary, so every TMA row request of the contraction
-  // kernel begins on a sector and line boundary (a 16-byte offset made each 64-byte row
-  // touch three sectors).
-  split_mem_ = ops::alloc((regular + extra) / 8);
-  split_.p = split_mem_;
-  split_.bytes = regular;
-  if (extra) {
-    split_extra_ = static_cast<unsigned char*>(split_.p) + regular;
-    split_extra_bytes_ = extra;
+  ops::sync(s_);
+  const size_t had = split_.bytes, had_extra = split_extra_bytes_;
+  auto make = [&](size_t r, size_t x) {
+    if (split_mem_) ops::release(split_mem_);
+    split_mem_ = nullptr;
+    split_.p = nullptr;
+    split_.bytes = 0;
+    split_extra_ = nullptr;
+    split_extra_bytes_ = 0;
+    if (r + x == 0) return;
+    // Allocations start on a 256-byte boundary, so every TMA row request of the contraction
+    // kernel begins on a sector and line boundary (a 16-byte offset made each 64-byte row
+    // touch three sectors).
+    split_mem_ = ops::alloc((r + x) / 8);
+    split_.p = split_mem_;
+    split_.bytes = r;
+    if (x) {
+      split_extra_ = static_cast<unsigned char*>(split_.p) + r;
+      split_extra_bytes_ = x;
+    }
+  };
+  try {
+    make(regular, extra);
+  } catch (const Error&) {
+    split_failed_ = regular + extra;
+    make(had, had_extra);  // what was there fits again
+    throw;
   }
 }
 
-SplitScratch& Schedule::split_ws() {
-  split_.fp64 = scratch_;
-  return split_;
+// Room for a contraction of the FP64 digit form, which has the FP64 tensor pipe to fall back
+// on: false where the device has none.  A size that did not fit is not tried again within
+// one call (an attempt waits for the stream and for the allocator).
+bool Schedule::split_room(size_t regular, size_t extra) {
+  if (regular <= split_.bytes && extra <= split_extra_bytes_) return true;
+  const size_t total = std::max(regular, split_.bytes) + std::max(extra, split_extra_bytes_);
+  if (split_failed_ && total >= split_failed_) return false;
+  try {
+    split_reserve(regular, extra);
+  } catch (const Error& e) {
+    if (e.status != ERR_OUT_OF_MEMORY) throw;
+    return false;
+  }
+  return true;
 }
 
 // The word in which a kernel records an expired wait: in memory of its own, so that it
@@ -103,6 +125,11 @@ void Schedule::error_word() {
   split_error_ = ops::alloc(2);
   ops::zero(split_error_, 2, s_);
   split_.error = reinterpret_cast<int*>(split_error_);
+}
+
+SplitScratch& Schedule::split_ws() {
+  split_.fp64 = scratch_;
+  return split_;
 }
 
 void Schedule::split_exec(const Contraction& c) {
@@ -117,15 +144,7 @@ void Schedule::fp64_exec(const Contraction& c) {
   if (digits_for(c, false) == 8) {
     Contraction d = c;
     d.digits = 8;
-    bool fits = true;
-    try {
-      const size_t need = gemm_split_scratch_bytes(d);
-      if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
-    } catch (const Error& e) {
-      if (e.status != ERR_OUT_OF_MEMORY) throw;
-      fits = false;  // no room for the digits: the FP64 tensor pipe needs none
-    }
-    if (fits) {
+    if (split_room(gemm_split_scratch_bytes(d), split_extra_bytes_)) {
       gemm_split(d, s_, split_ws());
       return;
     }
@@ -212,12 +231,11 @@ bool Schedule::zgemm_split(const Contraction& c, int64_t a_im, int64_t b_im, int
   Contraction d = c;
   d.digits = digits_for(c, big, true);
   if (!d.digits) return false;
-  try {
-    const size_t need = gemm_split_complex_scratch_bytes(d);
-    if (need > split_.bytes) split_reserve(need, split_extra_bytes_);
-  } catch (const Error& e) {
-    if (e.status != ERR_OUT_OF_MEMORY || d.digits != 8) throw;
-    return false;
+  const size_t need = gemm_split_complex_scratch_bytes(d);
+  if (d.digits == 8) {
+    if (!split_room(need, split_extra_bytes_)) return false;
+  } else if (need > split_.bytes) {
+    split_reserve(need, split_extra_bytes_);
   }
   const double f = 8.0 * double(c.M) * double(c.N) * double(c.K);
   if (count_flops_) flops_ += f;
@@ -534,6 +552,7 @@ int Schedule::device_error() {
 }
 
 void Schedule::check_device() {
+  split_failed_ = 0;  // the next call may find more room
   if (device_error()) throw Error(ERR_TIMEOUT, "a tensor-core kernel gave up a bounded wait");
 }
 

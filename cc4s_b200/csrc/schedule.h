@@ -161,8 +161,10 @@ class Schedule {
   // Makes the split scratch hold `regular` bytes for per-contraction packing plus a
   // second region of `extra` bytes (split_extra_) that survives those calls; may
   // reallocate (synchronises).  A later split_exec that needs more than `regular`
-  // reallocates with an extra region of the same size (its contents are lost).
+  // reallocates with an extra region of the same size (its contents are lost).  Without
+  // room the scratch keeps its sizes.
   void split_reserve(size_t regular, size_t extra);
+  bool split_room(size_t regular, size_t extra);
   void error_word();
   SplitScratch& split_ws();  // split_ with the partial-sum scratch of the FP64 pipe
   // One split contraction whose B was sliced by split_pack_b (recorded like tc_).
@@ -205,6 +207,7 @@ class Schedule {
   double* split_error_ = nullptr;
   void* split_extra_ = nullptr;
   size_t split_extra_bytes_ = 0;
+  size_t split_failed_ = 0;  // bytes that the device had no room for in this call
   // vertex description for the adjoint (set by each schedule)
   int64_t so_ = 0, sv_ = 0, sG_ = 0;
   bool scplx_ = false;

@@ -355,7 +355,17 @@ int energy_noalloc(const double* T1, const double* T2, const double* V, int64_t 
 
 namespace ops {
 
+// Test control: allocations of more than this many bytes find no memory (0: no limit).
+static size_t g_alloc_limit = 0;
+static uint64_t g_alloc_failures = 0;
+extern "C" void emu_alloc_limit(size_t bytes) { g_alloc_limit = bytes; }
+extern "C" uint64_t emu_alloc_failures() { return g_alloc_failures; }
+
 double* alloc(size_t elems) {
+  if (g_alloc_limit && elems * sizeof(double) > g_alloc_limit) {
+    ++g_alloc_failures;
+    throw Error(ERR_OUT_OF_MEMORY, "out of memory (test limit)");
+  }
   void* p = std::calloc(elems ? elems : 1, sizeof(double));
   if (!p) throw Error(ERR_OUT_OF_MEMORY, "host allocation failed");
   return static_cast<double*>(p);

@@ -234,3 +234,37 @@ def test_residual_in_eight_digits_matches_oracle(emu, cplx, slice_size):
     for q in range(2):
         assert np.abs(out[0][q] - Q[q]).max() < 1e-13 * np.abs(Q[q]).max()
     assert np.abs(out[0][1] - out[1][1]).max() > 0.0
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_fp64_runs_without_room_for_the_digits(emu, cplx):
+    """FP64 needs no digit scratch: where the device has no room for some of it (the ladder's
+    shared X panel with its per-contraction part, the larger contractions), the residual is
+    the oracle's all the same, what fits still runs in digits, and a size that did not fit is
+    not tried for again by every contraction of the call."""
+    from oracle import ccsd
+    o, v, G = 8, 24, 64
+    s = inputs.synthetic_system(o, v, G, complex=cplx, seed=3)
+    rng = np.random.default_rng(5)
+    T1 = rng.standard_normal((v, o)) * 0.02
+    T2 = rng.standard_normal((v, v, o, o)) * 0.02
+    T2 = T2 + T2.transpose(1, 0, 3, 2)
+    from cc4s_b200 import Solver
+    # the ladder's block size only trades memory for speed on the real path
+    sol = Solver({} if cplx else {"integralsSliceSize": 8}, lib=emu._name)
+    sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=not cplx)
+    emu.emu_alloc_failures.restype = ctypes.c_uint64
+    # above the amplitude vectors (n1^2 = 36864 values per plane), below the largest scratch
+    emu.emu_alloc_limit(ctypes.c_size_t(40000 * 8 * (2 if cplx else 1)))
+    try:
+        for _ in range(2):
+            f0, c0 = emu.emu_alloc_failures(), emu.emu_split_count()
+            R = sol.residual((T1, T2))
+            assert 1 <= emu.emu_alloc_failures() - f0 <= 4
+            assert emu.emu_split_count() > c0
+    finally:
+        emu.emu_alloc_limit(ctypes.c_size_t(0))
+        sol.close()
+    Q = ccsd.residuum((T1, T2), ccsd.CcsdInputs(s))
+    for q in range(2):
+        assert np.abs(R[q] - Q[q]).max() < 1e-13 * np.abs(Q[q]).max()
