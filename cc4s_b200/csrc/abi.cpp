@@ -315,7 +315,29 @@ void Handle::scatter_vertex_bar(const Schedule::VertexBar& vb, double* out) {
   struct Block { const double* d; int64_t row0, nx, col0, ny; };
   const Block blocks[4] = {{vb.Gpp, o, v, o, v}, {vb.Gph, o, v, 0, o}, {vb.Ghh, 0, o, 0, o},
                            {vb.Ghp, 0, o, o, v}};
-  double* dev = ops::alloc(total);
+  double* dev = nullptr;
+  try {
+    dev = ops::alloc(total);
+  } catch (const Error& e) {
+    if (e.status != ERR_OUT_OF_MEMORY) throw;
+  }
+  if (!dev) {  // no room for the whole vertex on the device: block by block on the host
+    std::memset(out, 0, sizeof(double) * total);
+    std::vector<double> h;
+    for (const Block& b : blocks) {
+      if (!b.d) continue;
+      h.resize(parts * NG * b.nx * b.ny);
+      ops::d2h(h.data(), b.d, h.size(), stream);
+      ops::sync(stream);
+      for (int64_t part = 0; part < parts; ++part)
+        for (int64_t x = 0; x < b.nx; ++x)
+          for (int64_t y = 0; y < b.ny; ++y)
+            for (int64_t k = 0; k < NG; ++k)
+              out[(k + NG * ((b.row0 + x) + Np * (b.col0 + y))) * es + part] =
+                  h[((part * NG + k) * b.nx + x) * b.ny + y];
+    }
+    return;
+  }
   try {
     ops::zero(dev, total, stream);
     for (const Block& b : blocks)

@@ -268,3 +268,27 @@ def test_fp64_runs_without_room_for_the_digits(emu, cplx):
     Q = ccsd.residuum((T1, T2), ccsd.CcsdInputs(s))
     for q in range(2):
         assert np.abs(R[q] - Q[q]).max() < 1e-13 * np.abs(Q[q]).max()
+
+
+@pytest.mark.parametrize("kind", ["real", "stacked", "complex"])
+def test_vertex_adjoint_without_room_for_a_device_copy(emu, kind):
+    """The vertex adjoint is put together on the host, with the same values, where the device
+    has no room for a copy of the whole vertex."""
+    emu.emu_force_digits(0)
+    from cc4s_b200 import Solver
+    s = _system(cplx=kind != "real")
+    sol = Solver({}, lib=emu._name)
+    sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=kind != "complex")
+    args = (_amplitudes(kind == "complex"), _amplitudes(kind == "complex", seed=4))
+    _, ref = sol.residual_vjp(*args)
+    emu.emu_alloc_failures.restype = ctypes.c_uint64
+    f0 = emu.emu_alloc_failures()
+    planes = 1 if kind == "real" else 2   # above every block, below the whole vertex
+    emu.emu_alloc_limit(ctypes.c_size_t(8 * planes * NG * (NV * NV + (NO + NV) ** 2) // 2))
+    try:
+        _, g = sol.residual_vjp(*args)
+    finally:
+        emu.emu_alloc_limit(ctypes.c_size_t(0))
+        sol.close()
+    assert emu.emu_alloc_failures() == f0 + 1
+    np.testing.assert_array_equal(g, ref)
