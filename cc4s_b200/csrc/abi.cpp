@@ -293,8 +293,17 @@ Schedule* Handle::adjoint_schedule() {
     ro.ppl = opt.ppl != 0;
     ro.slab = opt.integrals_slice_size;
     ro.adjoint = true;
-    if (complex_path) adj.reset(new CcsdComplex(csys, ro, stream));
-    else adj.reset(new CcsdReal(sys, ro, stream));
+    auto build = [&] {
+      if (complex_path) adj.reset(new CcsdComplex(csys, ro, stream));
+      else adj.reset(new CcsdReal(sys, ro, stream));
+    };
+    try {
+      build();
+    } catch (const Error& e) {
+      if (e.status != ERR_OUT_OF_MEMORY) throw;
+      ro.compact = true;
+      build();
+    }
   }
   // the handle's precision: the split form runs the recorded residual and the
   // large contractions of every reverse sweep on the tensor cores

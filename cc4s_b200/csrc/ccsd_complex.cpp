@@ -70,11 +70,13 @@ CcsdComplex::CcsdComplex(const ComplexSystem& sys, const RealOptions& opt, Strea
     // The off-diagonal slices of one a slice are contracted together, slab_group_ of them at
     // a time (2^26 complex values, 1 GiB): the same terms, and s^2 = o^2 rows per
     // contraction become s^2 slab_group_ (one 256 x 256 output of K = 25600 at
-    // o = 16, v = 160 filled 4 of 148 SMs).
+    // o = 16, v = 160 filled 4 of 148 SMs).  Not where the caller bounds the slab by
+    // integralsSliceSize, nor where the device has no room for it.
     const int64_t slice = slab_rows_ * slab_rows_ * slab_cols_ * v;
-    slab_group_ = std::max<int64_t>(
-        1, std::min<int64_t>((v + slab_rows_ - 1) / slab_rows_ - 1,
-                             std::min(budget, int64_t(1) << 26) / slice));
+    if (opt.slab <= 0 && !opt.compact)
+      slab_group_ = std::max<int64_t>(
+          1, std::min<int64_t>((v + slab_rows_ - 1) / slab_rows_ - 1,
+                               std::min(budget, int64_t(1) << 26) / slice));
     if (opt.ppl) slab_ = z(slab_group_ * slice);
   } catch (...) {
     release_all();

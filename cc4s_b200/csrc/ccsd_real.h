@@ -10,6 +10,7 @@ struct RealOptions {
   bool adjoint = false;     // reverse mode (separate buffers for every recorded value)
   bool ppl = true;          // particle-particle ladder from vertex slabs
   int64_t slab = 0;         // PPL block size in virtual orbitals (0: automatic)
+  bool compact = false;     // no buffers beyond what the formulation needs
 };
 
 // Device-resident inputs of the real path.  G counts stacked real rows: the

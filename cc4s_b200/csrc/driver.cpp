@@ -140,11 +140,23 @@ void Handle::set_inputs(const double* eps_h, int64_t No, const double* eps_p, in
     throw;
   }
   ops::release(staging);
-  allocate_state();
+  try {
+    allocate_state(false);
+  } catch (const Error& e) {
+    free_state();
+    if (e.status != ERR_OUT_OF_MEMORY) throw;
+    try {
+      allocate_state(true);
+    } catch (...) {
+      free_state();
+      throw;
+    }
+  }
 }
 
-void Handle::allocate_state() {
+void Handle::allocate_state(bool compact) {
   RealOptions ro;
+  ro.compact = compact;
   ro.ccd = opt.method == CC4S_METHOD_CCD;
   ro.ppl = opt.ppl != 0;
   // integralsSliceSize sets the ladder block size.  Real path: the ladder is
@@ -183,12 +195,7 @@ void Handle::allocate_state() {
   status_dev = reinterpret_cast<int*>(take(4));
   reset_mixer();
   ops::sync(stream);
-  try {
-    solver->check_device();  // the integrals were built above
-  } catch (...) {
-    free_state();
-    throw;
-  }
+  solver->check_device();  // the integrals were built above
 }
 
 void Handle::reset_mixer() {

@@ -29,7 +29,7 @@ struct Handle {
   // helpers
   double* take(size_t elems);
   void free_state();
-  void allocate_state();
+  void allocate_state(bool compact);
   void reset_mixer();
   void require_inputs() const;
   // Layout change between the caller's column-major T1/T2 and the device

@@ -355,22 +355,42 @@ int energy_noalloc(const double* T1, const double* T2, const double* V, int64_t 
 
 namespace ops {
 
-// Test control: allocations of more than this many bytes find no memory (0: no limit).
-static size_t g_alloc_limit = 0;
+// Test controls: single allocations of more than `bytes`, or all live ones together beyond
+// `total`, find no memory (0: no limit).
+static size_t g_alloc_limit = 0, g_total_limit = 0, g_live = 0, g_peak = 0;
 static uint64_t g_alloc_failures = 0;
-extern "C" void emu_alloc_limit(size_t bytes) { g_alloc_limit = bytes; }
-extern "C" uint64_t emu_alloc_failures() { return g_alloc_failures; }
-
-double* alloc(size_t elems) {
-  if (g_alloc_limit && elems * sizeof(double) > g_alloc_limit) {
-    ++g_alloc_failures;
-    throw Error(ERR_OUT_OF_MEMORY, "out of memory (test limit)");
-  }
-  void* p = std::calloc(elems ? elems : 1, sizeof(double));
-  if (!p) throw Error(ERR_OUT_OF_MEMORY, "host allocation failed");
-  return static_cast<double*>(p);
+extern "C" void emu_alloc_limit(size_t bytes, size_t total) {
+  g_alloc_limit = bytes;
+  g_total_limit = total;
 }
-void release(void* p) { std::free(p); }
+extern "C" uint64_t emu_alloc_failures() { return g_alloc_failures; }
+extern "C" size_t emu_live_bytes() { return g_live; }
+extern "C" size_t emu_peak_bytes(int reset) {
+  const size_t p = g_peak;
+  if (reset) g_peak = g_live;
+  return p;
+}
+
+double* alloc(size_t elems) {  // the size in a header of 64 bytes
+  const size_t bytes = std::max<size_t>(elems, 1) * sizeof(double);
+  void* p = nullptr;
+  if (!(g_alloc_limit && bytes > g_alloc_limit) && !(g_total_limit && g_live + bytes > g_total_limit))
+    p = std::calloc(bytes + 64, 1);
+  if (!p) {
+    ++g_alloc_failures;
+    throw Error(ERR_OUT_OF_MEMORY, "host allocation failed");
+  }
+  *static_cast<size_t*>(p) = bytes;
+  g_live += bytes;
+  g_peak = std::max(g_peak, g_live);
+  return static_cast<double*>(p) + 8;
+}
+void release(void* p) {
+  if (!p) return;
+  size_t* h = static_cast<size_t*>(p) - 8;
+  g_live -= *h;
+  std::free(h);
+}
 void zero(double* p, size_t n, Stream) { std::memset(p, 0, n * sizeof(double)); }
 void h2d(double* d, const double* s, size_t n, Stream) { std::memcpy(d, s, n * sizeof(double)); }
 void d2h(double* d, const double* s, size_t n, Stream) { std::memcpy(d, s, n * sizeof(double)); }

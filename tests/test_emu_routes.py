@@ -20,11 +20,16 @@ def emu():
     import build_emu
     from cc4s_b200 import _abi
     lib = _abi.load(build_emu.build())
-    lib.emu_split_count.restype = ctypes.c_uint64
+    lib.emu_split_count.restype = lib.emu_alloc_failures.restype = ctypes.c_uint64
+    lib.emu_live_bytes.restype = lib.emu_peak_bytes.restype = ctypes.c_size_t
     lib.emu_force_digits(1)
     yield lib
     lib.emu_force_digits(0)
     lib.emu_fail_split_in(-1)
+
+
+def _limit(lib, single=0, total=0):
+    lib.emu_alloc_limit(ctypes.c_size_t(single), ctypes.c_size_t(total))
 
 
 def _system(cplx=False, seed=7):
@@ -253,9 +258,8 @@ def test_fp64_runs_without_room_for_the_digits(emu, cplx):
     # the ladder's block size only trades memory for speed on the real path
     sol = Solver({} if cplx else {"integralsSliceSize": 8}, lib=emu._name)
     sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=not cplx)
-    emu.emu_alloc_failures.restype = ctypes.c_uint64
     # above the amplitude vectors (n1^2 = 36864 values per plane), below the largest scratch
-    emu.emu_alloc_limit(ctypes.c_size_t(40000 * 8 * (2 if cplx else 1)))
+    _limit(emu, 40000 * 8 * (2 if cplx else 1))
     try:
         for _ in range(2):
             f0, c0 = emu.emu_alloc_failures(), emu.emu_split_count()
@@ -263,7 +267,7 @@ def test_fp64_runs_without_room_for_the_digits(emu, cplx):
             assert 1 <= emu.emu_alloc_failures() - f0 <= 4
             assert emu.emu_split_count() > c0
     finally:
-        emu.emu_alloc_limit(ctypes.c_size_t(0))
+        _limit(emu)
         sol.close()
     Q = ccsd.residuum((T1, T2), ccsd.CcsdInputs(s))
     for q in range(2):
@@ -281,14 +285,49 @@ def test_vertex_adjoint_without_room_for_a_device_copy(emu, kind):
     sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=kind != "complex")
     args = (_amplitudes(kind == "complex"), _amplitudes(kind == "complex", seed=4))
     _, ref = sol.residual_vjp(*args)
-    emu.emu_alloc_failures.restype = ctypes.c_uint64
     f0 = emu.emu_alloc_failures()
     planes = 1 if kind == "real" else 2   # above every block, below the whole vertex
-    emu.emu_alloc_limit(ctypes.c_size_t(8 * planes * NG * (NV * NV + (NO + NV) ** 2) // 2))
+    _limit(emu, 8 * planes * NG * (NV * NV + (NO + NV) ** 2) // 2)
     try:
         _, g = sol.residual_vjp(*args)
     finally:
-        emu.emu_alloc_limit(ctypes.c_size_t(0))
+        _limit(emu)
         sol.close()
     assert emu.emu_alloc_failures() == f0 + 1
     np.testing.assert_array_equal(g, ref)
+
+
+def test_complex_ladder_slab_stays_within_the_caller_and_the_device(emu):
+    """The complex ladder contracts several slices together where it may: not where
+    integralsSliceSize bounds the slab, and not where the device has no room; the residual is
+    the same."""
+    emu.emu_force_digits(0)
+    from cc4s_b200 import Solver
+    s = _system(cplx=True)
+    T = _amplitudes(cplx=True)
+
+    def residual(limit=0, **options):
+        sol = Solver(options, lib=emu._name)
+        base = emu.emu_live_bytes()
+        emu.emu_peak_bytes(1)
+        _limit(emu, total=limit and base + limit)
+        try:
+            sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=False)
+            peak, live = emu.emu_peak_bytes(0) - base, emu.emu_live_bytes() - base
+        finally:
+            _limit(emu)
+        R = sol.residual(T)
+        if not limit and not options:   # the adjoint schedule too
+            sol.residual_vjp(T, T, gradient=False)
+        sol.close()
+        return R, peak, live
+    ref, peak1, live1 = residual()
+    one, peak0, live0 = residual(integralsSliceSize=NO)   # the default slices, one by one
+    slice_bytes = 16 * NO * NO * NV * NV
+    groups = NV // NO - 1
+    assert live1 - live0 == (groups - 1) * slice_bytes
+    tight, peak, live = residual(limit=max(peak0, live0) + 1024)
+    assert live == live0
+    for q in range(2):
+        assert np.abs(one[q] - ref[q]).max() < 1e-13 * np.abs(ref[q]).max()
+        np.testing.assert_array_equal(tight[q], one[q])
