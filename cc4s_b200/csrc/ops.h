@@ -23,17 +23,23 @@ void d2d(double* dst, const double* src, size_t elems, Stream s);
 // Large transfers of pageable host memory: worker threads move the host side through
 // pinned buffers of their own while the copy engine moves the last pieces.  Element k of
 // the device vector is element k * stride of the host one (2: one plane of interleaved
-// complex values).  Both return when the host memory is done with.  The buffers (32 MiB)
-// belong to the HostStage, made by its first transfer of STAGED_MIN elements or more;
-// smaller ones go straight.
+// complex values).  Both return when the host memory is done with.  The buffers (8 MiB)
+// belong to the HostStage.  Pinning and freeing them takes 8 to 10 ms, so they are made once
+// the transfers of STAGED_MIN elements or more have, by the rates below, lost about that
+// much by going straight.  Measured in ns per element, straight and staged: to the device
+// 0.7 and 0.26, from it into memory not touched before 3.6 and 0.53, every second element
+// 4.2 and 0.24 to, 5.4 and 0.35 from the device; at 2^21 elements 0.87 and 0.77 ms to, 1.2
+// and 0.6 ms from it, at 2^20 no difference.  (32 MiB: 20 ms to pin and free, 0.18 ns per
+// element to the device, the same into new memory.)
 struct HostStage {
   HostStage() = default;
   HostStage(const HostStage&) = delete;
   HostStage& operator=(const HostStage&) = delete;
   ~HostStage();
   void* pinned = nullptr;
+  int64_t lost = 0;  // in elements to the device
 };
-constexpr int64_t STAGED_MIN = int64_t(1) << 21;
+constexpr int64_t STAGED_MIN = int64_t(1) << 21, STAGED_LOST = int64_t(1) << 24;
 void h2d_staged(double* dst, const double* src, int64_t elems, int stride, HostStage& st, Stream s);
 void d2h_staged(double* dst, int stride, const double* src, int64_t elems, HostStage& st, Stream s);
 void sync(Stream s);

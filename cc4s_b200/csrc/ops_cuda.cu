@@ -665,7 +665,7 @@ void sync(Stream s) { CC_CHECK(cudaStreamSynchronize(s)); }
 
 namespace {
 constexpr int STAGE_THREADS = 8;
-constexpr int64_t STAGE_PIECE = int64_t(1) << 18;  // doubles: 2 MiB, two per thread
+constexpr int64_t STAGE_PIECE = int64_t(1) << 16;  // doubles: 512 KiB, two per thread
 
 // Runs body(t) for t < STAGE_THREADS on threads of this device; the caller takes the ones
 // the system would not start.  The first CUDA error wins.
@@ -691,8 +691,11 @@ void stage_run(F&& body) {
   CC_CHECK(static_cast<cudaError_t>(status.load()));
 }
 
-double* stage_buffers(HostStage& st) {
-  if (!st.pinned && cudaHostAlloc(&st.pinned, 2 * STAGE_THREADS * STAGE_PIECE * sizeof(double),
+// The buffers for a transfer of `elems` elements, each as costly without them as `weight`
+// plain ones to the device; null while they would not repay their making.
+double* stage_buffers(HostStage& st, int64_t elems, int weight) {
+  if (elems < STAGED_MIN) return nullptr;
+  if (!st.pinned && (st.lost += elems * weight) >= STAGED_LOST && cudaHostAlloc(&st.pinned, 2 * STAGE_THREADS * STAGE_PIECE * sizeof(double),
                                   cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();
     st.pinned = nullptr;
@@ -734,7 +737,7 @@ HostStage::~HostStage() {
 }
 
 void h2d_staged(double* dst, const double* src, int64_t elems, int stride, HostStage& st, Stream s) {
-  double* pinned = elems >= STAGED_MIN ? stage_buffers(st) : nullptr;
+  double* pinned = stage_buffers(st, elems, stride == 1 ? 1 : 8);
   if (!pinned) {
     std::vector<double> h;
     if (stride != 1) {
@@ -760,7 +763,7 @@ void h2d_staged(double* dst, const double* src, int64_t elems, int stride, HostS
 }
 
 void d2h_staged(double* dst, int stride, const double* src, int64_t elems, HostStage& st, Stream s) {
-  double* pinned = elems >= STAGED_MIN ? stage_buffers(st) : nullptr;
+  double* pinned = stage_buffers(st, elems, 8);
   if (!pinned) {
     std::vector<double> h(stride != 1 ? elems : 0);
     d2h(stride != 1 ? h.data() : dst, src, elems, s);

@@ -11,8 +11,8 @@ CSRC = os.path.join(ROOT, "cc4s_b200", "csrc")
 def build(name="split_check"):
     OUT = os.path.join(HERE, "_build", name)
     os.makedirs(os.path.dirname(OUT), exist_ok=True)
-    srcs = [os.path.join(HERE, name + ".cu"), os.path.join(CSRC, "split_gemm.cu"),
-            os.path.join(CSRC, "gemm_f64.cu")]
+    parts = ("ops_cuda.cu",) if name == "stage_check" else ("split_gemm.cu", "gemm_f64.cu")
+    srcs = [os.path.join(HERE, name + ".cu")] + [os.path.join(CSRC, p) for p in parts]
     deps = srcs + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     if os.path.exists(OUT) and os.path.getmtime(OUT) > max(os.path.getmtime(d) for d in deps):
         return OUT
