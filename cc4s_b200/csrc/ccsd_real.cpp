@@ -533,13 +533,13 @@ void CcsdReal::ppl(const double* Xd, double* R2, const double* dGpp) {
   for (int64_t c0 = 0; c0 < v; c0 += cn) {
     const int64_t nc = std::min(cn, v - c0);
     SplitPackedB pb;
-    if (prepack) {  // timed with the split contractions (no flops of its own)
+    if (prepack) {  // timed with the contractions of its form (no flops of its own)
       const bool prof = profile_ && count_flops_;
       const size_t k = ev_flops_.size();
       if (prof) {
         while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
         ev_flops_.push_back(0.0);
-        ev_split_.push_back(1);
+        ev_digits_.push_back(static_cast<char>(c_first.digits));
         ev_shape_.push_back({0, o * o, nc * v, 1});
         ops::event_record(ev_[2 * k], s_);
       }

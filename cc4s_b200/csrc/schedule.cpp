@@ -50,7 +50,7 @@ void Schedule::gemm_(const Contraction& c) {
     const size_t k = ev_flops_.size();
     while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
     ev_flops_.push_back(f);
-    ev_split_.push_back(0);
+    ev_digits_.push_back(static_cast<char>(c.batch == 1 ? digits_for(c, false) : 0));
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
     fp64_exec(c);
@@ -160,7 +160,7 @@ void Schedule::tc_packed_b_(const Contraction& c, const SplitPackedB& b) {
     const size_t k = ev_flops_.size();
     while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
     ev_flops_.push_back(f);
-    ev_split_.push_back(1);
+    ev_digits_.push_back(static_cast<char>(b.digits));
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
     gemm_split_packed_b(c, b, s_, split_ws());
@@ -180,7 +180,7 @@ void Schedule::tc_prepacked_(const Contraction& c, const SplitOperand& A, const 
     const size_t k = ev_flops_.size();
     while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
     ev_flops_.push_back(f);
-    ev_split_.push_back(1);
+    ev_digits_.push_back(static_cast<char>(A.digits));
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
     gemm_split_prepacked(c, A, ar, B, br, s_, split_ws());
@@ -214,7 +214,7 @@ void Schedule::tc_(const Contraction& c) {
     const size_t k = ev_flops_.size();
     while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
     ev_flops_.push_back(f);
-    ev_split_.push_back(1);
+    ev_digits_.push_back(4);
     ev_shape_.push_back({c.M, c.N, c.K, c.batch});
     ops::event_record(ev_[2 * k], s_);
     split_exec(c);
@@ -244,7 +244,7 @@ bool Schedule::zgemm_split(const Contraction& c, int64_t a_im, int64_t b_im, int
   if (prof) {
     while (ev_.size() < 2 * (k + 1)) ev_.push_back(ops::event_create());
     ev_flops_.push_back(f);
-    ev_split_.push_back(d.digits == 4);
+    ev_digits_.push_back(static_cast<char>(d.digits));
     ev_shape_.push_back({c.M, c.N, 2 * c.K, 2});
     ops::event_record(ev_[2 * k], s_);
   }
@@ -564,7 +564,7 @@ void Schedule::profile_finish() {
     p.gemm_seconds += sec;
     p.gemm_flops += ev_flops_[k];
     if (ev_flops_[k] > p.top_flops) { p.top_flops = ev_flops_[k]; p.top_seconds = sec; }
-    if (ev_split_[k]) {
+    if (ev_digits_[k] == 4) {
       p.split_seconds += sec;
       p.split_flops += ev_flops_[k];
       ++p.split_launches;
@@ -576,7 +576,7 @@ void Schedule::profile_finish() {
     std::map<std::array<int64_t, 5>, std::array<double, 3>> agg;  // count, seconds, flops
     for (size_t k = 0; k < ev_flops_.size(); ++k) {
       const auto& sh = ev_shape_[k];
-      auto& a = agg[{ev_split_[k] ? 1 : 0, sh[0], sh[1], sh[2], sh[3]}];
+      auto& a = agg[{ev_digits_[k], sh[0], sh[1], sh[2], sh[3]}];
       a[0] += 1;
       a[1] += 1e-3 * ops::event_ms(ev_[2 * k], ev_[2 * k + 1]);
       a[2] += ev_flops_[k];
@@ -590,14 +590,14 @@ void Schedule::profile_finish() {
       std::fprintf(f, "# kind M N K batch count seconds TFLOP/s(fp64-equivalent)\n");
       for (const auto& e : order) {
         const auto& a = agg[e.second];
-        std::fprintf(f, "%s %lld %lld %lld %lld %d %.5f %.2f\n", e.second[0] ? "split" : "dmma",
+        std::fprintf(f, "%s %lld %lld %lld %lld %d %.5f %.2f\n", e.second[0] == 4 ? "split" : e.second[0] == 8 ? "digits8" : "dmma",
                      (long long)e.second[1], (long long)e.second[2], (long long)e.second[3],
                      (long long)e.second[4], (int)a[0], a[1], a[2] / a[1] / 1e12);
       }
       std::fclose(f);
     }
   }
-  ev_split_.clear();
+  ev_digits_.clear();
   ev_flops_.clear();
   ev_shape_.clear();
   prof_ = p;

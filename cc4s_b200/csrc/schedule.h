@@ -227,7 +227,7 @@ class Schedule {
   Profile prof_;
   std::vector<void*> ev_;
   std::vector<double> ev_flops_;
-  std::vector<char> ev_split_;
+  std::vector<char> ev_digits_;  // digit form of each profiled launch (0: FP64 pipe)
   std::vector<std::array<int64_t, 4>> ev_shape_;  // M, N, K, batch of each profiled launch
 };
 

@@ -331,3 +331,26 @@ def test_complex_ladder_slab_stays_within_the_caller_and_the_device(emu):
     for q in range(2):
         assert np.abs(one[q] - ref[q]).max() < 1e-13 * np.abs(ref[q]).max()
         np.testing.assert_array_equal(tight[q], one[q])
+
+
+def test_profile_tells_the_forms_apart(emu, monkeypatch, tmp_path):
+    """An FP64 profile counts no split-precision launches, the slicing of the ladder's shared
+    panel included, and the log names the digit form."""
+    from cc4s_b200 import Solver
+    s = inputs.synthetic_system(8, 24, 64, seed=3)
+    rng = np.random.default_rng(5)
+    T2 = rng.standard_normal((24, 24, 8, 8)) * 0.02
+    T = rng.standard_normal((24, 8)) * 0.02, T2 + T2.transpose(1, 0, 3, 2)
+    for precision, kind in (("fp64", "digits8"), ("split3", "split")):
+        log = tmp_path / precision
+        monkeypatch.setenv("CC4S_PROFILE_LOG", str(log))
+        sol = Solver({"precision": precision, "integralsSliceSize": 8, "profile": True},
+                     lib=emu._name)
+        sol.set_inputs(s.eps_h, s.eps_p, s.gamma)
+        sol.residual(T)
+        n = sol.stats()["split_launches"]
+        sol.close()
+        kinds = {line.split()[0] for line in log.read_text().splitlines() if line[0] != "#"}
+        assert kind in kinds and "dmma" in kinds
+        assert (n > 0) == (precision == "split3")
+        assert precision == "split3" or "split" not in kinds
