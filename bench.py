@@ -129,6 +129,35 @@ def dgemm_peak(device):
     return 2.0 * n ** 3 / best / 1e12
 
 
+def int8_peak(device, pk):
+    """INT8 tensor peaks measured here (torch._int_mm 8192^3, CUDA events): best of 10, and
+    back to back for 2 s; twice the measured bf16 rates where the library has no such call."""
+    import torch
+    try:
+        dev = "cuda:%d" % device
+        a, b = (torch.randint(-128, 127, (8192, 8192), dtype=torch.int8, device=dev)
+                for _ in range(2))
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+
+        def timed(n):
+            e[0].record()
+            for _ in range(n):
+                torch._int_mm(a, b.t())
+            e[1].record()
+            torch.cuda.synchronize()
+            return n * 2.0 * 8192 ** 3 / e[0].elapsed_time(e[1]) / 1e9
+        timed(3)
+        burst = max(timed(1) for _ in range(10))
+        src = "torch._int_mm 8192^3 measured in this run, %s (of measured)"
+        return {"burst": burst, "sustained": timed(int(2.0 * burst * 1e12 / (2.0 * 8192 ** 3))),
+                "burst_source": src % "best of 10", "sustained_source": src % "2 s back to back"}
+    except (RuntimeError, AttributeError):
+        src = "2 x MEASURED_PEAKS.json %s (of measured)"
+        return {"burst": 2.0 * pk.get("bf16_tflops", 1686.1),
+                "sustained": 2.0 * pk.get("bf16_tflops_sustained", 1405.3),
+                "burst_source": src % "bf16_tflops", "sustained_source": src % "bf16_tflops_sustained"}
+
+
 def cores_available():
     try:
         return len(os.sched_getaffinity(0))
@@ -265,15 +294,6 @@ DEFAULT_VERTEX_SCALE = 0.2
 FP64_OVER_SPLIT_BOUND = 4.5
 
 
-# DRAM traffic of the split contraction kernel at c2 when its operands were three FP16
-# slices (6 bytes per element, now 4), from one ncu capture of the 851
-# split launches of one iteration (dram__bytes_read.sum + dram__bytes_write.sum with
-# -k regex:split_kernel -c 851 around `bench.py --config c2 --precision split3 --steps 1
-# --warmup 1 --no-cpu-baseline`): 15.09 TB in all, 17.73 GB per launch, 3.6x the
-# algorithmic bytes (packed slices of both operands read once, the output read and
-# written once).
-SPLIT_TRAFFIC_C2 = {"bytes_per_launch": 17.73e9, "algorithmic_bytes_per_launch": 4.9e9,
-                    "launches": 851}
 # Measured on one B200 at c2 (No=64, Nv=640, NG=2560, real): seconds per full
 # iteration of each form (CUDA events), and wall seconds of the host-side input
 # generation, of one handle's set-up (vertex upload, integral build) and of the
@@ -361,33 +381,29 @@ def run_ours(args, world, rank, local):
         else:
             fp64_note = ("skipped: projected %.0f s would pass the %.0f s time budget"
                          % (projected, args.time_budget))
-    dpeak = dgemm_peak(local)
+    dpeak, ipeak = dgemm_peak(local), int8_peak(local, pk)
     if head == "split3":
-        # executed INT8 tensor work: ten digit products per FP64-equivalent multiply-add,
-        # against twice the measured bf16 rate (the INT8 pipe's nominal ratio)
+        # executed INT8 tensor work: ten digit products per FP64-equivalent multiply-add
         achieved = 10.0 * ps["split_flops"] / ps["split_seconds"] / 1e12
-        peak = 2.0 * pk.get("bf16_tflops_sustained", 1405.3)
+        peak = ipeak["sustained"]
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": None,
                 "kernel": "split_kernel_persistent (tcgen05.mma kind::i8, TMEM, TMA) incl. operand "
                           "slicing: %d launches of the last timed iteration, CUDA events on the "
                           "library stream" % ps["split_launches"],
-                "peak_source": "2 x MEASURED_PEAKS.json bf16_tflops_sustained (of measured)",
+                "peak_source": ipeak["sustained_source"],
                 "fp64_equivalent_tflops": ps["split_flops"] / ps["split_seconds"] / 1e12}
-        if cfg == "c2":
-            roof["traffic"] = SPLIT_TRAFFIC_C2["bytes_per_launch"]
-            roof["traffic_note"] = (
-                "bytes per launch, mean over the %d split launches of one iteration (one ncu "
-                "capture); algorithmic %.2g bytes per launch" %
-                (SPLIT_TRAFFIC_C2["launches"], SPLIT_TRAFFIC_C2["algorithmic_bytes_per_launch"]))
     else:
         achieved = ps["gemm_flops"] / ps["gemm_seconds"] / 1e12
-        roof = {"bound": "tensor", "achieved": achieved, "peak": dpeak, "unit": "TFLOP/s",
-                "frac": achieved / dpeak, "traffic": None,
-                "kernel": "gemm_f64_kernel (mma.sync m16n8k16 f64): all %d contraction launches "
-                          "of the last timed iteration" % ps["gemm_profiled_launches"],
-                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (of measured; no FP64 "
-                               "entry in MEASURED_PEAKS.json)",
+        # one FP64 multiply-add is 36 INT8 digit products where the digit form applies
+        peak = ipeak["sustained"] / 36.0
+        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak, "traffic": None,
+                "kernel": "all %d contraction launches of the last timed iteration: the large ones "
+                          "split_kernel_persistent (36 INT8 digit products per multiply-add), the "
+                          "narrow ones gemm_f64_kernel (mma.sync m16n8k16 f64)"
+                          % ps["gemm_profiled_launches"],
+                "peak_source": ipeak["sustained_source"] + ", over 36",
                 "top_launch_tflops": ps["top_flops"] / ps["top_seconds"] / 1e12}
     kind = "complex" if cfg in COMPLEX_CONFIGS else "real"
     conf = {"workload": "CCSD %s: No=%d Nv=%d NG=%d %s, DIIS 5, %s" % (cfg, o, v, G, kind, head),
@@ -762,22 +778,24 @@ def run_triples(args, local):
     torch.cuda.synchronize()
     t_e2e = time.perf_counter() - t0
     pk = peaks()
-    dpeak = dgemm_peak(local)
+    dpeak, ipeak = dgemm_peak(local), int8_peak(local, pk)
     if head == "split3":
         achieved = 10.0 * hr["executed_flops"] / hr["seconds"] / 1e12
-        peak = 2.0 * pk.get("bf16_tflops", 1686.1)
+        peak = ipeak["burst"]
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": None,
                 "kernel": "whole (T) block loop: split_kernel contractions (particle and hole "
                           "halves over K = v + o), singles and energy kernels (ten INT8 digit "
                           "products per executed FP64 multiply-add)",
-                "peak_source": "2 x MEASURED_PEAKS.json bf16_tflops (of measured)"}
+                "peak_source": ipeak["burst_source"]}
     else:
         achieved = hr["executed_flops"] / hr["seconds"] / 1e12
-        roof = {"bound": "tensor", "achieved": achieved, "peak": dpeak, "unit": "TFLOP/s",
-                "frac": achieved / dpeak, "traffic": None,
-                "kernel": "whole (T) block loop (gemm_f64_kernel contractions + bandwidth kernels)",
-                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (of measured)"}
+        peak = ipeak["burst"] / 36.0
+        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak, "traffic": None,
+                "kernel": "whole (T) block loop (split_kernel contractions of 36 INT8 digit products "
+                          "per multiply-add, or gemm_f64_kernel ones, and bandwidth kernels)",
+                "peak_source": ipeak["burst_source"] + ", over 36"}
     line = {"metric": "(T) perturbative triples energy TFLOP/s (reference flop count) on 1 B200",
             "value": F / hr["seconds"] / 1e12, "unit": "TFLOP/s", "n_gpus": 1,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * hr["seconds"],
