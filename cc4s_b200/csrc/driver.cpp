@@ -24,7 +24,7 @@ Handle::Handle(const cc4s_cc_options& o) : opt(o) {
   if (opt.mixer == CC4S_MIXER_DIIS && (opt.max_residua < 1 || opt.max_residua > 8))
     throw Error(ERR_UNSUPPORTED, "maxResidua must be in [1, 8]");
   if (opt.precision != CC4S_PRECISION_FP64 && opt.precision != CC4S_PRECISION_SPLIT3)
-    throw Error(ERR_UNSUPPORTED, "precision must be FP64 or the three-slice split form");
+    throw Error(ERR_UNSUPPORTED, "precision must be FP64 or the split form");
   if (opt.max_iterations < 0) throw Error(ERR_INVALID_ARGUMENT, "maxIterations < 0");
   stream = ops::stream_create(opt.device);
   ev0 = ops::event_create();

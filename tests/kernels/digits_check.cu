@@ -37,6 +37,11 @@ int main(int argc, char** argv) {
   auto ia = [&](int64_t m, int64_t k) { return tA ? k * M + m : m * K + k; };
   auto ib = [&](int64_t k, int64_t n) { return tB ? n * K + k : k * N + n; };
   enum { EVEN, GRADED, INFINITE };
+  for (int digits : {4, 8}) {  // the k ranges of the launch, and S32 spans of a tile
+    const int tn = digits == 8 ? 64 : 128;
+    const int parts = split_k_parts((M + 127) / 128 * ((N + tn - 1) / tn), M, N, (K + 31) / 32 * 32, digits);
+    printf("digits=%d parts=%d spans=%ld\n", digits, parts, (long)((K + parts * 16384 - 1) / (parts * 16384)));
+  }
   for (int digits : {4, 8})
     for (double beta : {0.0, 1.0})
       for (int kind : {EVEN, GRADED, INFINITE}) {

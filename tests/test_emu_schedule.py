@@ -94,7 +94,7 @@ def test_run_matches_oracle(emu_lib, mixer):
 
 
 def test_split_precision_form_accuracy(emu_lib):
-    """Three-slice split products (exact model of the tensor-core scheme) on the
+    """Four-digit split products (exact model of the tensor-core scheme) on the
     ladder/ring/vertex contractions: the converged energy stays far inside 1 uEh."""
     from cc4s_b200 import Solver
     s = inputs.synthetic_system(6, 30, 60, seed=0)  # large enough for the split path (>= 64)

@@ -195,8 +195,8 @@ def test_complex_residual_parity(Solver, shape, hermitian):
 
 
 def test_split_precision_residual(Solver):
-    """Three-slice tensor-core form of the residual vs the FP64 oracle: the split
-    products carry 28 bits of each operand row/column, so the residual agrees to
+    """Four-digit tensor-core form of the residual vs the FP64 oracle: the split
+    products carry 30 bits of each operand row/column, so the residual agrees to
     ~1e-7 of its largest element (tolerance 1e-5)."""
     s = inputs.synthetic_system(16, 128, 256, seed=2)
     rng = np.random.default_rng(3)
