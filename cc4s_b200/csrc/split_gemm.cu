@@ -1135,7 +1135,7 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws,
 // ones and the digit form: 512 x 512 x 256 82 and 91, 512 x 512 x 512 122 and 114,
 // 1024 x 1024 x 64 62 and 67, x 256 187 and 86, 64 x 32768 x 1024 737 and 939.
 bool digits8_pays(const Contraction& c, bool cplx) {
-  if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K < 64) return false;
+  if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K * (cplx ? 2 : 1) < 64) return false;
   const double M = double(c.M), N = double(c.N), K = double(c.K), P = cplx ? 2.0 : 1.0;
   auto up = [](double x, double t) { return std::ceil(x / t) * t; };
   const double tiles = up(M, 128) * up(N, 64) / (128 * 64);

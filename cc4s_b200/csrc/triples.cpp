@@ -484,10 +484,14 @@ TriplesOutcome Triples::run(const double* T) {
   concat_operands(T, Vppph_, Vhhhp_, Ac_, Bc_);
   if (complete_) concat_operands(T, Ip_, Ih_, AcM_, BcM_);
   // Both operands sliced once here where the contractions' K = v + o is long enough: in
-  // four digits (split precision), or in eight (FP64) once a block of pairs fills tiles (the
-  // block loop of 16/128, 224 pairs, 260 -> 184 ms; below a tile's 128 rows most of it is
-  // padding).
-  digits_ = kc_ < 64 ? 0 : precision_ == 3 ? 4 : nb * o >= 128 ? 8 : 0;
+  // four digits (split precision), or in eight (FP64).  Real FP64 blocks gain from 32 pairs
+  // on (block loops, FP64 pipe or slicing per contraction against sliced once: 8/100 with 32
+  // pairs 316 and 262 ms, 16/100 with 64 341 and 282, 16/128 with 224 186 and 147); complex
+  // ones up to 150, beyond which two contractions over both planes, sliced each time, store
+  // half as often (16/80 with 64 pairs 571 and 516, with 128 136 and 125, with 176 112 and
+  // 132; 12/80 with 180 49 and 62 ms).
+  const bool once = cplx_ ? nb * o < 150 : nb * o >= 32;
+  digits_ = kc_ < 64 ? 0 : precision_ == 3 ? 4 : once ? 8 : 0;
   if (digits_) {
     try {
       pack_operands(0, Ac_, Bc_);
@@ -506,9 +510,14 @@ TriplesOutcome Triples::run(const double* T) {
   out.setup_seconds += ops::event_ms(e0, e1) * 1e-3;
   const int64_t Lm = nb * o;
   double* Mi = complete_ && cplx_ ? Mb_ + si_ : nullptr;
-  // The block array holds the connected terms alone where the energy adds the singles (the
-  // cT branch needs their sum in memory).
-  const bool cubes = !complete_ && ops::triples_cube_fits(o, cplx_);
+  // The block array holds the connected terms alone where the energy adds the singles from
+  // cubes in shared memory (the cT branch needs their sum in memory).  A cube takes a block of
+  // 512 threads, which o^3 elements have to fill and as many cubes as SMs to use (block
+  // loops without and with cubes: real 4/60 1.5 and 3.0 ms, 8/100 14.9 and 16.1, 10/100 25.3
+  // and 26.0, 12/100 41.6 and 41.0, 16/128 186 and 171, 24/100 in blocks of 2 2512 and 3053;
+  // complex 8/64 9.7 and 9.9, 10/60 16.3 and 16.0, 16/80 112 and 102).
+  const bool cubes = !complete_ && o >= (cplx_ ? 10 : 12) && nb >= 4 &&
+                     ops::triples_cube_fits(o, cplx_);
   // profile: events around the four phases of every block triple
   std::vector<void*> pev;
   if (profile_) {

@@ -73,8 +73,8 @@ static uint64_t g_refused = 0;
 extern "C" void emu_force_digits(int on) { g_force_digits = on; }
 extern "C" void emu_fail_split_in(int n) { g_fail_in = n; }
 extern "C" uint64_t emu_split_count() { return g_split; }
-bool digits8_pays(const Contraction& c, bool) {
-  return g_force_digits && c.batch == 1 && c.M >= 64 && c.N >= 64 && c.K >= 64;
+bool digits8_pays(const Contraction& c, bool cplx) {
+  return g_force_digits && c.batch == 1 && c.M >= 64 && c.N >= 64 && c.K * (cplx ? 2 : 1) >= 64;
 }
 uint64_t split_launch_count() { return g_split; }
 uint64_t split_pack_launch_count() { return g_pack; }

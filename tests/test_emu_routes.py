@@ -354,3 +354,36 @@ def test_profile_tells_the_forms_apart(emu, monkeypatch, tmp_path):
         assert kind in kinds and "dmma" in kinds
         assert (n > 0) == (precision == "split3")
         assert precision == "split3" or "split" not in kinds
+
+
+@pytest.mark.parametrize("cplx,shape,block", [(False, (12, 5, 9), 4), (True, (10, 5, 9), 4),
+                                              (False, (2, 63, 20), 16), (True, (2, 63, 20), 16)])
+def test_triples_cubes_and_operands_sliced_in_eight_digits(emu, cplx, shape, block):
+    """(T) where the energy adds the singles (hole cubes), and where FP64 operands are sliced
+    once, against the oracle; operands that eight digits refuse run on the FP64 pipe, with
+    the same agreement."""
+    from cc4s_b200 import Solver
+    from oracle import triples
+    No, Nv, NGs = shape
+    s = inputs.synthetic_system(No, Nv, NGs, complex=cplx, seed=6)
+    rng = np.random.default_rng(3)
+    T1 = rng.standard_normal((Nv, No)) * 0.03
+    T2 = rng.standard_normal((Nv, Nv, No, No)) * 0.02
+    if cplx:
+        T1 = T1 + 1j * rng.standard_normal(T1.shape) * 0.03
+        T2 = T2 + 1j * rng.standard_normal(T2.shape) * 0.02
+    T2 = T2 + T2.transpose(1, 0, 3, 2)
+    for graded in (False, True):
+        if graded:  # T falls along the virtual index that the contractions sum over
+            w = 1e-9 ** (np.arange(Nv) / (Nv - 1))
+            T2 = T2 * w[:, None, None, None] * w[None, :, None, None]
+        ref = triples.triples_reference(T1, T2, triples.triples_integrals(s), s.eps_h, s.eps_p)
+        sol = Solver({}, lib=emu._name)
+        sol.set_inputs(s.eps_h, s.eps_p, s.gamma, half_grid=not cplx)
+        sol.set_initial_amplitudes(T1, T2)
+        before = emu.emu_split_count()
+        e = sol.perturbative_triples(block, reference_form=True)["correlation"]
+        used = emu.emu_split_count() - before
+        sol.close()
+        assert abs(e - ref) < 1e-11 * abs(ref), (e, ref)
+        assert Nv < 60 or (used > 0) == (not graded)
