@@ -290,7 +290,7 @@ def timed_run(opts, inputs, W, K, world, local, keep_amplitudes=False):
 DEFAULT_VERTEX_SCALE = 0.2
 # Upper bound of the FP64 form's time per iteration relative to the split form,
 # used only to decide whether the FP64 comparison still fits the time budget
-# (measured at c2: 3.3).
+# (measured at c2: 3.25).
 FP64_OVER_SPLIT_BOUND = 4.5
 
 
@@ -299,7 +299,7 @@ FP64_OVER_SPLIT_BOUND = 4.5
 # generation, of one handle's set-up (vertex upload, integral build) and of the
 # CPU baseline leg.  projected_seconds() uses them to check that the default
 # benchmark command (--steps 20 --warmup 5) fits a 1800 s limit.
-MEASURED_C2 = {"split3": 12.0, "fp64": 69.7, "inputs": 60.0, "setup": 30.0, "cpu": 40.0,
+MEASURED_C2 = {"split3": 8.6, "fp64": 27.8, "inputs": 60.0, "setup": 30.0, "cpu": 40.0,
                "download": 15.0}
 
 

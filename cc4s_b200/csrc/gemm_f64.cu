@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(T::THREADS, 1) gemm_f64_kernel(KParams p) {
 
 // Fixed-order reduction of split-K partials, then the alpha/beta epilogue.  GROUPS = 8
 // (eight splits and more): 32 elements per block, the eight warps sum every eighth split
-// and the eight sums are added in order; GROUPS = 1: one thread per element (one thread per element left a 16 x 16 output with 512 splits to one block's
-// chain of 512 loads).
+// and the eight sums are added in order.  GROUPS = 1: one thread per element (which left a
+// 16 x 16 output with 512 splits to one block's chain of 512 loads).
 template <int GROUPS>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(KParams p) {
   if (p.nothing()) return;

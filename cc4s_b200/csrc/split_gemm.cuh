@@ -25,8 +25,11 @@
 // 2^-53 (FP64 chain, eight digits), by the product sum over sqrt(K): even Gaussian rows 0.1
 // .. 0.8: 3, 0.4 .. 0.04; one element 300 times the others 1e-3 .. 7e-3: 14, 2 .. 0.5; A
 // falling and B rising along k over a factor of 300 2e-3 .. 3e-3: 3, 4 .. 0.7, over 1000
-// 7e-4 .. 1e-3: 3, 12 .. 2 (refused up to K = 2048), over 1e6 1e-6: 3, 14000 .. 2000.
-// (Seven digits of 34 products were at 17 on the factor of 100 that eight hold at 1.)
+// 7e-4 .. 1e-3: 3, 12 .. 2 (refused), over 1e6 1e-6: 3, 14000 .. 2000.
+// (Seven digits of 34 products were at 17 on the factor of 100 that eight hold at 1.)  What
+// passes was at most 1.25 times as far off as the FP64 chain.  The rule holds for 8 rows at a
+// time: where a single row falls along k among even ones while B rises, its outputs are held
+// to the 2^-61 sqrt(K) of the maxima only.
 // In four digits, a row or column holding an Inf or NaN gives NaN in all its outputs.
 #pragma once
 
