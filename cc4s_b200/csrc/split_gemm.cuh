@@ -19,11 +19,11 @@
 // sum is large enough.  The slicing pass takes a profile over k of every 64 rows of an
 // operand (the least, over its groups of 8 rows, of their mean of |x| 2^-e); the product
 // sum of two profiles stands for sum_k |a_k b_k| 2^-(ea+eb) of that 64 x 64 block of the
-// output, and a block below 2^-10 sqrt(K), or with a non-finite element or a row maximum
+// output, and a block below 2^-9 sqrt(K), or with a non-finite element or a row maximum
 // outside 2^+-400, is refused: gemm() computes it on the FP64 tensor pipe, all decided on
 // the device.  Measured on 64 x 64 outputs, K = 64 .. 4096, largest error over sum |a b| in
 // 2^-53 (FP64 chain, eight digits), by the product sum over sqrt(K): even Gaussian rows 0.1
-// .. 0.8: 3, 0.4 .. 0.04; one element 300 times the others 1e-3 .. 7e-3: 14, 2 .. 0.5; A
+// .. 0.8: 3, 0.4 .. 0.04; one element 300 times the others 1e-3 (refused) .. 7e-3: 14, 2 .. 0.5; A
 // falling and B rising along k over a factor of 300 2e-3 .. 3e-3: 3, 4 .. 0.7, over 1000
 // 7e-4 .. 1e-3: 3, 12 .. 2 (refused), over 1e6 1e-6: 3, 14000 .. 2000.
 // (Seven digits of 34 products were at 17 on the factor of 100 that eight hold at 1.)  What
@@ -51,6 +51,7 @@ struct SplitScratch {
 inline float split_profile_least(int64_t K) {
   return static_cast<float>(std::sqrt(static_cast<double>(K)) * 0x1p-9);
 }
+// Row maxima within these powers of two keep every scale and partial product normal.
 constexpr int kSplitMaxExponent = 400;
 
 // Ranges of k that share out the SMs when an output has few tiles (each range writes its
