@@ -1128,12 +1128,12 @@ void split_panel(const Contraction& g, cudaStream_t s, SplitScratch& ws,
 
 // FP64 contractions: the eight-digit form where its time (launches, slicing at 24 bytes per
 // element, waves of one tile per SM) is below the FP64 tensor pipe's.  The constants follow
-// measured contractions that accumulate (FP64 pipe, eight digits, us): 512 x 512 x 512 30 and 55,
-// 1024 x 1024 x 256 47 and 51, x 1024 107 and 70; 128 x 8192 x 1024 108 and 135,
+// measured contractions that accumulate (FP64 pipe, eight digits, us): 512 x 512 x 512 31 and
+// 54, 1024 x 1024 x 256 47 and 46, x 1024 107 and 65; 128 x 8192 x 1024 108 and 126,
 // 64 x 32768 x 1024 184 and 376 (slicing of an operand used 64 times), 1067 x 1067 x 512 68
-// and 70, 2048 x 2048 x 256 160 and 82, 256 x 256 x 16384 111 and 142; complex, four real
+// and 64, 2048 x 2048 x 256 157 and 75, 256 x 256 x 16384 112 and 139; complex, four real
 // ones and the digit form: 512 x 512 x 256 82 and 91, 512 x 512 x 512 122 and 114,
-// 1024 x 1024 x 64 62 and 67, x 256 187 and 86, 64 x 32768 x 1024 737 and 939.
+// 1024 x 1024 x 64 64 and 67, x 256 186 and 86, 64 x 32768 x 1024 737 and 944.
 bool digits8_pays(const Contraction& c, bool cplx) {
   if (c.batch != 1 || c.M < 64 || c.N < 64 || c.K * (cplx ? 2 : 1) < 64) return false;
   const double M = double(c.M), N = double(c.N), K = double(c.K), P = cplx ? 2.0 : 1.0;
@@ -1141,7 +1141,7 @@ bool digits8_pays(const Contraction& c, bool cplx) {
   const double tiles = up(M, 128) * up(N, 64) / (128 * 64);
   const double rows = cplx ? M + N + std::min(M, N) : M + N;
   const int parts = split_k_parts(static_cast<int64_t>(tiles), c.M, c.N, c.K * (cplx ? 2 : 1), 8);
-  const double d8 = (cplx ? 58.0 : 38.0) + 24.0 * rows * P * K / 3.5e6 +
+  const double d8 = (cplx ? 58.0 : 36.0) + 24.0 * rows * P * K / 3.5e6 +
                     P * ((parts > 1 ? 6.0 : 0.0) +
                          std::ceil(tiles * parts / 148.0) * (3.3 + 0.021 * up(P * K, 32) / parts));
   // (outputs beyond 2^22 elements no longer stay in L2 between their load and their store)
